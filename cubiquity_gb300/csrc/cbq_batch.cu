@@ -216,7 +216,7 @@ cbq_status launch_batch_variant(const dev::JobDesc* d_jobs, uint32_t njobs, uint
     if constexpr (!SHARED) {
         if (bl.registers56) kernel = dev::cbq_k_flat_batch_r56<COMPACT, SORTED>;
     }
-    if (cudaMemsetAsync(counter, 0, sizeof(uint64_t), s) != cudaSuccess) return CBQ_ERR_CUDA;
+    if (!bl.counter_zeroed && cudaMemsetAsync(counter, 0, sizeof(uint64_t), s) != cudaSuccess) return CBQ_ERR_CUDA;
     // The prefix offsets, then (shared stack) one column of stack_rows slots per thread.
     const size_t smem = (size_t)(njobs + 1) * 8 + (SHARED ? (size_t)std::max(1, bl.stack_rows) * bl.block * 4 : 0);
     if (smem > 227u * 1024u) return CBQ_ERR_CAPACITY;
@@ -253,18 +253,6 @@ cbq_status launch_batch_kernel(const dev::JobDesc* d_jobs, uint32_t njobs, uint6
     if (total == 0 || njobs == 0) return CBQ_OK;
     return compact ? launch_batch_layout<true>(d_jobs, njobs, total, counter, device, s, bl)
                    : launch_batch_layout<false>(d_jobs, njobs, total, counter, device, s, bl);
-}
-
-cbq_status launch_batch_kernel(const dev::JobDesc* d_jobs, uint32_t njobs, uint64_t total, uint64_t* counter,
-                               int block, uint32_t refill, uint32_t steps, bool compact, int device, cudaStream_t s,
-                               bool registers56)
-{
-    BatchLaunch bl;
-    bl.block = block;
-    bl.refill = refill;
-    bl.steps = steps;
-    bl.registers56 = registers56;
-    return launch_batch_kernel(d_jobs, njobs, total, counter, compact, device, s, bl);
 }
 
 cbq_status launch_batch_octant_sort(const dev::JobDesc* d_jobs, uint32_t njobs, uint64_t total, uint32_t* scratch,

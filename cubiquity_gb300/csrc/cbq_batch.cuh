@@ -38,18 +38,14 @@ struct BatchLaunch {
     bool shared_stack = false;       // descent stack in shared memory (stack_rows rows) instead of local
     int stack_rows = 0;              // max SubDAG height over the jobs
     const uint32_t* perm = nullptr;  // octant order (launch_batch_octant_sort), or null
+    bool counter_zeroed = false;     // the work counter is already zero, in stream order
 };
 
 // Launches the persistent multi-volume kernel over `njobs` device-resident job
 // descriptors holding `total` rays; all jobs' volumes have the compact layout,
-// or none.  `counter` is zeroed on `stream` first.
+// or none.  `counter` is zeroed on `stream` first, unless it is already.
 cbq_status launch_batch_kernel(const dev::JobDesc* d_jobs, uint32_t njobs, uint64_t total, uint64_t* counter,
                                bool compact, int device, cudaStream_t stream, const BatchLaunch& bl);
-
-// The same with the default shape but for block, refill, steps and register cap.
-cbq_status launch_batch_kernel(const dev::JobDesc* d_jobs, uint32_t njobs, uint64_t total, uint64_t* counter,
-                               int block, uint32_t refill, uint32_t steps, bool compact, int device,
-                               cudaStream_t stream, bool registers56 = false);
 
 // Groups each job's rays by octant (direction sign bits): perm[g] for g in a
 // job's range [first, first + count) is a ray of the same job, all of its

@@ -8,6 +8,8 @@
 //    and hit buffers and a launch slot is free.  Each admitted group becomes one
 //    launch on the slot's stream: copies in, one persistent multi-volume
 //    traversal (one job per request, each with its own query), copies out.
+//    Page-locked buffers are copied by one kernel in and one kernel out per
+//    launch (cbq_k_stage_in / cbq_k_stage_out), others by the copy engine.
 //    Groups are launched while earlier ones are still running, so requests that
 //    arrive during a launch overlap it on the device.
 //  - A completion thread waits for each launch's event, frees the requests'
@@ -51,9 +53,12 @@ struct Request {
     uint64_t offset = 0;
     bool direct = false;     // served in place: the kernel reads and writes the caller's host buffers
     bool out_async = true;   // every hit buffer is page-locked (a copy into it does not block the host)
+    bool rays_mapped = false;  // the rays, 16-byte aligned, and
+    bool hits_mapped = false;  // every hit buffer are host memory the GPU can address (d_*)
     const float* d_o = nullptr;
     const float* d_d = nullptr;
     cbq_hits d_hits{};
+    dev::JobDesc job{};      // filled when the request is launched
     Clock::time_point submitted;
     cbq_status status = CBQ_OK;
 };
@@ -84,35 +89,110 @@ bool copy_into_is_async(const void* p)
     return a.type != cudaMemoryTypeUnregistered;
 }
 
-bool hits_copy_async(const cbq_hits& h)
-{
-    const void* fields[] = {h.hit, h.distance, h.material, h.position, h.normal, h.voxel, h.status};
-    for (const void* f : fields)
-        if (f && !copy_into_is_async(f)) return false;
-    return true;
-}
-
-// Resolves every buffer of a request to a device alias; false if any needs staging.
-bool resolve_direct(Request& rq)
+// Finds the device aliases of a request's buffers (rays_mapped, hits_mapped)
+// and whether copies into its hit buffers are asynchronous (out_async).
+void resolve_buffers(Request& rq)
 {
     const cbq_request& r = rq.r;
-    if (((uintptr_t)r.host_origin_tmax & 15u) || ((uintptr_t)r.host_direction & 15u)) return false;
-    rq.d_o = (const float*)device_alias(r.host_origin_tmax);
-    rq.d_d = (const float*)device_alias(r.host_direction);
-    if (!rq.d_o || !rq.d_d) return false;
+    if (!((uintptr_t)r.host_origin_tmax & 15u) && !((uintptr_t)r.host_direction & 15u)) {
+        rq.d_o = (const float*)device_alias(r.host_origin_tmax);
+        rq.d_d = rq.d_o ? (const float*)device_alias(r.host_direction) : nullptr;
+        rq.rays_mapped = rq.d_o && rq.d_d;
+    }
     const cbq_hits& h = r.host_hits;
     cbq_hits& d = rq.d_hits;
     struct F { void* host; void** dev; };
     const F fields[] = {{h.hit, (void**)&d.hit}, {h.distance, (void**)&d.distance}, {h.material, (void**)&d.material},
                         {h.position, (void**)&d.position}, {h.normal, (void**)&d.normal},
                         {h.voxel, (void**)&d.voxel}, {h.status, (void**)&d.status}};
+    rq.hits_mapped = true;
     for (const F& f : fields) {
         *f.dev = nullptr;
         if (!f.host) continue;
-        *f.dev = (void*)device_alias(f.host);
-        if (!*f.dev) return false;
+        if (rq.hits_mapped) *f.dev = (void*)device_alias(f.host);
+        if (*f.dev) continue;
+        rq.hits_mapped = false;
+        rq.out_async = rq.out_async && copy_into_is_async(f.host);
     }
-    return true;
+}
+
+// Copies of a launch between its requests' page-locked buffers and the pool.
+// The copy engine took two copies in, the job table, the counter's memset and
+// up to seven copies out per request, each a call of 2-4 us on the launching
+// thread and a few us of the stream's time.  Two kernels do all of it for
+// every request of a launch: 24 requests of 1 Ki to 64 Ki rays submitted from
+// one Python thread 1,040 -> 828 us (median latency of one 136 -> 107 us).  They are bound by the host link and their launches; 16-byte accesses by whole warps on the host
+// side, so that the link carries full lines.
+struct StageIn {
+    const float4 *o, *d;   // host rays
+    float4 *dst_o, *dst_d;
+    uint64_t count;
+    uint64_t pad;
+};
+struct StageOut {
+    const char* src;       // pool, 4-byte aligned
+    char* dst;             // host, any alignment
+    uint64_t bytes;
+};
+constexpr int kStageBlock = 256;
+constexpr uint64_t kStageRequestsMax = 4096;  // per launch: seven times that are grid rows
+constexpr int kHitFields = 7;
+
+// Row y of the grid copies the rays of in[y]; the last row the job table (in
+// 8-byte words) and the zero of the work counter.
+__global__ void __launch_bounds__(kStageBlock) cbq_k_stage_in(const StageIn* __restrict__ in, uint32_t rows,
+                                                             const uint64_t* __restrict__ h_table,
+                                                             uint64_t* __restrict__ d_table, uint32_t table_words,
+                                                             unsigned long long* __restrict__ counter)
+{
+    const uint64_t first = (uint64_t)blockIdx.x * kStageBlock + threadIdx.x;
+    const uint64_t stride = (uint64_t)gridDim.x * kStageBlock;
+    if (blockIdx.y == rows) {
+        if (first == 0) *counter = 0ull;
+        for (uint64_t i = first; i < table_words; i += stride) d_table[i] = __ldcs(h_table + i);
+        return;
+    }
+    const StageIn s = in[blockIdx.y];
+    for (uint64_t i = first; i < s.count; i += stride) {
+        const float4 o = __ldcs(s.o + i), d = __ldcs(s.d + i);
+        s.dst_o[i] = o;
+        s.dst_d[i] = d;
+    }
+}
+
+// Row y copies out[y]: 16-byte stores to the host side, the source words
+// shifted into place where the two sides' alignments differ; the unaligned
+// ends byte by byte.  Reads at most 3 bytes beyond the source's end, which the
+// pool's padding covers.
+__global__ void __launch_bounds__(kStageBlock) cbq_k_stage_out(const StageOut* __restrict__ out)
+{
+    const StageOut s = out[blockIdx.y];
+    const uint64_t first = (uint64_t)blockIdx.x * kStageBlock + threadIdx.x;
+    const uint64_t stride = (uint64_t)gridDim.x * kStageBlock;
+    const uint64_t lead = (16u - ((uintptr_t)s.dst & 15u)) & 15u, head = lead < s.bytes ? lead : s.bytes;
+    const uint64_t body = (s.bytes - head) / 16u, tail = head + body * 16u;
+    if (first < head) s.dst[first] = s.src[first];
+    if (first < s.bytes - tail) s.dst[tail + first] = s.src[tail + first];
+    const uint32_t* words = (const uint32_t*)(s.src + (head & ~(uint64_t)3u));
+    const uint32_t shift = (uint32_t)(head & 3u) * 8u;
+    uint4* dst = (uint4*)(s.dst + head);
+    for (uint64_t i = first; i < body; i += stride) {
+        const uint32_t* w = words + 4 * i;
+        uint4 v = make_uint4(__ldcs(w), __ldcs(w + 1), __ldcs(w + 2), __ldcs(w + 3));
+        if (shift != 0u) {
+            const uint32_t next = __ldcs(w + 4);
+            v = make_uint4(__funnelshift_r(v.x, v.y, shift), __funnelshift_r(v.y, v.z, shift),
+                           __funnelshift_r(v.z, v.w, shift), __funnelshift_r(v.w, next, shift));
+        }
+        dst[i] = v;
+    }
+}
+
+// Blocks per row for rows of up to `items` 16-byte accesses: two per thread,
+// at most 64 (16,384 threads keep enough lines in flight for the host link).
+unsigned stage_blocks(uint64_t items)
+{
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(64, (items + 2 * kStageBlock - 1) / (2 * kStageBlock)));
 }
 
 // First-fit allocator over [0, size).
@@ -159,7 +239,9 @@ private:
 struct Slot {
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
-    dev::JobDesc* h_table = nullptr;  // pinned
+    dev::JobDesc* h_table = nullptr;  // pinned, followed by the staging tables
+    StageIn* h_in = nullptr;
+    StageOut* h_out = nullptr;
     dev::JobDesc* d_table = nullptr;
     uint64_t* d_counter = nullptr;
     std::vector<Request*> reqs;
@@ -233,16 +315,51 @@ void cbq_server::launch_group(int si, std::vector<Request*>& group, std::unique_
     cv_complete.notify_one();
 }
 
+// A request's hit arrays in the pool, in the order of copy_hits_back.
+struct PoolHits {
+    dev::HitsOut out;
+    const char* src[kHitFields];
+    uint64_t bytes[kHitFields];
+};
+
+static PoolHits pool_hits(char* h, uint64_t n)
+{
+    PoolHits p;
+    const uint64_t bytes[kHitFields] = {n * 12, n * 12, n * 12, n * 4, n * 4, n, n};
+    char* at[kHitFields];
+    for (int f = 0; f < kHitFields; f++) {
+        at[f] = h;
+        p.src[f] = h;
+        p.bytes[f] = bytes[f];
+        h += align_up(bytes[f]);
+    }
+    p.out.position = (float*)at[0];
+    p.out.normal = (float*)at[1];
+    p.out.voxel = (int32_t*)at[2];
+    p.out.distance = (float*)at[3];
+    p.out.material = (uint32_t*)at[4];
+    p.out.hit = (uint8_t*)at[5];
+    p.out.status = (uint8_t*)at[6];
+    return p;
+}
+
 cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
 {
-    uint32_t njobs = 0;
-    uint64_t total = 0;
+    const bool stage = group.size() <= kStageRequestsMax;
+    uint32_t njobs = 0, rows_in = 0, rows_out = 0;
+    uint64_t total = 0, most_rays = 0, most_bytes = 0;
+    // First pass: where every request's rays and hits are on the device, the job and
+    // staging tables, and the copies in that the staging kernel does not make.
     for (Request* rq : group) {
         const uint64_t n = rq->r.ray_count;
+        dev::JobDesc jd;
+        std::memset(&jd, 0, sizeof(jd));
+        fill_job_volume(jd, rq->r.dag);
+        jd.count = n;
+        jd.q.compute_surface = rq->r.query.compute_surface;
+        jd.q.max_footprint = rq->r.query.max_footprint;
+        jd.q.flags = rq->r.query.flags;
         if (rq->direct) {  // the kernel reads the rays and writes the hits in host memory itself
-            dev::JobDesc jd;
-            std::memset(&jd, 0, sizeof(jd));
-            fill_job_volume(jd, rq->r.dag);
             jd.orig = (const float4*)rq->d_o;
             jd.dir = (const float4*)rq->d_d;
             const cbq_hits& dh = rq->d_hits;
@@ -253,70 +370,75 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
             jd.out.normal = dh.normal;
             jd.out.voxel = dh.voxel;
             jd.out.status = dh.status;
-            jd.count = n;
-            jd.q.compute_surface = rq->r.query.compute_surface;
-            jd.q.max_footprint = rq->r.query.max_footprint;
-            jd.q.flags = rq->r.query.flags;
-            if (!rq->r.dag->flat_ok) {
-                cbq_rays rays{rq->d_o, rq->d_d};
-                cbq_status st = cbq_intersect(rq->r.dag, &rays, n, &rq->r.query, &dh, (cbq_stream_t)s.stream);
-                if (st != CBQ_OK) return st;
-                continue;
+        } else {
+            char* p = d_pool + rq->offset;
+            float* o = (float*)p;
+            float* d = (float*)(p + n * 16);
+            const PoolHits hits = pool_hits(p + n * 32, n);
+            jd.orig = (const float4*)o;
+            jd.dir = (const float4*)d;
+            jd.out = hits.out;
+            if (stage && rq->rays_mapped) {
+                s.h_in[rows_in++] = StageIn{(const float4*)rq->d_o, (const float4*)rq->d_d, (float4*)o, (float4*)d, n, 0};
+                most_rays = std::max(most_rays, n);
+            } else if (cudaMemcpyAsync(o, rq->r.host_origin_tmax, n * 16, cudaMemcpyHostToDevice, s.stream) !=
+                           cudaSuccess ||
+                       cudaMemcpyAsync(d, rq->r.host_direction, n * 16, cudaMemcpyHostToDevice, s.stream) !=
+                           cudaSuccess) {
+                return CBQ_ERR_CUDA;
             }
-            jd.first = total;
-            s.h_table[njobs++] = jd;
-            total += n;
-            continue;
+            if (stage && rq->hits_mapped) {
+                const cbq_hits& hh = rq->d_hits;
+                void* dst[kHitFields] = {hh.position, hh.normal, hh.voxel, hh.distance, hh.material, hh.hit, hh.status};
+                for (int f = 0; f < kHitFields; f++) {
+                    if (!dst[f]) continue;
+                    s.h_out[rows_out++] = StageOut{hits.src[f], (char*)dst[f], hits.bytes[f]};
+                    most_bytes = std::max(most_bytes, hits.bytes[f]);
+                }
+            }
         }
-        char* p = d_pool + rq->offset;
-        float* o = (float*)p;
-        float* d = (float*)(p + n * 16);
-        char* h = p + n * 32;
-        dev::HitsOut out;
-        out.position = (float*)h; h += align_up(n * 12);
-        out.normal = (float*)h; h += align_up(n * 12);
-        out.voxel = (int32_t*)h; h += align_up(n * 12);
-        out.distance = (float*)h; h += align_up(n * 4);
-        out.material = (uint32_t*)h; h += align_up(n * 4);
-        out.hit = (uint8_t*)h; h += align_up(n);
-        out.status = (uint8_t*)h;
-        if (cudaMemcpyAsync(o, rq->r.host_origin_tmax, n * 16, cudaMemcpyHostToDevice, s.stream) != cudaSuccess ||
-            cudaMemcpyAsync(d, rq->r.host_direction, n * 16, cudaMemcpyHostToDevice, s.stream) != cudaSuccess)
-            return CBQ_ERR_CUDA;
-        dev::JobDesc jd;
-        std::memset(&jd, 0, sizeof(jd));
-        fill_job_volume(jd, rq->r.dag);
-        jd.orig = (const float4*)o;
-        jd.dir = (const float4*)d;
-        jd.out = out;
-        jd.count = n;
-        jd.q.compute_surface = rq->r.query.compute_surface;
-        jd.q.max_footprint = rq->r.query.max_footprint;
-        jd.q.flags = rq->r.query.flags;
-        if (!rq->r.dag->flat_ok) {  // integer positions (far coordinates, huge stores): launched on its own
-            cbq_rays rays{o, d};
-            cbq_hits hits{out.hit, out.distance, out.material, out.position, out.normal, out.voxel, out.status};
-            cbq_status st = cbq_intersect(rq->r.dag, &rays, n, &rq->r.query, &hits, (cbq_stream_t)s.stream);
-            if (st != CBQ_OK) return st;
-            continue;
-        }
+        rq->job = jd;
+        if (!rq->r.dag->flat_ok) continue;  // integer positions (far coordinates, huge stores): launched on its own
         jd.first = total;
         s.h_table[njobs++] = jd;
         total += n;
     }
-    if (njobs) {
-        if (cudaMemcpyAsync(s.d_table, s.h_table, njobs * sizeof(dev::JobDesc), cudaMemcpyHostToDevice, s.stream) !=
-            cudaSuccess)
-            return CBQ_ERR_CUDA;
-        cbq_status st = launch_batch_kernel(s.d_table, njobs, total, s.d_counter, cfg.block, cfg.refill_min,
-                                            kBatchStepsDefault, group[0]->r.dag->layout == CBQ_DAG_LAYOUT_COMPACT,
-                                            device, s.stream);
+    static_assert(sizeof(dev::JobDesc) % 8 == 0, "the job table is copied in 8-byte words");
+    if (rows_in || njobs) {
+        const uint32_t words = njobs * (uint32_t)(sizeof(dev::JobDesc) / 8);
+        const dim3 grid(stage_blocks(std::max<uint64_t>(2 * most_rays, words)), rows_in + 1);
+        cbq_k_stage_in<<<grid, kStageBlock, 0, s.stream>>>(s.h_in, rows_in, (const uint64_t*)s.h_table,
+                                                           (uint64_t*)s.d_table, words,
+                                                           (unsigned long long*)s.d_counter);
+        if (cudaGetLastError() != cudaSuccess) return CBQ_ERR_CUDA;
+    }
+    for (Request* rq : group) {
+        if (rq->r.dag->flat_ok) continue;
+        const dev::JobDesc& jd = rq->job;
+        cbq_rays rays{(const float*)jd.orig, (const float*)jd.dir};
+        cbq_hits hits{jd.out.hit, jd.out.distance, jd.out.material, jd.out.position, jd.out.normal, jd.out.voxel,
+                      jd.out.status};
+        cbq_status st = cbq_intersect(rq->r.dag, &rays, rq->r.ray_count, &rq->r.query, &hits, (cbq_stream_t)s.stream);
         if (st != CBQ_OK) return st;
     }
-    // Results back to page-locked host buffers; pageable ones are copied by the completion
-    // thread once the launch is done, so that this thread never waits for the device.
+    if (njobs) {
+        BatchLaunch bl;
+        bl.block = cfg.block;
+        bl.refill = cfg.refill_min;
+        bl.counter_zeroed = true;
+        cbq_status st = launch_batch_kernel(s.d_table, njobs, total, s.d_counter,
+                                            group[0]->r.dag->layout == CBQ_DAG_LAYOUT_COMPACT, device, s.stream, bl);
+        if (st != CBQ_OK) return st;
+    }
+    if (rows_out) {
+        const dim3 grid(stage_blocks(most_bytes / 16), rows_out);
+        cbq_k_stage_out<<<grid, kStageBlock, 0, s.stream>>>(s.h_out);
+        if (cudaGetLastError() != cudaSuccess) return CBQ_ERR_CUDA;
+    }
+    // Results back to the other page-locked host buffers; pageable ones are copied by the
+    // completion thread once the launch is done, so that this thread never waits for the device.
     for (Request* rq : group) {
-        if (rq->direct || !rq->out_async) continue;
+        if (rq->direct || !rq->out_async || (stage && rq->hits_mapped)) continue;
         const cbq_status st = copy_hits_back(rq, s.stream);
         if (st != CBQ_OK) return st;
     }
@@ -326,15 +448,12 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
 cbq_status cbq_server::copy_hits_back(const Request* rq, cudaStream_t stream) const
 {
     const uint64_t n = rq->r.ray_count;
-    char* h = d_pool + rq->offset + n * 32;
+    const PoolHits hits = pool_hits(d_pool + rq->offset + n * 32, n);
     const cbq_hits& hh = rq->r.host_hits;
-    struct Copy { void* dst; size_t bytes; };
-    const Copy copies[] = {{hh.position, n * 12}, {hh.normal, n * 12}, {hh.voxel, n * 12},
-                           {hh.distance, n * 4}, {hh.material, n * 4}, {hh.hit, n}, {hh.status, n}};
-    for (const Copy& c : copies) {
-        if (c.dst && cudaMemcpyAsync(c.dst, h, c.bytes, cudaMemcpyDeviceToHost, stream) != cudaSuccess)
+    void* dst[kHitFields] = {hh.position, hh.normal, hh.voxel, hh.distance, hh.material, hh.hit, hh.status};
+    for (int f = 0; f < kHitFields; f++) {
+        if (dst[f] && cudaMemcpyAsync(dst[f], hits.src[f], hits.bytes[f], cudaMemcpyDeviceToHost, stream) != cudaSuccess)
             return CBQ_ERR_CUDA;
-        h += align_up(c.bytes);
     }
     return CBQ_OK;
 }
@@ -477,14 +596,20 @@ cbq_status cbq_server_create(const cbq_server_config* cfg, cbq_server** out)
     s->pool.init(c.device_memory_budget);
     s->slots.resize(c.max_inflight_launches);
     const size_t table = (size_t)c.max_batch_requests * sizeof(dev::JobDesc);
+    const size_t staged = std::min<size_t>((size_t)c.max_batch_requests, kStageRequestsMax);
     bool ok = true;
     for (int i = 0; i < c.max_inflight_launches && ok; i++) {
         Slot& sl = s->slots[i];
         ok = cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking) == cudaSuccess &&
              cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming) == cudaSuccess &&
-             cudaMallocHost((void**)&sl.h_table, table) == cudaSuccess &&
+             cudaMallocHost((void**)&sl.h_table, table + staged * (sizeof(StageIn) + kHitFields * sizeof(StageOut))) ==
+                 cudaSuccess &&
              cudaMalloc((void**)&sl.d_counter, 256 + table) == cudaSuccess;
-        if (ok) sl.d_table = (dev::JobDesc*)((char*)sl.d_counter + 256);
+        if (ok) {
+            sl.d_table = (dev::JobDesc*)((char*)sl.d_counter + 256);
+            sl.h_in = (StageIn*)((char*)sl.h_table + table);
+            sl.h_out = (StageOut*)(sl.h_in + staged);
+        }
         s->free_slots.push_back(i);
     }
     if (!ok) {
@@ -518,9 +643,9 @@ cbq_status cbq_server_submit(cbq_server* s, const cbq_request* r, uint64_t* tick
     if (!rq) return CBQ_ERR_OUT_OF_MEMORY;
     rq->submitted = Clock::now();
     rq->r = *r;
-    rq->direct = r->ray_count > 0 && (s->cfg.flags & CBQ_SERVER_IN_PLACE) && resolve_direct(*rq);
+    if (r->ray_count > 0) resolve_buffers(*rq);
+    rq->direct = (s->cfg.flags & CBQ_SERVER_IN_PLACE) && rq->rays_mapped && rq->hits_mapped;
     rq->bytes = rq->direct ? 0 : request_bytes(r->ray_count);
-    rq->out_async = rq->direct || hits_copy_async(r->host_hits);
     if (rq->bytes > s->cfg.device_memory_budget) {
         delete rq;
         return CBQ_ERR_CAPACITY;
