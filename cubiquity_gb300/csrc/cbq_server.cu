@@ -121,8 +121,9 @@ void resolve_buffers(Request& rq)
 // up to seven copies out per request, each a call of 2-4 us on the launching
 // thread and a few us of the stream's time.  Two kernels do all of it for
 // every request of a launch: 24 requests of 1 Ki to 64 Ki rays submitted from
-// one Python thread 1,040 -> 828 us (median latency of one 136 -> 107 us).  They are bound by the host link and their launches; 16-byte accesses by whole warps on the host
-// side, so that the link carries full lines.
+// one Python thread 1,040 -> 828 us (median latency of one 136 -> 107 us).
+// They are bound by the host link and their launches; 16-byte accesses by whole
+// warps on the host side, so that the link carries full lines.
 struct StageIn {
     const float4 *o, *d;   // host rays
     float4 *dst_o, *dst_d;
