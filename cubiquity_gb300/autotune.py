@@ -39,7 +39,8 @@ def cache_key(dag: cbq.Dag, direction) -> str:
     gpu = torch.cuda.get_device_name() if torch.cuda.is_available() else "cpu"
     size_class = int(round(math.log2(max(1, dag.bytes))))
     layout = "|compact" if getattr(dag, "layout", 0) == cbq.LAYOUT_COMPACT else ""
-    return f"{gpu}|dag2^{size_class}{layout}|{ray_mix(direction)}"
+    # "walk2": shapes tuned for another walk are not taken over.
+    return f"{gpu}|dag2^{size_class}{layout}|{ray_mix(direction)}|walk2"
 
 
 def _load() -> dict:

@@ -17,7 +17,7 @@ using namespace cbq;
 namespace {
 
 constexpr int kFlatBlockDefault = 128;  // GB300, terrain-4096: 64, 128 and 256 threads within 1-3%
-constexpr uint32_t kRefillDefault = 8;
+constexpr uint32_t kRefillDefault = 16;
 
 bool use_flat(const cbq_dag* dag)
 {
@@ -47,7 +47,9 @@ dev::DagParams make_dag_params(const cbq_dag* dag)
 {
     dev::DagParams p;
     p.nodes = dag->d_nodes;
+    p.occupied = 0u;
     for (int i = 0; i < 8; i++) {
+        if (dag->sd_ref[i] != 0u) p.occupied |= 1u << i;
         p.sd[i].lx = dag->subdags[i].lower_bound[0];
         p.sd[i].ly = dag->subdags[i].lower_bound[1];
         p.sd[i].lz = dag->subdags[i].lower_bound[2];
@@ -63,6 +65,7 @@ dev::QueryParams make_query(const cbq_query* q)
     dev::QueryParams p;
     p.compute_surface = q ? q->compute_surface : 1;
     p.max_footprint = q ? q->max_footprint : CBQ_MAX_FOOTPRINT_DISABLED;
+    p.footprint_tmax = footprint_exit_max(p.max_footprint);
     p.flags = q ? q->flags : 0u;
     p.image_width = q ? q->image_width : 0u;  // checked against each launch's ray count by launch_flat
     return p;
@@ -206,8 +209,7 @@ __global__ void __launch_bounds__(kPersistBlock) cbq_k_intersect_persistent(
 {
     extern __shared__ uint32_t smem_stack[];
     dev::SharedStack stack;
-    stack.base = smem_stack + threadIdx.x;
-    stack.stride = blockDim.x;
+    stack.init(smem_stack + threadIdx.x, blockDim.x);
     const unsigned lane = threadIdx.x & 31u;
     for (;;) {
         unsigned long long base = 0;

@@ -26,15 +26,13 @@ __device__ __forceinline__ void flat_body(const Ctx& c, uint64_t n, unsigned lon
 {
     extern __shared__ uint32_t smem_stack[];
     SharedStack sstack;
-    sstack.base = smem_stack + threadIdx.x;
-    sstack.stride = blockDim.x;
+    sstack.init(smem_stack + threadIdx.x, blockDim.x);
     LocalStack lstack;
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t below = (1u << lane) - 1u;
 
     Lane L;
     L.mode = kLaneIdle;
-    L.held = 0u;
     bool more = PERSISTENT;  // warp-uniform: the queue may still hold rays
     if (!PERSISTENT) {
         const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -60,18 +58,21 @@ __device__ __forceinline__ void flat_body(const Ctx& c, uint64_t n, unsigned lon
             if (!more) break;
             continue;
         }
-        lane_settle(L, c);
-        // Up to `steps` ESVO steps per outer iteration: amortises the refill
-        // ballot and the settle check over several node fetches.
         if (SHARED)
-            warp_walk_steps(L, c, sstack, steps);
+            lane_settle(L, c, sstack);
         else
-            warp_walk_steps(L, c, lstack, steps);
+            lane_settle(L, c, lstack);
+        // The walk goes on until refill_min lanes are idle (checked every
+        // `steps` iterations) or, with no rays left, until all are.
+        if (SHARED)
+            warp_walk_steps(L, c, sstack, steps, PERSISTENT && more ? refill_min : 32u);
+        else
+            warp_walk_steps(L, c, lstack, steps, PERSISTENT && more ? refill_min : 32u);
     }
 }
 
 template <bool PERSISTENT, bool SHARED, bool SORTED, typename Ctx>
-__global__ void __launch_bounds__(256) cbq_k_flat(Ctx c, uint64_t n, unsigned long long* __restrict__ counter,
+__global__ void __launch_bounds__(256, PERSISTENT && !Ctx::kIntPos ? 5 : 4) cbq_k_flat(Ctx c, uint64_t n, unsigned long long* __restrict__ counter,
                                                   uint32_t refill_min, const uint32_t* __restrict__ perm,
                                                   uint32_t steps)
 {
@@ -214,7 +215,9 @@ cbq_status launch_variant(const Ctx& c, uint64_t n, const FlatLaunch& fl, int ro
             return CBQ_ERR_CUDA;
         per_sm = std::max(per_sm, 1);
         if (cudaMemsetAsync(fl.counter, 0, sizeof(uint64_t), stream) != cudaSuccess) return CBQ_ERR_CUDA;
-        kernel<<<sms * per_sm, fl.block, smem, stream>>>(c, n, (unsigned long long*)fl.counter, fl.refill_min,
+        // No more blocks than the rays fill.
+        const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sms * per_sm, (n + fl.block - 1) / fl.block);
+        kernel<<<grid, fl.block, smem, stream>>>(c, n, (unsigned long long*)fl.counter, fl.refill_min,
                                                           fl.perm, fl.steps ? fl.steps : 1u);
     }
     return cudaGetLastError() == cudaSuccess ? CBQ_OK : CBQ_ERR_CUDA;
@@ -289,20 +292,26 @@ cbq_status launch_flat(const cbq_dag* dag, const dev::DagParams& dp, const dev::
         one.perm = nullptr;
         if (dag->layout == CBQ_DAG_LAYOUT_COMPACT)
             return launch_variant<false, false, false>(
-                make_ctx<dev::FlatCtxT<true, true>>(dp, q, out, orig, dir, fetch_out), n, one, rows, stream, dv);
+                make_ctx<dev::FlatCtxT<true, true, false, true>>(dp, q, out, orig, dir, fetch_out), n, one, rows, stream, dv);
         if (!dag->flat_ok)
             return launch_variant<false, false, false>(
                 make_ctx<dev::FlatCtxT<false, true, true>>(dp, q, out, orig, dir, fetch_out), n, one, rows, stream,
                 dv);
         return launch_variant<false, false, false>(
-            make_ctx<dev::FlatCtxT<false, true>>(dp, q, out, orig, dir, fetch_out), n, one, rows, stream, dv);
+            make_ctx<dev::FlatCtxT<false, true, false, true>>(dp, q, out, orig, dir, fetch_out), n, one, rows, stream, dv);
     }
+    const bool lod = !(q.max_footprint < 0.0f);
     if (dag->layout == CBQ_DAG_LAYOUT_COMPACT)
-        return launch_ctx(make_ctx<dev::FlatCtxT<true>>(dp, q, out, orig, dir, nullptr), n, fl, rows, stream, dv);
+        return lod ? launch_ctx(make_ctx<dev::FlatCtxT<true, false, false, true>>(dp, q, out, orig, dir, nullptr), n,
+                                fl, rows, stream, dv)
+                   : launch_ctx(make_ctx<dev::FlatCtxT<true>>(dp, q, out, orig, dir, nullptr), n, fl, rows, stream,
+                                dv);
     if (!dag->flat_ok)  // coordinates beyond +-2^21 or 2^29 nodes or more: integer positions
         return launch_ctx(make_ctx<dev::FlatCtxT<false, false, true>>(dp, q, out, orig, dir, nullptr), n, fl, rows,
                           stream, dv);
-    return launch_ctx(make_ctx<dev::FlatCtxT<false>>(dp, q, out, orig, dir, nullptr), n, fl, rows, stream, dv);
+    return lod ? launch_ctx(make_ctx<dev::FlatCtxT<false, false, false, true>>(dp, q, out, orig, dir, nullptr), n, fl,
+                            rows, stream, dv)
+               : launch_ctx(make_ctx<dev::FlatCtxT<false>>(dp, q, out, orig, dir, nullptr), n, fl, rows, stream, dv);
 }
 
 }  // namespace cbq

@@ -65,6 +65,20 @@ cbq_status validate_nodes(const uint32_t* nodes, uint64_t node_count, uint32_t r
     return CBQ_OK;
 }
 
+float footprint_exit_max(float mf)
+{
+    if (mf < 0.0f) return std::numeric_limits<float>::infinity();
+    if (!(mf < std::numeric_limits<float>::infinity())) return -1.0f;  // infinite or NaN: no quotient is larger
+    // 1.0f / t does not increase with t, so the answer is the boundary next to 1 / mf.
+    const float big = std::numeric_limits<float>::max();
+    if (1.0f / big > mf) return big;
+    float t = 1.0f / mf;
+    if (!(t < big)) t = big;
+    while (t > 0.0f && !(1.0f / t > mf)) t = std::nextafter(t, 0.0f);
+    for (float up = std::nextafter(t, big); up > t && 1.0f / up > mf; up = std::nextafter(t, big)) t = up;
+    return t;
+}
+
 namespace {
 std::atomic<cbq_log_fn> g_log_fn{nullptr};
 std::atomic<void*> g_log_user{nullptr};

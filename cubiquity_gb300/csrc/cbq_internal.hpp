@@ -19,6 +19,12 @@ cbq_status find_subdags(const uint32_t* nodes, uint64_t node_count, uint32_t roo
 // Full structural check of a host node array.
 cbq_status validate_nodes(const uint32_t* nodes, uint64_t node_count, uint32_t root);
 
+// The largest t >= 0 with 1.0f / t > max_footprint (infinity for a negative
+// max_footprint, -1 where there is none): for a child of size s, a power of
+// two, and an exit distance t >= 0 in the range where the quotient neither
+// overflows nor underflows, s / t > max_footprint exactly when t <= s * that.
+float footprint_exit_max(float max_footprint);
+
 // printf-style message to the registered log handler (no-op without one).
 void log(int level, const char* fmt, ...)
 #if defined(__GNUC__)
@@ -91,12 +97,9 @@ struct cbq_dag {
     int device = 0;
     bool flat_ok = false;          // float-position flat kernel applies (coordinates within +-2^21,
                                    // under 2^29 nodes); otherwise the integer-position form
-    // Defaults from GB300 sweeps of untuned shapes on terrain-4096 (primary and bounce
-    // rays) and the city pathtracer: persistent refill (block 128, 8 idle lanes), stack in
-    // shared memory, 16 ESVO steps per loop iteration; against the 56-register
-    // local-stack kernel at 8 steps: primary 6.47 vs 6.05, bounce 3.65 vs 3.55 Grays/s,
-    // city frame 42.5 vs 43.0 ms.
-    cbq_launch_config cfg{CBQ_KERNEL_AUTO, 0, 0, 0, CBQ_STACK_SHARED, CBQ_FORM_PERSISTENT, 16, 0};
+    // Defaults from GB300 sweeps of the ordered walk: persistent refill (block 128, 16 idle
+    // lanes), stack in shared memory, 8 iterations between the checks for idle lanes.
+    cbq_launch_config cfg{CBQ_KERNEL_AUTO, 0, 0, 0, CBQ_STACK_SHARED, CBQ_FORM_PERSISTENT, 8, 0};
 
     // Staging sets of cbq_intersect_host, created as concurrent calls need them.
     std::mutex stages_lock;

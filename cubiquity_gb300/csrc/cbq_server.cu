@@ -349,6 +349,7 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
     const bool stage = group.size() <= kStageRequestsMax;
     uint32_t njobs = 0, rows_in = 0, rows_out = 0;
     uint64_t total = 0, most_rays = 0, most_bytes = 0;
+    int stack_rows = 1;
     // First pass: where every request's rays and hits are on the device, the job and
     // staging tables, and the copies in that the staging kernel does not make.
     for (Request* rq : group) {
@@ -359,6 +360,7 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
         jd.count = n;
         jd.q.compute_surface = rq->r.query.compute_surface;
         jd.q.max_footprint = rq->r.query.max_footprint;
+        jd.q.footprint_tmax = footprint_exit_max(jd.q.max_footprint);
         jd.q.flags = rq->r.query.flags;
         if (rq->direct) {  // the kernel reads the rays and writes the hits in host memory itself
             jd.orig = (const float4*)rq->d_o;
@@ -403,6 +405,7 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
         jd.first = total;
         s.h_table[njobs++] = jd;
         total += n;
+        stack_rows = std::max(stack_rows, (int)rq->r.dag->max_height);
     }
     static_assert(sizeof(dev::JobDesc) % 8 == 0, "the job table is copied in 8-byte words");
     if (rows_in || njobs) {
@@ -427,6 +430,8 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
         bl.block = cfg.block;
         bl.refill = cfg.refill_min;
         bl.counter_zeroed = true;
+        bl.stack_rows = stack_rows;
+        bl.shared_stack = batch_stack_in_shared(njobs, stack_rows, cfg.block);
         cbq_status st = launch_batch_kernel(s.d_table, njobs, total, s.d_counter,
                                             group[0]->r.dag->layout == CBQ_DAG_LAYOUT_COMPACT, device, s.stream, bl);
         if (st != CBQ_OK) return st;
@@ -581,7 +586,7 @@ cbq_status cbq_server_create(const cbq_server_config* cfg, cbq_server** out)
     if (c.max_batch_requests <= 0) c.max_batch_requests = 256;
     if (c.max_batch_rays == 0) c.max_batch_rays = 4ull << 20;
     if (c.block <= 0) c.block = 128;
-    if (c.refill_min == 0) c.refill_min = 8;
+    if (c.refill_min == 0) c.refill_min = 16;
     if (c.block > 256 || (c.block % 32) || c.refill_min > 32 || c.max_inflight_launches > 64 ||
         c.max_batch_requests > 65536 || (c.flags & ~(uint32_t)CBQ_SERVER_IN_PLACE)) {
         delete s;

@@ -34,12 +34,14 @@ struct SubDag {
 
 struct DagParams {
     const uint32_t* __restrict__ nodes;
+    uint32_t occupied;  // bit k: SubDAG k is not empty
     SubDag sd[8];
 };
 
 struct QueryParams {
     int32_t compute_surface;
     float max_footprint;
+    float footprint_tmax;  // footprint_exit_max(max_footprint): the ordered walk's form of the test
     uint32_t flags;
     uint32_t image_width;  // flat kernels: rays dealt in 4x8 tiles of an image this wide (0: in order)
 };
@@ -108,6 +110,21 @@ __device__ __forceinline__ uint32_t child_of(const uint32_t* __restrict__ nodes,
     }
 }
 
+// Child `slot` of a node given as the walk's own reference: in the reference
+// layout the word index of its first child (node * 8), in the compact one the
+// node reference itself.
+template <bool COMPACT>
+__device__ __forceinline__ uint32_t child_at(const uint32_t* __restrict__ nodes, uint32_t ref, uint32_t slot,
+                                             uint32_t& loads)
+{
+    if constexpr (COMPACT) {
+        return load_child_compact(nodes, ref, slot, loads);
+    } else {
+        loads++;
+        return __ldg(nodes + (ref | slot));
+    }
+}
+
 // Per-ray constants in the reflected frame.
 struct RayFrame {
     float ox, oy, oz;      // (origin + 0.5) * sign
@@ -132,32 +149,62 @@ __device__ __forceinline__ uint32_t first_child(const RayFrame& f, float entry, 
 // (raytracing.cpp:276).  With the LOD disabled (maxFootprint < 0) and a positive
 // exit the quotient is positive, so the division is skipped; every other case
 // divides exactly as the reference does.
-__device__ __forceinline__ bool large_footprint(int32_t cns, float t_exit, float mf)
+__device__ __forceinline__ bool large_footprint(float cns, float t_exit, float mf)
 {
     if (mf < 0.0f && t_exit > 0.0f) return true;
-    return ((float)cns / t_exit) > mf;
+    return (cns / t_exit) > mf;
+}
+__device__ __forceinline__ bool large_footprint(int32_t cns, float t_exit, float mf)
+{
+    return large_footprint((float)cns, t_exit, mf);
 }
 
 // Stack held in a per-thread local array (L1-resident).
 struct LocalStack {
     alignas(16) uint32_t slot[32];
     __device__ __forceinline__ void put(int h, uint32_t v) { slot[h & 31] = v; }
+    __device__ __forceinline__ uint32_t at(int h) const { return (uint32_t)h; }
+    __device__ __forceinline__ uint32_t below(uint32_t a) const { return a - 1u; }
+    __device__ __forceinline__ void store(uint32_t a, uint32_t v) { slot[a & 31u] = v; }
+    __device__ __forceinline__ uint32_t load(uint32_t a) const { return slot[a & 31u]; }
     __device__ __forceinline__ uint32_t get(int h) const { return slot[h & 31]; }
     // Zeroes every slot (eight 16-byte stores); `top` is for the shared form.
     __device__ __forceinline__ void clear(int /*top*/)
     {
 #pragma unroll
         for (int i = 0; i < 8; i++) reinterpret_cast<uint4*>(slot)[i] = make_uint4(0u, 0u, 0u, 0u);
+        // Keeps the array in memory: its indices are run-time values, and the
+        // compiler otherwise turned it into 32 registers and selects.
+        asm volatile("" ::"l"(slot) : "memory");
     }
 };
 
 // Stack held in shared memory, one column per thread: slot h at
 // base[(h - 1) * stride].  Heights run 1..max_height.
 struct SharedStack {
-    uint32_t* base;
-    uint32_t stride;
-    __device__ __forceinline__ void put(int h, uint32_t v) { base[(uint32_t)(h - 1) * stride] = v; }
-    __device__ __forceinline__ uint32_t get(int h) const { return base[(uint32_t)(h - 1) * stride]; }
+    uint32_t base;    // shared-memory address of the column's first slot
+    uint32_t stride;  // bytes between slots
+    __device__ __forceinline__ void init(uint32_t* column, uint32_t threads)
+    {
+        base = (uint32_t)__cvta_generic_to_shared(column);
+        stride = threads * 4u;
+    }
+    // Address of slot h, and of the slot below an address: the walks that keep
+    // the address of their current slot store and load without computing it.
+    __device__ __forceinline__ uint32_t at(int h) const { return base + (uint32_t)(h - 1) * stride; }
+    __device__ __forceinline__ uint32_t below(uint32_t a) const { return a - stride; }
+    __device__ __forceinline__ void store(uint32_t a, uint32_t v)
+    {
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v));
+    }
+    __device__ __forceinline__ uint32_t load(uint32_t a) const
+    {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+        return v;
+    }
+    __device__ __forceinline__ void put(int h, uint32_t v) { store(at(h), v); }
+    __device__ __forceinline__ uint32_t get(int h) const { return load(at(h)); }
     // Zeroes slots 1..top.
     __device__ __forceinline__ void clear(int top)
     {

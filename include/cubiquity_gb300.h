@@ -195,8 +195,8 @@ typedef struct cbq_launch_config {
     uint32_t refill_min;      /* flat persistent: idle lanes that trigger a refill, 0 = default */
     int32_t stack;            /* CBQ_STACK_* (flat kernel; shared by default) */
     int32_t form;             /* CBQ_FORM_*, used by cbq_intersect_auto */
-    int32_t steps;            /* flat kernel: ESVO steps per loop iteration (1..32, 16 by
-                                 default), 0 = 1 */
+    int32_t steps;            /* flat kernel: walk iterations between a warp's checks for
+                                 idle lanes (1..32, 8 by default), 0 = 1 */
     int32_t registers;        /* 0 (the default), or 56: the persistent local-stack
                                  kernel held to 56 registers per thread (more
                                  resident warps); other forms ignore it */
@@ -322,7 +322,7 @@ cbq_status cbq_batch_get_config(const cbq_batch* b, int32_t* block, uint32_t* re
 typedef struct cbq_batch_config {
     int32_t block;            /* threads per block: 32..256, a multiple of 32 */
     uint32_t refill_min;      /* idle lanes that trigger a warp's refill: 1..32 */
-    int32_t steps;            /* ESVO steps per loop iteration: 1..32 */
+    int32_t steps;            /* walk iterations between a warp's checks for idle lanes: 1..32 */
     int32_t registers;        /* 0, or 56: the local-stack kernel held to 56 registers */
     int32_t stack;            /* CBQ_STACK_LOCAL or CBQ_STACK_SHARED (descent stack placement) */
     int32_t form;             /* CBQ_FORM_PERSISTENT: rays in the order given; CBQ_FORM_SORTED: each
@@ -374,7 +374,7 @@ typedef struct cbq_server_config {
     int32_t max_batch_requests;     /* requests per launch (0 = 256) */
     uint64_t max_batch_rays;        /* rays per launch (0 = 4 Mi) */
     int32_t block;                  /* threads per block (0 = 128) */
-    uint32_t refill_min;            /* idle lanes that trigger a refill (0 = 8) */
+    uint32_t refill_min;            /* idle lanes that trigger a refill (0 = 16) */
     uint32_t flags;                 /* CBQ_SERVER_* */
 } cbq_server_config;
 
