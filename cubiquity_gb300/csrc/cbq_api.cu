@@ -39,6 +39,7 @@ FlatLaunch flat_launch(const cbq_dag* dag, bool persistent, uint64_t* counter, u
     return fl;
 }
 
+constexpr uint64_t kTaggedMaxNodes = 1ull << 24;  // a tagged reference holds 24 bits of node index
 constexpr int kPlainBlock = 128;
 constexpr int kPersistBlock = 256;
 constexpr uint32_t kDefaultChunk = 64;
@@ -225,6 +226,25 @@ __global__ void __launch_bounds__(kPersistBlock) cbq_k_intersect_persistent(
     }
 }
 
+// The tagged store (dev::Store::kTagged) of a reference node array: one word per
+// thread; a word that refers to an internal node reads that node's 32 bytes for
+// its occupancy mask.  The material slots stay as they are.
+__global__ void __launch_bounds__(256) cbq_k_tag_nodes(const uint4* __restrict__ nodes, uint64_t words,
+                                                       uint32_t* __restrict__ tagged)
+{
+    const uint32_t* w = (const uint32_t*)nodes;
+    for (uint64_t i = (uint64_t)blockIdx.x * 256u + threadIdx.x; i < words; i += (uint64_t)gridDim.x * 256u) {
+        uint32_t c = __ldg(w + i);
+        if (c >= dev::kMaterialCount) {
+            const uint4 a = __ldg(nodes + 2ull * c), b = __ldg(nodes + 2ull * c + 1u);
+            const uint32_t mask = (a.x ? 1u : 0u) | (a.y ? 2u : 0u) | (a.z ? 4u : 0u) | (a.w ? 8u : 0u) |
+                                  (b.x ? 16u : 0u) | (b.y ? 32u : 0u) | (b.z ? 64u : 0u) | (b.w ? 128u : 0u);
+            c = (c << 8) | mask;
+        }
+        tagged[i] = c;
+    }
+}
+
 namespace {
 
 cbq_status preload_nested_persistent()
@@ -292,10 +312,32 @@ cbq_status cbq_dag_create_ex(const uint32_t* host_nodes, uint64_t node_count, ui
         }
     }
     dag->device_bytes = bytes;
+    const bool tag = dag->flat_ok && dag->layout == CBQ_DAG_LAYOUT_REFERENCE && node_count <= kTaggedMaxNodes;
     cudaError_t e = cudaMalloc((void**)&dag->d_nodes, bytes);
     if (e != cudaSuccess) { cudaGetLastError(); delete dag; return CBQ_ERR_OUT_OF_MEMORY; }
     e = cudaMemcpy(dag->d_nodes, src, bytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { cudaFree(dag->d_nodes); delete dag; return CBQ_ERR_CUDA; }
+    if (tag && cudaMalloc((void**)&dag->d_tagged, bytes) != cudaSuccess) {
+        cudaGetLastError();  // without it the walk takes the reference layout
+        dag->d_tagged = nullptr;
+    }
+    if (dag->d_tagged) {
+        const uint64_t words = node_count * 8u;
+        cbq_k_tag_nodes<<<(unsigned)std::min<uint64_t>((words + 255) / 256, 1u << 20), 256, 0, cudaStreamLegacy>>>(
+            (const uint4*)dag->d_nodes, words, dag->d_tagged);
+        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
+            cudaFree(dag->d_nodes);
+            cudaFree(dag->d_tagged);
+            delete dag;
+            return CBQ_ERR_CUDA;
+        }
+        for (int i = 0; i < 8; i++) {
+            const uint32_t r = dag->subdags[i].node_index;
+            uint32_t mask = 0;
+            for (int k = 0; k < 8; k++) mask |= host_nodes[(uint64_t)r * 8 + k] != 0u ? 1u << k : 0u;
+            dag->tagged_ref[i] = r == 0u ? 0u : (r << 8) | mask;
+        }
+    }
     cbq::log(CBQ_LOG_INFO,
              "DAG uploaded to device %d: %llu nodes, %s layout (%.1f MB), root %u, max sub-DAG height %d, %s kernel",
              dag->device, (unsigned long long)node_count,
@@ -309,6 +351,7 @@ cbq_status cbq_dag_destroy(cbq_dag* dag)
 {
     if (!dag) return CBQ_ERR_INVALID_ARGUMENT;
     cudaFree(dag->d_nodes);
+    if (dag->d_tagged) cudaFree(dag->d_tagged);
     for (auto& kv : dag->stream_counters) cudaFree(kv.second);
     for (auto& hs : dag->stages) {
         if (hs->d_stage) cudaFree(hs->d_stage);
@@ -348,7 +391,7 @@ cbq_status cbq_dag_set_l2_persistence(const cbq_dag* dag, cbq_stream_t stream, f
         const size_t want = (size_t)((double)max_persist * fraction);
         if (cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, want) != cudaSuccess) return CBQ_ERR_CUDA;
         const size_t window = std::min<size_t>(dag->device_bytes, (size_t)max_window);
-        attr.accessPolicyWindow.base_ptr = dag->d_nodes;
+        attr.accessPolicyWindow.base_ptr = (void*)dag->walk_nodes();
         attr.accessPolicyWindow.num_bytes = window;
         attr.accessPolicyWindow.hitRatio = (float)std::min(1.0, (double)want / (double)window);
         attr.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;

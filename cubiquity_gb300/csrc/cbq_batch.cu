@@ -18,11 +18,12 @@
 namespace cbq {
 namespace dev {
 
-template <bool COMPACT>
+template <Store STORE>
 struct BatchSrc {
-    static constexpr bool kCompact = COMPACT;
+    static constexpr Store kStore = STORE;
     static constexpr bool kLod = true;      // each job has its own query
-    static constexpr bool kIntPos = false;  // jobs whose DAG needs integer positions run on their own
+    static constexpr bool kOrdered = true;
+    static constexpr bool kIntPos = false;  // such jobs run on their own (cbq_dag::batch_ok)
     const JobDesc* __restrict__ jobs;
 
     __device__ __forceinline__ const QueryParams& query(const Lane& L) const { return jobs[L.job].q; }
@@ -69,7 +70,7 @@ __device__ __forceinline__ void batch_body(const JobDesc* __restrict__ jobs, uin
     SharedStack sstack;
     sstack.init((uint32_t*)(prefix + njobs + 1) + threadIdx.x, blockDim.x);
 
-    BatchSrc<COMPACT> c;
+    BatchSrc<COMPACT ? Store::kCompact : Store::kTagged> c;
     c.jobs = jobs;
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t below = (1u << lane) - 1u;
@@ -116,7 +117,7 @@ __device__ __forceinline__ void batch_body(const JobDesc* __restrict__ jobs, uin
 }
 
 template <bool COMPACT, bool SHARED, bool SORTED>
-__global__ void __launch_bounds__(256, 5) cbq_k_flat_batch(const JobDesc* __restrict__ jobs, uint32_t njobs,
+__global__ void __launch_bounds__(256, 4) cbq_k_flat_batch(const JobDesc* __restrict__ jobs, uint32_t njobs,
                                                         uint64_t total, unsigned long long* __restrict__ counter,
                                                         uint32_t refill_min, uint32_t steps,
                                                         const uint32_t* __restrict__ perm)
@@ -197,16 +198,16 @@ __global__ void __launch_bounds__(256) cbq_k_batch_octant_scatter(const JobDesc*
 
 void fill_job_volume(dev::JobDesc& d, const cbq_dag* dag)
 {
-    d.nodes = dag->d_nodes;
+    d.nodes = dag->walk_nodes();
     d.occupied = 0u;
     for (int k = 0; k < 8; k++) {
-        if (dag->sd_ref[k] != 0u) d.occupied |= 1u << k;
+        if (dag->walk_root(k) != 0u) d.occupied |= 1u << k;
         const cbq_subdag& s = dag->subdags[k];
         d.sd[k].lx = s.lower_bound[0];
         d.sd[k].ly = s.lower_bound[1];
         d.sd[k].lz = s.lower_bound[2];
         d.sd[k].height = s.node_height;
-        d.sd[k].node = dag->sd_ref[k];
+        d.sd[k].node = dag->walk_root(k);
         d.sd[k].pad[0] = d.sd[k].pad[1] = d.sd[k].pad[2] = 0;
     }
 }
@@ -293,7 +294,7 @@ constexpr int32_t kBatchStepsDefault = 8;
 struct cbq_batch {
     int device = 0;
     std::vector<cbq_job> jobs;              // as given (host copy)
-    std::vector<int> nested_jobs;           // jobs whose DAG needs integer positions (launched on their own)
+    std::vector<int> nested_jobs;           // jobs whose DAG the batch kernel does not take (launched on their own)
     dev::JobDesc* d_jobs = nullptr;         // reference-layout jobs, then compact-layout jobs
     uint32_t njobs = 0;                     // jobs in the device table
     uint32_t njobs_ref = 0;                 // of which reference layout (one launch per layout)
@@ -470,7 +471,7 @@ cbq_status cbq_batch_create(const cbq_job* jobs, int32_t job_count, const cbq_qu
         }
         b->jobs.push_back(jb);
         if (jb.ray_count == 0) continue;
-        if (!jb.dag->flat_ok) { b->nested_jobs.push_back(j); continue; }
+        if (!jb.dag->batch_ok()) { b->nested_jobs.push_back(j); continue; }
         b->stack_rows = std::max(b->stack_rows, (int)jb.dag->max_height);
         dev::JobDesc d;
         std::memset(&d, 0, sizeof(d));
@@ -583,7 +584,7 @@ cbq_status cbq_batch_set_l2_persistence(cbq_batch* b, const cbq_dag* dag, float 
     if (max_window <= 0 || max_persist <= 0) return CBQ_OK;  // not supported: caching stays as it is
     const size_t want = (size_t)((double)max_persist * fraction);
     if (cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, want) != cudaSuccess) return CBQ_ERR_CUDA;
-    b->l2_base = dag->d_nodes;
+    b->l2_base = (void*)dag->walk_nodes();
     b->l2_bytes = std::min<size_t>(dag->device_bytes, (size_t)max_window);
     b->l2_hit_ratio = (float)std::min(1.0, (double)want / (double)b->l2_bytes);
     return CBQ_OK;

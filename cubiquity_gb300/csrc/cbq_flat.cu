@@ -72,7 +72,7 @@ __device__ __forceinline__ void flat_body(const Ctx& c, uint64_t n, unsigned lon
 }
 
 template <bool PERSISTENT, bool SHARED, bool SORTED, typename Ctx>
-__global__ void __launch_bounds__(256, PERSISTENT && !Ctx::kIntPos ? 5 : 4) cbq_k_flat(Ctx c, uint64_t n, unsigned long long* __restrict__ counter,
+__global__ void __launch_bounds__(256, 4) cbq_k_flat(Ctx c, uint64_t n, unsigned long long* __restrict__ counter,
                                                   uint32_t refill_min, const uint32_t* __restrict__ perm,
                                                   uint32_t steps)
 {
@@ -167,6 +167,19 @@ bool float_positions_exact(const cbq_dag* dag)
 
 namespace {
 
+// The single-volume contexts: tagged and compact stores, with and without LOD;
+// plain stores of 2^24 nodes or more; integer positions.
+template <bool LOD>
+using TaggedCtx = dev::FlatCtxT<dev::Store::kTagged, false, false, LOD>;
+template <bool LOD>
+using CompactCtx = dev::FlatCtxT<dev::Store::kCompact, false, false, LOD>;
+using PlainCtx = dev::FlatCtxT<dev::Store::kPlain, false, false, true>;
+using IntCtx = dev::FlatCtxT<dev::Store::kPlain, false, true>;
+// The fetch-count pass.
+using CountCompactCtx = dev::FlatCtxT<dev::Store::kCompact, true, false, true>;
+using CountPlainCtx = dev::FlatCtxT<dev::Store::kPlain, true, false, true>;
+using CountIntCtx = dev::FlatCtxT<dev::Store::kPlain, true, true>;
+
 template <typename Ctx>
 bool query_persistent_kernels()
 {
@@ -186,8 +199,9 @@ bool query_persistent_kernels()
 // memory).  Done for every persistent traversal kernel when a DAG is created.
 cbq_status preload_persistent_kernels()
 {
-    const bool ok = query_persistent_kernels<dev::FlatCtxT<false>>() && query_persistent_kernels<dev::FlatCtxT<true>>() &&
-                    query_persistent_kernels<dev::FlatCtxT<false, false, true>>();
+    const bool ok = query_persistent_kernels<TaggedCtx<false>>() && query_persistent_kernels<TaggedCtx<true>>() &&
+                    query_persistent_kernels<CompactCtx<false>>() && query_persistent_kernels<CompactCtx<true>>() &&
+                    query_persistent_kernels<PlainCtx>() && query_persistent_kernels<IntCtx>();
     if (!ok) cudaGetLastError();
     return ok ? CBQ_OK : CBQ_ERR_CUDA;
 }
@@ -291,27 +305,29 @@ cbq_status launch_flat(const cbq_dag* dag, const dev::DagParams& dp, const dev::
         one.local_stack = true;
         one.perm = nullptr;
         if (dag->layout == CBQ_DAG_LAYOUT_COMPACT)
-            return launch_variant<false, false, false>(
-                make_ctx<dev::FlatCtxT<true, true, false, true>>(dp, q, out, orig, dir, fetch_out), n, one, rows, stream, dv);
+            return launch_variant<false, false, false>(make_ctx<CountCompactCtx>(dp, q, out, orig, dir, fetch_out), n,
+                                                       one, rows, stream, dv);
         if (!dag->flat_ok)
-            return launch_variant<false, false, false>(
-                make_ctx<dev::FlatCtxT<false, true, true>>(dp, q, out, orig, dir, fetch_out), n, one, rows, stream,
-                dv);
-        return launch_variant<false, false, false>(
-            make_ctx<dev::FlatCtxT<false, true, false, true>>(dp, q, out, orig, dir, fetch_out), n, one, rows, stream, dv);
+            return launch_variant<false, false, false>(make_ctx<CountIntCtx>(dp, q, out, orig, dir, fetch_out), n, one,
+                                                       rows, stream, dv);
+        return launch_variant<false, false, false>(make_ctx<CountPlainCtx>(dp, q, out, orig, dir, fetch_out), n, one,
+                                                   rows, stream, dv);
     }
     const bool lod = !(q.max_footprint < 0.0f);
     if (dag->layout == CBQ_DAG_LAYOUT_COMPACT)
-        return lod ? launch_ctx(make_ctx<dev::FlatCtxT<true, false, false, true>>(dp, q, out, orig, dir, nullptr), n,
-                                fl, rows, stream, dv)
-                   : launch_ctx(make_ctx<dev::FlatCtxT<true>>(dp, q, out, orig, dir, nullptr), n, fl, rows, stream,
-                                dv);
+        return lod ? launch_ctx(make_ctx<CompactCtx<true>>(dp, q, out, orig, dir, nullptr), n, fl, rows, stream, dv)
+                   : launch_ctx(make_ctx<CompactCtx<false>>(dp, q, out, orig, dir, nullptr), n, fl, rows, stream, dv);
     if (!dag->flat_ok)  // coordinates beyond +-2^21 or 2^29 nodes or more: integer positions
-        return launch_ctx(make_ctx<dev::FlatCtxT<false, false, true>>(dp, q, out, orig, dir, nullptr), n, fl, rows,
-                          stream, dv);
-    return lod ? launch_ctx(make_ctx<dev::FlatCtxT<false, false, false, true>>(dp, q, out, orig, dir, nullptr), n, fl,
-                            rows, stream, dv)
-               : launch_ctx(make_ctx<dev::FlatCtxT<false>>(dp, q, out, orig, dir, nullptr), n, fl, rows, stream, dv);
+        return launch_ctx(make_ctx<IntCtx>(dp, q, out, orig, dir, nullptr), n, fl, rows, stream, dv);
+    if (dag->d_tagged) {
+        dev::DagParams tagged = dp;
+        tagged.nodes = dag->d_tagged;
+        for (int k = 0; k < 8; k++) tagged.sd[k].node = dag->tagged_ref[k];
+        return lod ? launch_ctx(make_ctx<TaggedCtx<true>>(tagged, q, out, orig, dir, nullptr), n, fl, rows, stream, dv)
+                   : launch_ctx(make_ctx<TaggedCtx<false>>(tagged, q, out, orig, dir, nullptr), n, fl, rows, stream,
+                                dv);
+    }
+    return launch_ctx(make_ctx<PlainCtx>(dp, q, out, orig, dir, nullptr), n, fl, rows, stream, dv);
 }
 
 }  // namespace cbq

@@ -57,21 +57,22 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b)
 
 // What a lane keeps of its ray and walk.  Registers decide how many warps an SM
 // holds: the ray itself, the octant distances and a finished ray's results are
-// read or computed again where they are needed (48 registers a thread, 40 warps
-// an SM, instead of 64 and 32).
+// read or computed again where they are needed (56 registers a thread, 36 warps
+// an SM, instead of 64 and 32).  Held to 48 registers the walk spills and was
+// slower (bounce rays 562 against 549 us, camera rays 362 against 345).
 struct Lane {
     float rox, roy, roz;         // reflected origin
     float ix, iy, iz;            // 1 / |dir|
     uint32_t sign, oct, moves;   // octant (reflected) and how many octant transitions led to it
     // ESVO walk state
-    uint32_t node, cid;
+    uint32_t node, cid;          // ordered walk: `cid` is the child slot (child id ^ sign)
     int32_t cns;                 // child size (integer-position form)
     float fx, fy, fz, fcns;      // child position and size as exact floats (float-position form)
     int32_t px, py, pz;          // child position as wrapping i32 (integer-position form)
     int h;                       // height of `node`; ordered walk: its stack address
     uint32_t limit;              // size of the SubDAG
-    float last_exit;             // ordered walk: max(entry distance of the child cell, FLT_MIN)
-    uint32_t fetches, mode;
+    float last_exit;             // ordered walk: the entry distance of the child cell
+    uint32_t fetches, mode;      // ordered walk: `fetches` is an upper bound
     bool fast;                   // float positions: the ordered walk applies; integer positions: no slab
                                  // distance can be NaN or -0, so min/max need no NaN ordering
     uint32_t loads;              // node loads made (fetches minus skipped empty children)
@@ -82,14 +83,14 @@ struct Lane {
 
 // Where a lane's volume, rays and outputs are.  The lane functions below are
 // templates over this "source" so that the single-volume kernel and the
-// multi-volume batch kernel share the same arithmetic.  COMPACT selects the
-// node store layout; COUNT_LOADS is the fetch-count pass (cbq_count_fetches),
+// multi-volume batch kernel share the same arithmetic.  STORE is how
+// they refer to nodes; COUNT_LOADS is the fetch-count pass (cbq_count_fetches),
 // which writes per ray the node loads (child probes in the reference layout,
 // fewer in the compact one) to fetch_out.  It is a separate instantiation, so
 // the traversal kernels carry no counting code (measured: 1-2% faster).
-template <bool COMPACT, bool COUNT_LOADS = false, bool INT_POS = false, bool LOD = false>
+template <Store STORE, bool COUNT_LOADS = false, bool INT_POS = false, bool LOD = false>
 struct FlatCtxT {
-    static constexpr bool kCompact = COMPACT;
+    static constexpr Store kStore = STORE;
     // INT_POS: child positions as wrapping i32 converted to float where a slab
     // plane is needed (the reference's own arithmetic, any coordinates, 64-bit
     // node offsets); otherwise exact floats (coordinates within +-2^21, fewer
@@ -98,6 +99,8 @@ struct FlatCtxT {
     // LOD: the query may stop at a footprint (max_footprint >= 0); without it
     // the ordered walk leaves the test out.
     static constexpr bool kLod = LOD;
+    // The fetch-count pass takes the reference form only: the ordered walk does not count.
+    static constexpr bool kOrdered = !COUNT_LOADS && !INT_POS;
     DagParams dag;
     QueryParams q;
     HitsOut out;
@@ -128,7 +131,7 @@ struct FlatCtxT {
     __device__ __forceinline__ void write(const Lane& L, const RayResult& r) const
     {
         write_result(out, L.ray, r);
-        if constexpr (COUNT_LOADS) fetch_out[L.ray] = COMPACT ? L.loads : L.fetches;
+        if constexpr (COUNT_LOADS) fetch_out[L.ray] = STORE == Store::kCompact ? L.loads : L.fetches;
     }
 };
 
@@ -205,8 +208,9 @@ struct OctantWalk {
 };
 
 // Per-ray set-up: intersectVolume up to the octant loop (raytracing.cpp:409-434).
+// `ordered` false: by the reference form, whatever the ray.
 template <typename Src>
-__device__ __forceinline__ void lane_begin(Lane& L, const Src& c, uint64_t i)
+__device__ __forceinline__ void lane_begin(Lane& L, const Src& c, uint64_t i, bool ordered = true)
 {
     L.ray = i;
     const float4 o = c.ray_origin(L, i);
@@ -232,7 +236,8 @@ __device__ __forceinline__ void lane_begin(Lane& L, const Src& c, uint64_t i)
         L.fast = rdx >= FLT_MIN && rdy >= FLT_MIN && rdz >= FLT_MIN && fabsf(L.rox) <= FLT_MAX &&
                  fabsf(L.roy) <= FLT_MAX && fabsf(L.roz) <= FLT_MAX;
     } else {
-        L.fast = ordered_axis(rdx, L.rox) && ordered_axis(rdy, L.roy) && ordered_axis(rdz, L.roz);
+        L.fast = Src::kOrdered && ordered && ordered_axis(rdx, L.rox) && ordered_axis(rdy, L.roy) &&
+                 ordered_axis(rdz, L.roz);
     }
     // The octant of the origin: distToOrigin = -o' / |dir| below 0
     // (raytracing.cpp:424-434), which is o' > 0 for an ordered ray.
@@ -283,7 +288,7 @@ __device__ __forceinline__ void flush_held(Lane& L, const Src& c)
         const float tce = max3_ref(c0x, c0y, c0z);
         uint32_t material = 0u;
         if (c.query(L).compute_surface)
-            material = nearest_material<Src::kCompact, INT>(c.nodes(L), L.node, L.sign, L.fetches, r.status, L.loads);
+            material = nearest_material<Src::kStore, INT>(c.nodes(L), L.node, L.sign, L.fetches, r.status, L.loads);
         if (r.status == kRayOk && !((c.query(L).flags & 1u) && !(tce <= o.w))) {
             r.hit = true;
             r.distance = tce;
@@ -340,6 +345,36 @@ __device__ __forceinline__ void lane_next(Lane& L, const Src& c)
     L.mode = kLaneEnter;
 }
 
+// Whether a child exists, and the child (0 where it does not), in the ordered
+// walk, whose references to plain nodes are word indices (node * 8).  Plain and
+// tagged stores hold a 0 for an empty child, so it is loaded like any other: a
+// test or a branch around the load costs more.
+template <Store S>
+__device__ __forceinline__ bool walk_occupied(const uint32_t* __restrict__ nodes, uint32_t ref, uint32_t slot)
+{
+    if constexpr (S == Store::kPlain)
+        return __ldg(nodes + (ref | slot)) != 0u;
+    else
+        return ((ref >> slot) & 1u) != 0u;
+}
+template <Store S>
+__device__ __forceinline__ uint32_t walk_child(const uint32_t* __restrict__ nodes, uint32_t ref, uint32_t slot)
+{
+    if constexpr (S == Store::kPlain) {
+        return __ldg(nodes + (ref | slot));
+    } else if constexpr (S == Store::kTagged) {
+        uint32_t child;
+        asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; mov.u32 %0, 0; @p ld.global.nc.u32 %0, [%1]; }"
+                     : "=r"(child) : "l"(occupied_at<S>(nodes, ref, slot)), "r"((ref >> slot) & 1u));
+        return child;
+    } else {
+        uint32_t child;
+        asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; mov.u32 %0, 0; @p ld.global.nc.u32 %0, [%1]; }"
+                     : "=r"(child) : "l"(occupied_at<S>(nodes, ref, slot)), "r"((ref >> slot) & 1u));
+        return child;
+    }
+}
+
 // Enters the SubDAG of the current octant: the slab test and set-up at the top
 // of intersectRayNodeESVO (raytracing.cpp:218-250, 443-460).
 template <typename Src, typename Stack>
@@ -387,11 +422,12 @@ __device__ __forceinline__ void lane_enter(Lane& L, const Src& c, Stack& stack)
         L.fy = fpy + ((L.cid & 2u) ? L.fcns : 0.0f);
         L.fz = fpz + ((L.cid & 4u) ? L.fcns : 0.0f);
         if (L.fast) {
-            L.last_exit = fmaxf(entry, FLT_MIN);
+            L.last_exit = entry;
+            L.cid ^= L.sign;
             L.fx += kPosBias;
             L.fy += kPosBias;
             L.fz += kPosBias;
-            if (!Src::kCompact) L.node *= 8u;
+            if (Src::kStore == Store::kPlain) L.node *= 8u;  // the word index of its children
             L.h = (int)stack.at(s.height);
             if (s.height > 0) stack.store((uint32_t)L.h, L.node);
             // Origin inside the SubDAG: descend to the cell that holds it here,
@@ -399,27 +435,30 @@ __device__ __forceinline__ void lane_enter(Lane& L, const Src& c, Stack& stack)
             // entry <= 0 < tChildExit, so the first child is the one that holds
             // the origin and no distance is needed (terrain-4096 bounce rays:
             // 8.9 of 18 descents; 774 -> 744 us when it was added).
-            if (entry <= 0.0f && exit_ > 0.0f && L.fetches == 0u && (!Src::kLod || c.query(L).max_footprint < 0.0f)) {
-                for (;;) {
-                    const uint32_t child = child_at<Src::kCompact>(c.nodes(L), L.node, L.cid ^ L.sign, L.loads);
-                    if (child < kMaterialCount) {  // fetched again by the walk
-                        if (child != 0u) L.loads--;
-                        break;
+            if (entry <= 0.0f && exit_ > 0.0f) {
+                const uint32_t* nodes = c.nodes(L);
+                while (walk_occupied<Src::kStore>(nodes, L.node, L.cid)) {
+                    if constexpr (Src::kLod) {
+                        const float sb = L.fcns - kPosBias;
+                        const float tcx = fminf(fminf(((L.fx + sb) - L.rox) * L.ix, ((L.fy + sb) - L.roy) * L.iy),
+                                                ((L.fz + sb) - L.roz) * L.iz);
+                        if (!(tcx <= L.fcns * c.query(L).footprint_tmax)) break;
                     }
-                    L.fetches++;
-                    L.node = Src::kCompact ? child : child * 8u;
+                    const uint32_t child = walk_child<Src::kStore>(nodes, L.node, L.cid);
+                    if (child < kMaterialCount) break;  // fetched again by the walk
+                    L.node = Src::kStore == Store::kPlain ? child * 8u : child;
                     L.h = (int)stack.below((uint32_t)L.h);
                     stack.store((uint32_t)L.h, L.node);
                     L.fcns *= 0.5f;
                     const float sb = L.fcns - kPosBias;
                     const bool bx = L.rox >= L.fx + sb, by = L.roy >= L.fy + sb, bz = L.roz >= L.fz + sb;
-                    L.cid = (uint32_t)bx | ((uint32_t)by << 1) | ((uint32_t)bz << 2);
+                    L.cid = ((uint32_t)bx | ((uint32_t)by << 1) | ((uint32_t)bz << 2)) ^ L.sign;
                     if (bx) L.fx += L.fcns;
                     if (by) L.fy += L.fcns;
                     if (bz) L.fz += L.fcns;
                 }
             }
-            L.fetches++;
+            L.fetches += 64u;  // more than were made here
         } else {
             L.last_exit = exit_;
             L.h = s.height;
@@ -447,14 +486,14 @@ __device__ __forceinline__ float slab_max3(float x, float y, float z)
 // slab distances are strictly increasing along each axis (ordered_axis).  It
 // takes the reference's decisions, cell by cell and fetch by fetch, with fewer
 // operations:
-//  - The entry distance E = max3(childT0) is carried (as max(E, FLT_MIN), in
-//    last_exit) instead of recomputed.  A descent keeps it: the entry axis's
-//    centre plane lies beyond E, so its bit stays 0, and E <= 0 stays <= 0.  An
-//    advance makes it tChildExit, which no entry distance of the child exceeds
-//    unless both are <= 0.
-//  - findFirstChild's two tests are one: where E <= 0 the behind-origin test
-//    o' >= centre is "centre distance <= 0", and no distance lies strictly
-//    between 0 and FLT_MIN, so both are "centre distance < max(E, FLT_MIN)".
+//  - The entry distance E = max3(childT0) is carried (in last_exit) instead of
+//    recomputed.  A descent at E > 0 keeps it: the entry axis's centre plane
+//    lies beyond E, so its bit stays 0.  An advance makes it tChildExit, which
+//    no entry distance of the child exceeds unless both are <= 0.
+//  - findFirstChild is one compare per axis where E > 0.  Where E <= 0 < exit
+//    the origin lies in the cell, and the first child is the one that holds it
+//    (lane_enter).  Where both are <= 0 the SubDAG lies behind the origin; such
+//    rays start again in the reference form at their first descent.
 //  - A descent always stores its node.  The reference skips the store when
 //    tChildExit equals the node's own exit; the child then shares the node's
 //    exit plane, and a walk that leaves the child through it pops past the
@@ -466,6 +505,12 @@ __device__ __forceinline__ float slab_max3(float x, float y, float z)
 //    size is subtracted from the bias instead (sb), which is exact.
 //  - max_footprint: see footprint_exit_max, one compare instead of a division
 //    (which the compiler had moved out of its branch: 12 instructions a step).
+//  - References carry their node's occupancy mask (Store), so that an empty
+//    child costs no load: 18 loads per terrain-4096 bounce ray instead of 37
+//    (bounce rays 592 -> 545 us; the compact store's 196 -> 156).  Loading empty
+//    children too, without a test, was slower (575 us).
+//  - Fetches are not counted: an upper bound decides when a ray may come near
+//    the fetch cap.
 //
 // One iteration is an advance, if the child is empty, and then a descent, if
 // the child reached is not.  Both sections run in nearly every iteration of an
@@ -473,96 +518,77 @@ __device__ __forceinline__ float slab_max3(float x, float y, float z)
 // price of one: 16.5 iterations per terrain-4096 bounce ray instead of 30.8
 // steps.  The x and y planes are computed with packed instructions, and the
 // axis bits move positions and form the child id through multiply-adds, off the
-// integer pipe.  Bound by instruction issue and the latency of its two
-// dependent loads (70-74% of issue slots, 15.5 / 23.5 active lanes per
-// instruction on incoherent / coherent rays).  With the forms it replaced, in
-// Grays/s: terrain-4096 camera rays 6.9 -> 11.3, bounce rays 3.8 -> 6.8.
-
-// In an ordered lane, `fetches` counts the fetch of the current cell's child
-// from the moment the cell is reached.
-
-// Hands a lane over to the reference form for the rest of its ray, at the
-// current cell.  The reference form stores on its next descent (last_exit
-// infinite) and then carries on as if it had walked all along.
-__device__ __forceinline__ void lane_to_reference(Lane& L, bool compact)
-{
-    L.fast = false;
-    L.fetches--;
-    L.h = 32 - __clz((uint32_t)L.fcns);
-    if (!compact) L.node >>= 3;
-    L.fx -= kPosBias;
-    L.fy -= kPosBias;
-    L.fz -= kPosBias;
-    L.last_exit = __int_as_float(0x7f800000);
-}
+// integer pipe.  Bound by instruction issue (76% of issue slots, the ALU pipe
+// 62%) and the latency of a dependent load (16 / 24 active lanes per
+// instruction on incoherent / coherent rays).  4 Mi rays on terrain-4096, from
+// the reference's steps: camera rays 607 -> 343 us, bounce rays 1,100 -> 545 us.
 
 // Up to `steps` iterations of a walking ordered lane.
 template <typename Src, typename Stack>
 __device__ __forceinline__ void lane_walk_ordered(Lane& L, const Src& c, Stack& stack, uint32_t steps)
 {
-    const float tmax1 = Src::kLod ? c.query(L).footprint_tmax : 0.0f;
-    // One or two fetches per iteration: within two of the fetch cap the
-    // reference form counts them one by one.
-    const uint32_t budget = (kMaxFetches - L.fetches) >> 1;
-    if (budget == 0u) {
-        lane_to_reference(L, Src::kCompact);
+    constexpr Store S = Src::kStore;
+    // At most two fetches per iteration, and a hit's material within 512 more.
+    // A ray that may come near the fetch cap starts again in the reference
+    // form, which counts every fetch.
+    L.fetches += 2u * steps;
+    if (L.fetches + 512u >= kMaxFetches) {
+        lane_begin(L, c, L.ray, false);
         return;
     }
-    uint32_t left = steps < budget ? steps : budget;
-    uint32_t child;
-    float tcx;
-    bool down;
-    float sb = L.fcns - kPosBias;
+    const float tmax1 = Src::kLod ? c.query(L).footprint_tmax : 0.0f;
     const float2 nro = make_float2(-L.rox, -L.roy), inv = make_float2(L.ix, L.iy);
     const uint32_t* nodes = c.nodes(L);
+    float sb = L.fcns - kPosBias;
+    uint32_t child;
+    bool stopped;
     do {
-        float2 c1 = mul2(add2(add2(make_float2(L.fx, L.fy), make_float2(sb, sb)), nro), inv);
-        float c1z = ((L.fz + sb) - L.roz) * L.iz;
-        tcx = fminf(fminf(c1.x, c1.y), c1z);
-        child = child_at<Src::kCompact>(nodes, L.node, L.cid ^ L.sign, L.loads);
-        if (child == 0u) {
+        if (!walk_occupied<S>(nodes, L.node, L.cid)) {
+            const float2 c1 = mul2(add2(add2(make_float2(L.fx, L.fy), make_float2(sb, sb)), nro), inv);
+            const float c1z = ((L.fz + sb) - L.roz) * L.iz;
+            const float tcx = fminf(fminf(c1.x, c1.y), c1z);
+            L.last_exit = tcx;
             const float nx = __fmaf_rn(c1.x <= tcx ? 1.0f : 0.0f, L.fcns, L.fx);
             const float ny = __fmaf_rn(c1.y <= tcx ? 1.0f : 0.0f, L.fcns, L.fy);
             const float nz = __fmaf_rn(c1z <= tcx ? 1.0f : 0.0f, L.fcns, L.fz);
             const uint32_t cx = __float_as_uint(nx), cy = __float_as_uint(ny), cz = __float_as_uint(nz);
             const uint32_t diff = (cx ^ __float_as_uint(L.fx)) | (cy ^ __float_as_uint(L.fy)) |
                                   (cz ^ __float_as_uint(L.fz));
-            const bool inside = diff < L.limit;
-            L.last_exit = fmaxf(tcx, FLT_MIN);
             const int msb = 31 - __clz(diff);
             const uint32_t m = 1u << msb;
             const uint32_t keep = 0u - m;
+            L.cid = (((cx & m) + ((cy & m) << 1) + ((cz & m) << 2)) >> msb) ^ L.sign;
             L.h = (int)stack.at(msb + 1);
-            L.node = 0u;  // outside the SubDAG: the empty node, which ends the loop
-            if (inside) L.node = stack.load((uint32_t)L.h);
-            L.cid = ((cx & m) + ((cy & m) << 1) + ((cz & m) << 2)) >> msb;
+            // Outside the SubDAG: the empty node, and the loop's last iteration.
+            const bool inside = diff < L.limit;
+            L.node = stack.load_if((uint32_t)L.h, inside, 0u);
+            if (!inside) steps = 1u;
             L.fcns = __uint_as_float((uint32_t)(127 + msb) << 23);  // 2^msb
             sb = L.fcns - kPosBias;
             L.fx = __uint_as_float(cx & keep);
             L.fy = __uint_as_float(cy & keep);
             L.fz = __uint_as_float(cz & keep);
-            if constexpr (Src::kLod) {
-                c1 = mul2(add2(add2(make_float2(L.fx, L.fy), make_float2(sb, sb)), nro), inv);
-                c1z = ((L.fz + sb) - L.roz) * L.iz;
-                tcx = fminf(fminf(c1.x, c1.y), c1z);
-            }
-            child = child_at<Src::kCompact>(nodes, L.node, L.cid ^ L.sign, L.loads);
-            L.fetches++;
         }
         // The value is opaque here, so that lanes that did not advance wait for
         // the others: the compiler otherwise sent them straight to their
         // descent, which then ran twice (1,086 instead of 960 us, bounce rays).
-        // The same below for the loop's end, where it gave descending lanes a
-        // loop of their own (1,523 instead of 592 us).
-        asm volatile("" : "+r"(child));
-        // hasLargeFootprint (raytracing.cpp:276).  Without LOD a child whose
-        // exit is not behind the origin is large; an advance only moves the
-        // exit on, so the exit of the cell before it will do.
-        const bool large = tcx >= 0.0f && (!Src::kLod || tcx <= L.fcns * tmax1);
-        down = child >= kMaterialCount && large;
+        // A loop whose condition the compiler can tell from `down` has the same
+        // fault at its end (1,523 instead of 592 us): `steps` is all it tests.
+        asm volatile("" : "+r"(L.node));
+        child = walk_child<S>(nodes, L.node, L.cid);
+        // hasLargeFootprint (raytracing.cpp:276).  Without LOD every child is
+        // large whose exit is not behind the origin, which an entry beyond it
+        // ensures.  Cells with an entry at or behind the origin are left to the
+        // reference form (those that hold the origin were passed on entering).
+        bool down = child >= kMaterialCount && L.last_exit > 0.0f;
+        if constexpr (Src::kLod) {
+            const float2 c1 = mul2(add2(add2(make_float2(L.fx, L.fy), make_float2(sb, sb)), nro), inv);
+            const float tcx = fminf(fminf(c1.x, c1.y), ((L.fz + sb) - L.roz) * L.iz);
+            down = down && tcx <= L.fcns * tmax1;
+        }
+        stopped = child != 0u && !down;
         if (down) {
-            L.fetches++;
-            L.node = Src::kCompact ? child : child * 8u;
+            L.node = S == Store::kPlain ? child * 8u : child;
             L.h = (int)stack.below((uint32_t)L.h);
             stack.store((uint32_t)L.h, L.node);
             L.fcns *= 0.5f;
@@ -573,27 +599,20 @@ __device__ __forceinline__ void lane_walk_ordered(Lane& L, const Src& c, Stack& 
             const float bx = mm.x < te ? 1.0f : 0.0f, by = mm.y < te ? 1.0f : 0.0f, bz = mz < te ? 1.0f : 0.0f;
             // The three bits as the low bits of a subnormal: 2^-149, 2^-148, 2^-147.
             L.cid = __float_as_uint(__fmaf_rn(bz, __uint_as_float(4u), __fmaf_rn(by, __uint_as_float(2u),
-                                              bx * __uint_as_float(1u))));
+                                              bx * __uint_as_float(1u)))) ^ L.sign;
             L.fx = __fmaf_rn(bx, L.fcns, L.fx);
             L.fy = __fmaf_rn(by, L.fcns, L.fy);
             L.fz = __fmaf_rn(bz, L.fcns, L.fz);
         }
-        uint32_t go = down || (child == 0u && L.node != 0u);
-        asm volatile("" : "+r"(go));
-        if (go == 0u) break;
-    } while (--left != 0u);
-    if (down) return;
-    if (child != 0u) {
-        if (child >= kMaterialCount && tcx < 0.0f && (!Src::kLod || c.query(L).max_footprint < 0.0f)) {
-            L.loads--;  // the reference form fetches this child again
-            lane_to_reference(L, Src::kCompact);
-        } else {
-            L.node = child;  // a hit at this child
-            L.mode = kLaneHit;
-        }
-    } else if (L.node == 0u) {  // left the SubDAG: on to the next octant
-        L.fetches--;            // without a child to fetch
-        L.mode = kLaneNext;
+        steps = stopped ? 0u : steps - 1u;
+    } while (steps != 0u);
+    if (!stopped) {
+        if (L.node == 0u) L.mode = kLaneNext;  // left the SubDAG
+    } else if (child >= kMaterialCount && !(L.last_exit > 0.0f)) {
+        lane_begin(L, c, L.ray, false);
+    } else {
+        L.node = child;  // a hit at this child
+        L.mode = kLaneHit;
     }
 }
 
@@ -607,7 +626,7 @@ __device__ __forceinline__ void lane_walk(Lane& L, const Src& c, Stack& stack)
     const float c1y = ((INT ? (float)wadd(L.py, L.cns) : L.fy + L.fcns) - L.roy) * L.iy;
     const float c1z = ((INT ? (float)wadd(L.pz, L.cns) : L.fz + L.fcns) - L.roz) * L.iz;
     const float tcx = slab_min3<FAST>(c1x, c1y, c1z);
-    const uint32_t child = child_of<Src::kCompact, INT>(c.nodes(L), L.node, L.cid ^ L.sign, L.loads);
+    const uint32_t child = child_of<Src::kStore, INT>(c.nodes(L), L.node, L.cid ^ L.sign, L.loads);
     L.fetches++;
     if (child > 0u) {
         if (child >= kMaterialCount && large_footprint(INT ? (float)L.cns : L.fcns, tcx, c.query(L).max_footprint)) {
@@ -723,9 +742,10 @@ __device__ __forceinline__ void lane_walk_steps(Lane& L, const Src& c, Stack& st
 }
 
 // The walk of a whole warp (all 32 lanes must call it), then the results of
-// the rays that finished in it are written.  Float positions: each lane's ray
-// takes the ordered walk or the reference's forms for its whole life.  Integer
-// positions: the FAST min/max when every walking lane's ray allows it.
+// the rays that finished in it are written.  Float positions: ordered lanes walk
+// until `idle_min` of the warp's lanes do not (checked every `steps`
+// iterations), the others take up to `steps` steps of the reference form.
+// Integer positions: the FAST min/max when every walking lane's ray allows it.
 template <typename Src, typename Stack>
 __device__ __forceinline__ void warp_walk_steps(Lane& L, const Src& c, Stack& stack, uint32_t steps,
                                                 uint32_t idle_min)

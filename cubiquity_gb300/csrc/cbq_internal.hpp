@@ -90,6 +90,15 @@ struct cbq_dag {
     uint32_t layout = CBQ_DAG_LAYOUT_REFERENCE;
     uint64_t device_bytes = 0;     // size of the device node store
     uint32_t sd_ref[8] = {};       // SubDAG roots as the device store refers to them
+    // The store of the flat kernels' float form where d_nodes is the reference layout and has
+    // fewer than 2^24 nodes: a copy of it whose references carry occupancy masks (made on the
+    // device by cbq_dag_create; null where there is none), and the SubDAG roots in it.
+    uint32_t* d_tagged = nullptr;
+    uint32_t tagged_ref[8] = {};
+    const uint32_t* walk_nodes() const { return d_tagged ? d_tagged : d_nodes; }
+    uint32_t walk_root(int k) const { return d_tagged ? tagged_ref[k] : sd_ref[k]; }
+    // The batch kernel takes tagged and compact stores; other DAGs are launched on their own.
+    bool batch_ok() const { return flat_ok && (d_tagged || layout == CBQ_DAG_LAYOUT_COMPACT); }
     uint64_t node_count = 0;
     uint32_t root = 0;
     cbq_subdag subdags[8];

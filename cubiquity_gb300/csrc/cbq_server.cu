@@ -401,7 +401,7 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
             }
         }
         rq->job = jd;
-        if (!rq->r.dag->flat_ok) continue;  // integer positions (far coordinates, huge stores): launched on its own
+        if (!rq->r.dag->batch_ok()) continue;  // far coordinates, huge stores: launched on its own
         jd.first = total;
         s.h_table[njobs++] = jd;
         total += n;
@@ -417,7 +417,7 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
         if (cudaGetLastError() != cudaSuccess) return CBQ_ERR_CUDA;
     }
     for (Request* rq : group) {
-        if (rq->r.dag->flat_ok) continue;
+        if (rq->r.dag->batch_ok()) continue;
         const dev::JobDesc& jd = rq->job;
         cbq_rays rays{(const float*)jd.orig, (const float*)jd.dir};
         cbq_hits hits{jd.out.hit, jd.out.distance, jd.out.material, jd.out.position, jd.out.normal, jd.out.voxel,

@@ -84,44 +84,41 @@ __device__ __forceinline__ uint32_t load_child32(const uint32_t* __restrict__ no
     return __ldg(nodes + (node * 8u + slot));
 }
 
-// Child `slot` of node reference `node` in the compact store (the occupancy
-// mask is the reference's low byte, the packed children start at unit
-// node >> 8 of 8 bytes): an empty child costs no load.  `loads` counts loads.
-__device__ __forceinline__ uint32_t load_child_compact(const uint32_t* __restrict__ nodes, uint32_t node,
-                                                       uint32_t slot, uint32_t& loads)
+// How a walk refers to nodes and finds their children.
+//   kPlain:   the reference's node array; a reference is the node's index.
+//   kTagged:  the same array with every child that is an internal node stored
+//             as (index << 8) | occupancy mask; materials as they are.  Stores
+//             of fewer than 2^24 nodes.
+//   kCompact: only the occupied children, packed: (unit << 8) | mask, the
+//             children from word 2 * unit on, in slot order.
+// With a mask in the reference an empty child costs no load.
+enum class Store { kPlain, kTagged, kCompact };
+
+// Where child `slot` of `ref`, whose mask (kTagged, kCompact) has that bit, is.
+template <Store S>
+__device__ __forceinline__ const uint32_t* occupied_at(const uint32_t* __restrict__ nodes, uint32_t ref, uint32_t slot)
 {
-    const uint32_t m = node & 0xffu;
-    if (!((m >> slot) & 1u)) return 0u;
-    loads++;
-    return __ldg(nodes + ((node >> 8) * 2u + __popc(m & ((1u << slot) - 1u))));  // offsets < 2^25 words
+    static_assert(S != Store::kPlain, "plain references carry no mask");
+    if constexpr (S == Store::kTagged)
+        return nodes + (((ref >> 5) & ~7u) | slot);
+    else
+        return nodes + ((ref >> 8) * 2u + __popc(ref & 0xffu & ((1u << slot) - 1u)));  // offsets < 2^25 words
 }
 
-// WIDE: 64-bit word index (the nested and integer-position kernels, any store
-// size); otherwise the store has fewer than 2^29 nodes.
-template <bool COMPACT, bool WIDE = false>
-__device__ __forceinline__ uint32_t child_of(const uint32_t* __restrict__ nodes, uint32_t node, uint32_t slot,
+// Child `slot` of `ref`, 0 where empty.  WIDE: 64-bit word index (the nested
+// and integer-position kernels, plain stores of any size); otherwise a plain
+// store has fewer than 2^29 nodes.  `loads` counts loads.
+template <Store S, bool WIDE = false>
+__device__ __forceinline__ uint32_t child_of(const uint32_t* __restrict__ nodes, uint32_t ref, uint32_t slot,
                                              uint32_t& loads)
 {
-    if constexpr (COMPACT) {
-        return load_child_compact(nodes, node, slot, loads);
-    } else {
+    if constexpr (S == Store::kPlain) {
         loads++;
-        return WIDE ? load_child(nodes, node, slot) : load_child32(nodes, node, slot);
-    }
-}
-
-// Child `slot` of a node given as the walk's own reference: in the reference
-// layout the word index of its first child (node * 8), in the compact one the
-// node reference itself.
-template <bool COMPACT>
-__device__ __forceinline__ uint32_t child_at(const uint32_t* __restrict__ nodes, uint32_t ref, uint32_t slot,
-                                             uint32_t& loads)
-{
-    if constexpr (COMPACT) {
-        return load_child_compact(nodes, ref, slot, loads);
+        return WIDE ? load_child(nodes, ref, slot) : load_child32(nodes, ref, slot);
     } else {
+        if (!((ref >> slot) & 1u)) return 0u;
         loads++;
-        return __ldg(nodes + (ref | slot));
+        return __ldg(occupied_at<S>(nodes, ref, slot));
     }
 }
 
@@ -167,6 +164,11 @@ struct LocalStack {
     __device__ __forceinline__ uint32_t below(uint32_t a) const { return a - 1u; }
     __device__ __forceinline__ void store(uint32_t a, uint32_t v) { slot[a & 31u] = v; }
     __device__ __forceinline__ uint32_t load(uint32_t a) const { return slot[a & 31u]; }
+    __device__ __forceinline__ uint32_t load_if(uint32_t a, bool valid, uint32_t otherwise) const
+    {
+        const uint32_t v = slot[a & 31u];
+        return valid ? v : otherwise;
+    }
     __device__ __forceinline__ uint32_t get(int h) const { return slot[h & 31]; }
     // Zeroes every slot (eight 16-byte stores); `top` is for the shared form.
     __device__ __forceinline__ void clear(int /*top*/)
@@ -203,6 +205,14 @@ struct SharedStack {
         asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
         return v;
     }
+    // The slot at `a` where `valid`, else `otherwise`; `a` may then be anything.
+    __device__ __forceinline__ uint32_t load_if(uint32_t a, bool valid, uint32_t otherwise) const
+    {
+        uint32_t v = otherwise;
+        asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; @p ld.shared.u32 %0, [%1]; }"
+                     : "+r"(v) : "r"(a), "r"((uint32_t)valid));
+        return v;
+    }
     __device__ __forceinline__ void put(int h, uint32_t v) { store(at(h), v); }
     __device__ __forceinline__ uint32_t get(int h) const { return load(at(h)); }
     // Zeroes slots 1..top.
@@ -221,8 +231,8 @@ struct EsvoOut {
 
 // findNearestMaterial (raytracing.cpp:134-162).
 // `fetches` counts child probes (the reference's loads, which also bound the
-// walk); `loads` the loads actually made (fewer in the compact layout).
-template <bool COMPACT = false, bool WIDE = false>
+// walk); `loads` the loads actually made (fewer where references carry masks).
+template <Store S, bool WIDE = false>
 __device__ __forceinline__ uint32_t nearest_material(const uint32_t* __restrict__ nodes, uint32_t node,
                                                      uint32_t sign_bits, uint32_t& fetches, uint32_t& status,
                                                      uint32_t& loads)
@@ -230,7 +240,7 @@ __device__ __forceinline__ uint32_t nearest_material(const uint32_t* __restrict_
     const uint32_t order = (0x76534210u | 0x88888888u) ^ (sign_bits * 0x11111111u);
     while (node >= kMaterialCount) {
         for (uint32_t ids = order; ids != 0u; ids >>= 4) {
-            const uint32_t c = child_of<COMPACT, WIDE>(nodes, node, ids & 7u, loads);
+            const uint32_t c = child_of<S, WIDE>(nodes, node, ids & 7u, loads);
             fetches++;
             if (c > 0u) { node = c; break; }
         }
@@ -302,7 +312,7 @@ __device__ __forceinline__ EsvoOut esvo(const uint32_t* __restrict__ nodes, cons
                 res.distance = tce;
                 if (q.compute_surface) {
                     uint32_t loads = 0;
-                    res.material = nearest_material<false, true>(nodes, child, f.sign_bits, fetches, status, loads);
+                    res.material = nearest_material<Store::kPlain, true>(nodes, child, f.sign_bits, fetches, status, loads);
                     if (status != kRayOk) { res.hit = false; return res; }
                     const float sx = (f.sign_bits & 1u) ? 1.0f : -1.0f;  // -rayDirSign
                     const float sy = (f.sign_bits & 2u) ? 1.0f : -1.0f;

@@ -121,7 +121,8 @@ typedef struct cbq_dag_info {
     cbq_subdag subdags[8];
     const uint32_t* device_nodes;
     uint32_t layout;          /* CBQ_DAG_LAYOUT_* in use */
-    uint64_t device_bytes;    /* bytes of the device node store */
+    uint64_t device_bytes;    /* bytes of the device node store (the reference layout
+                                 keeps as much again for the walk's own copy) */
 } cbq_dag_info;
 
 /* ---------------------------------------------------------------- basics */

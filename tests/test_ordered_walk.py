@@ -183,3 +183,32 @@ def test_kernels_against_the_oracle(seed, orc):
                             if k == "material":
                                 g, w = g.astype(np.uint32), w.astype(np.uint32)
                             assert oracle.same_bits_nan_equal(g, w), (what, k, mf, layout, stack, form, refill)
+
+
+@pytest.mark.gpu
+def test_store_beyond_the_tagged_range(orc):
+    """2^24 + 1 nodes (padded with unused ones): the walk on the plain store, alone, in a
+    batch beside a tagged volume and in a server, against the oracle."""
+    torch = pytest.importorskip("torch")
+    torch.cuda.set_device(0)
+    small, root, centre, edge = _volume(3)
+    nodes = np.zeros(((1 << 24) + 1) * 8, np.uint32)
+    nodes[:small.size] = small
+    sd = orc.find_subdags(small, root)
+    o, d = _rays(3, centre, edge)
+    to, td = torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda()
+    dag, tagged = cbq.Dag(nodes, root), cbq.Dag(small, root)
+    for mf in (-1.0, 0.02):
+        want = orc.intersect(small, sd, o, d, True, mf)
+        got = cbq.intersect_volume(dag, to, td, True, mf)
+        batch = cbq.Batch([(dag, to, td), (tagged, to, td)], True, mf)
+        batch.launch()
+        server = cbq.Server(device_memory_budget=16 << 20)
+        ticket, served = server.submit(dag, o, d, cbq.Query(True, mf))
+        assert server.wait(ticket, 20_000_000) == 0
+        torch.cuda.synchronize()
+        for res in (got, batch.outputs[0], batch.outputs[1], served):
+            for k in FIELDS:
+                g = res[k] if isinstance(res[k], np.ndarray) else res[k].cpu().numpy()
+                assert oracle.same_bits_nan_equal(g.astype(want[k].dtype) if k == "material" else g, want[k]), (k, mf)
+        server.close()
