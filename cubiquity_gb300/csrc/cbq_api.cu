@@ -18,6 +18,7 @@ namespace {
 
 constexpr int kFlatBlockDefault = 128;  // GB300, terrain-4096: 64, 128 and 256 threads within 1-3%
 constexpr uint32_t kRefillDefault = 16;
+constexpr uint32_t kStepsDefault = 8;
 
 bool use_flat(const cbq_dag* dag)
 {
@@ -32,11 +33,20 @@ FlatLaunch flat_launch(const cbq_dag* dag, bool persistent, uint64_t* counter, u
     fl.persistent = persistent;
     fl.counter = counter;
     fl.block = flat_block(dag);
-    fl.refill_min = refill ? refill : (dag->cfg.refill_min ? dag->cfg.refill_min : kRefillDefault);
+    fl.refill_min = refill ? refill : dag->cfg.refill_min;
     fl.local_stack = dag->cfg.stack == CBQ_STACK_LOCAL;
-    fl.steps = dag->cfg.steps > 0 ? (uint32_t)dag->cfg.steps : 1u;
-    fl.registers56 = dag->cfg.registers == 56;
+    fl.steps = (uint32_t)dag->cfg.steps;
+    // Either alone takes the other's default; neither leaves both to the kernel (WarpRefill).
+    if (fl.steps && !fl.refill_min) fl.refill_min = kRefillDefault;
+    if (!fl.steps) fl.steps = kStepsDefault;
     return fl;
+}
+
+// Rays per warp where a launch without a shape of the caller's is spread (spread_warp_rays), else 0.
+uint32_t spread_rays(const cbq_dag* dag, uint64_t n)
+{
+    const bool own = dag->cfg.refill_min != 0 || dag->cfg.steps != 0 || dag->cfg.form != CBQ_FORM_PERSISTENT;
+    return own ? 0u : spread_warp_rays(n, dag->device);
 }
 
 constexpr uint64_t kTaggedMaxNodes = 1ull << 24;  // a tagged reference holds 24 bits of node index
@@ -419,8 +429,11 @@ cbq_status cbq_intersect(const cbq_dag* dag, const cbq_rays* rays, uint64_t n, c
     if (st != CBQ_OK) return st;
     if (use_flat(dag)) {
         // The DAG's form: persistent (the default, with this stream's work counter) or plain.
-        uint64_t* counter = dag->cfg.form != CBQ_FORM_PLAIN ? stream_counter(dag, (cudaStream_t)stream) : nullptr;
-        const FlatLaunch fl = counter ? flat_launch(dag, true, counter, 0u) : flat_launch(dag, false, nullptr, 0u);
+        const uint32_t spread = spread_rays(dag, n);
+        uint64_t* counter =
+            dag->cfg.form != CBQ_FORM_PLAIN && !spread ? stream_counter(dag, (cudaStream_t)stream) : nullptr;
+        FlatLaunch fl = counter ? flat_launch(dag, true, counter, 0u) : flat_launch(dag, false, nullptr, 0u);
+        if (spread) fl.warp_rays = spread;
         return launch_flat(dag, make_dag_params(dag), make_query(query), make_hits(hits),
                            (const float4*)rays->origin_tmax, (const float4*)rays->direction, n, nullptr, fl,
                            (cudaStream_t)stream);
@@ -492,27 +505,22 @@ cbq_status cbq_autotune(cbq_dag* dag, const cbq_rays* rays, uint64_t n, const cb
     float win_ms = 1e30f;
     cbq_status st = CBQ_OK;
     static const int blocks[] = {64, 128, 256};
-    static const uint32_t refills[] = {4, 8, 16};
+    static const uint32_t refills[] = {8, 16, 24};
     static const int stacks[] = {CBQ_STACK_SHARED, CBQ_STACK_LOCAL};
-    static const int step_counts[] = {2, 4, 8, 16, 32};
-    constexpr int kSteps = 5;
+    static const int step_counts[] = {4, 8, 16, 32};
     for (int form = CBQ_FORM_PLAIN; form <= CBQ_FORM_SORTED && st == CBQ_OK; form++) {
         for (int blk : blocks) {
             for (uint32_t rf : refills) {
                 if (form == CBQ_FORM_PLAIN && rf != refills[0]) continue;  // refill unused
-                // stack x steps, plus the 56-register kernel for the persistent local-stack form
-                for (int v = 0; v < 3 * kSteps; v++) {
-                    const int stk = v < 2 * kSteps ? stacks[v & 1] : CBQ_STACK_LOCAL;
-                    const int regs = v < 2 * kSteps ? 0 : 56;
-                    if (regs && form == CBQ_FORM_PLAIN) continue;
+                for (int v = 0; v < 8; v++) {
                     cbq_launch_config c = saved;
                     c.kernel = CBQ_KERNEL_FLAT;
                     c.block = blk;
                     c.refill_min = rf;
-                    c.stack = stk;
+                    c.stack = stacks[v & 1];
                     c.form = form;
-                    c.steps = v < 2 * kSteps ? step_counts[v >> 1] : step_counts[v - 2 * kSteps];
-                    c.registers = regs;
+                    c.steps = step_counts[v >> 1];
+                    c.registers = 0;
                     dag->cfg = c;
                     st = cbq_intersect_auto(dag, rays, n, query, hits, scratch, scratch_bytes, stream);  // warm-up
                     if (st != CBQ_OK) break;
@@ -536,9 +544,9 @@ cbq_status cbq_autotune(cbq_dag* dag, const cbq_rays* rays, uint64_t n, const cb
     dag->cfg = st == CBQ_OK ? winner : saved;
     if (st == CBQ_OK)
         cbq::log(CBQ_LOG_INFO,
-                 "autotune over %llu rays: form %d, block %d, refill %u, stack %s, steps %d, registers %d: %.3f ms",
+                 "autotune over %llu rays: form %d, block %d, refill %u, stack %s, steps %d: %.3f ms",
                  (unsigned long long)n, winner.form, winner.block, winner.refill_min,
-                 winner.stack == CBQ_STACK_LOCAL ? "local" : "shared", winner.steps, winner.registers, win_ms);
+                 winner.stack == CBQ_STACK_LOCAL ? "local" : "shared", winner.steps, win_ms);
     if (best) *best = dag->cfg;
     if (best_ms) *best_ms = st == CBQ_OK ? win_ms : 0.0f;
     return st;
@@ -552,6 +560,7 @@ cbq_status cbq_dag_get_launch_config(const cbq_dag* dag, cbq_launch_config* cfg)
     if (cfg->block == 0) cfg->block = use_flat(dag) ? kFlatBlockDefault : kPlainBlock;
     if (cfg->chunk == 0) cfg->chunk = kDefaultChunk;
     if (cfg->refill_min == 0) cfg->refill_min = kRefillDefault;
+    if (cfg->steps == 0) cfg->steps = kStepsDefault;
     return CBQ_OK;
 }
 
@@ -585,11 +594,14 @@ cbq_status cbq_intersect_persistent(const cbq_dag* dag, const cbq_rays* rays, ui
     if (n == 0) return CBQ_OK;  // an empty batch may carry NULL buffers
     cbq_status st = check_rays(rays);
     if (st != CBQ_OK) return st;
-    if (use_flat(dag))
+    if (use_flat(dag)) {
+        const uint32_t spread = chunk == 0 ? spread_rays(dag, n) : 0u;
+        FlatLaunch fl = flat_launch(dag, !spread, spread ? nullptr : work_counter, std::min<uint32_t>(chunk, 32u));
+        if (spread) fl.warp_rays = spread;
         return launch_flat(dag, make_dag_params(dag), make_query(query), make_hits(hits),
-                           (const float4*)rays->origin_tmax, (const float4*)rays->direction, n, nullptr,
-                           flat_launch(dag, true, work_counter, std::min<uint32_t>(chunk, 32u)),
+                           (const float4*)rays->origin_tmax, (const float4*)rays->direction, n, nullptr, fl,
                            (cudaStream_t)stream);
+    }
     if (chunk == 0) chunk = dag->cfg.chunk ? dag->cfg.chunk : kDefaultChunk;
     const int stack_h = std::max(1, (int)dag->max_height);
     const size_t smem = (size_t)stack_h * kPersistBlock * sizeof(uint32_t);

@@ -61,7 +61,7 @@ __device__ __forceinline__ uint32_t job_of(const uint64_t* prefix, uint32_t njob
 template <bool COMPACT, bool SHARED, bool SORTED>
 __device__ __forceinline__ void batch_body(const JobDesc* __restrict__ jobs, uint32_t njobs, uint64_t total,
                                            unsigned long long* __restrict__ counter, uint32_t refill_min,
-                                           uint32_t steps, const uint32_t* __restrict__ perm)
+                                           uint32_t steps, const uint32_t* __restrict__ perm, uint32_t warp_rays)
 {
     extern __shared__ uint64_t prefix[];  // njobs + 1 entries, then the shared stack
     for (uint32_t j = threadIdx.x; j <= njobs; j += blockDim.x) prefix[j] = j < njobs ? jobs[j].first : total;
@@ -78,26 +78,34 @@ __device__ __forceinline__ void batch_body(const JobDesc* __restrict__ jobs, uin
     L.mode = kLaneIdle;
     L.job = 0;
     L.nodes = nullptr;
-    bool more = true;
+    bool more = warp_rays == 0u;
+    WarpRefill refill(refill_min, steps);
+    // Starts global ray g on this lane; its direction.
+    auto begin = [&](uint64_t g) {
+        if (SORTED) g = __ldg(perm + g);
+        const uint32_t j = job_of(prefix, njobs, g);
+        L.job = j;
+        L.nodes = jobs[j].nodes;
+        return lane_begin(L, c, g - prefix[j]);
+    };
+    if (!more) {  // a spread launch: each warp its own rays
+        const uint64_t g = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * warp_rays + lane;
+        if (lane < warp_rays && g < total) begin(g);
+    }
     for (;;) {
         if (more) {
             const uint32_t idle = __ballot_sync(kFullMask, L.mode == kLaneIdle);
             const uint32_t cnt = __popc(idle);
-            if (cnt == 32u || (cnt != 0u && cnt >= refill_min)) {
+            if (cnt == 32u || (cnt != 0u && cnt >= refill.idle_min)) {
                 const int leader = __ffs(idle) - 1;
                 unsigned long long base = 0;
                 if ((int)lane == leader) base = atomicAdd(counter, (unsigned long long)cnt);
                 base = __shfl_sync(kFullMask, base, leader);
-                if (L.mode == kLaneIdle) {
-                    uint64_t g = base + __popc(idle & below);
-                    if (g < total) {
-                        if (SORTED) g = __ldg(perm + g);
-                        const uint32_t j = job_of(prefix, njobs, g);
-                        L.job = j;
-                        L.nodes = jobs[j].nodes;
-                        lane_begin(L, c, g - prefix[j]);
-                    }
-                }
+                const uint64_t g = base + __popc(idle & below);
+                const bool fresh = L.mode == kLaneIdle && g < total;
+                float4 d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (fresh) d = begin(g);
+                refill.look(fresh, d);
                 if (base + cnt >= total) more = false;
             }
         }
@@ -110,9 +118,9 @@ __device__ __forceinline__ void batch_body(const JobDesc* __restrict__ jobs, uin
         else
             lane_settle(L, c, lstack);
         if (SHARED)
-            warp_walk_steps(L, c, sstack, steps, more ? refill_min : 32u);
+            warp_walk_steps(L, c, sstack, refill.steps, more ? refill.idle_min : 32u);
         else
-            warp_walk_steps(L, c, lstack, steps, more ? refill_min : 32u);
+            warp_walk_steps(L, c, lstack, refill.steps, more ? refill.idle_min : 32u);
     }
 }
 
@@ -120,20 +128,9 @@ template <bool COMPACT, bool SHARED, bool SORTED>
 __global__ void __launch_bounds__(256, 4) cbq_k_flat_batch(const JobDesc* __restrict__ jobs, uint32_t njobs,
                                                         uint64_t total, unsigned long long* __restrict__ counter,
                                                         uint32_t refill_min, uint32_t steps,
-                                                        const uint32_t* __restrict__ perm)
+                                                        const uint32_t* __restrict__ perm, uint32_t warp_rays)
 {
-    batch_body<COMPACT, SHARED, SORTED>(jobs, njobs, total, counter, refill_min, steps, perm);
-}
-
-// The local-stack form held to 56 registers per thread (more resident warps);
-// a batch autotuner choice like the single-volume kernel's.
-template <bool COMPACT, bool SORTED>
-__global__ void __maxnreg__(56) cbq_k_flat_batch_r56(const JobDesc* __restrict__ jobs, uint32_t njobs,
-                                                     uint64_t total, unsigned long long* __restrict__ counter,
-                                                     uint32_t refill_min, uint32_t steps,
-                                                     const uint32_t* __restrict__ perm)
-{
-    batch_body<COMPACT, false, SORTED>(jobs, njobs, total, counter, refill_min, steps, perm);
+    batch_body<COMPACT, SHARED, SORTED>(jobs, njobs, total, counter, refill_min, steps, perm, warp_rays);
 }
 
 // Octant of a ray: its direction sign bits (raytracing.cpp:416-417).
@@ -219,10 +216,9 @@ cbq_status launch_batch_variant(const dev::JobDesc* d_jobs, uint32_t njobs, uint
                                 int device, cudaStream_t s, const BatchLaunch& bl)
 {
     auto kernel = dev::cbq_k_flat_batch<COMPACT, SHARED, SORTED>;
-    if constexpr (!SHARED) {
-        if (bl.registers56) kernel = dev::cbq_k_flat_batch_r56<COMPACT, SORTED>;
-    }
-    if (!bl.counter_zeroed && cudaMemsetAsync(counter, 0, sizeof(uint64_t), s) != cudaSuccess) return CBQ_ERR_CUDA;
+    const uint32_t warp_rays = bl.spread ? spread_warp_rays(total, device) : 0u;
+    if (!warp_rays && !bl.counter_zeroed && cudaMemsetAsync(counter, 0, sizeof(uint64_t), s) != cudaSuccess)
+        return CBQ_ERR_CUDA;
     // The prefix offsets, then (shared stack) one column of stack_rows slots per thread.
     const size_t smem = (size_t)(njobs + 1) * 8 + (SHARED ? (size_t)std::max(1, bl.stack_rows) * bl.block * 4 : 0);
     if (smem > 227u * 1024u) return CBQ_ERR_CAPACITY;
@@ -236,9 +232,11 @@ cbq_status launch_batch_variant(const dev::JobDesc* d_jobs, uint32_t njobs, uint
     per_sm = std::max(per_sm, 1);
     // No more blocks than the rays fill: a small launch (a server's requests) starts
     // faster and leaves the SMs to the launches beside it.
-    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sms * per_sm, (total + bl.block - 1) / bl.block);
+    const uint64_t per_block = (uint64_t)bl.block / 32u * (warp_rays ? warp_rays : 32u);
+    const uint64_t blocks = (total + per_block - 1) / per_block;
+    const unsigned grid = (unsigned)(warp_rays ? blocks : std::min<uint64_t>((uint64_t)sms * per_sm, blocks));
     kernel<<<grid, bl.block, smem, s>>>(d_jobs, njobs, total, (unsigned long long*)counter, bl.refill,
-                                                bl.steps ? bl.steps : 1u, bl.perm);
+                                        bl.steps ? bl.steps : 1u, bl.perm, warp_rays);
     return cudaGetLastError() == cudaSuccess ? CBQ_OK : CBQ_ERR_CUDA;
 }
 
@@ -308,6 +306,7 @@ struct cbq_batch {
     // stack's place is set by batch_stack_in_shared.
     cbq_batch_config cfg{kBatchBlockDefault, kBatchRefillDefault, kBatchStepsDefault, 0, CBQ_STACK_LOCAL,
                          CBQ_FORM_PERSISTENT};
+    bool own_shape = false;                 // refill or steps set by the caller or the tuner
     cudaGraphExec_t exec = nullptr;
     // Persisting L2 window set on the graph's kernel nodes (l2_bytes 0: none).
     void* l2_base = nullptr;
@@ -323,9 +322,9 @@ BatchLaunch batch_launch(const cbq_batch* b, const uint32_t* perm)
     bl.block = b->cfg.block;
     bl.refill = b->cfg.refill_min;
     bl.steps = (uint32_t)b->cfg.steps;
-    bl.registers56 = b->cfg.registers == 56 && b->cfg.stack == CBQ_STACK_LOCAL;
     bl.shared_stack = b->cfg.stack == CBQ_STACK_SHARED;
     bl.stack_rows = b->stack_rows;
+    bl.spread = !b->own_shape;
     bl.perm = perm;
     return bl;
 }
@@ -522,6 +521,7 @@ cbq_status cbq_batch_set_config(cbq_batch* b, int32_t block, uint32_t refill_min
     if (!b || block < 0 || block > 256 || (block % 32) != 0 || refill_min > 32) return CBQ_ERR_INVALID_ARGUMENT;
     b->cfg.block = block ? block : kBatchBlockDefault;
     b->cfg.refill_min = refill_min ? refill_min : kBatchRefillDefault;
+    b->own_shape = refill_min != 0;
     drop_graph(b);
     return CBQ_OK;
 }
@@ -542,6 +542,7 @@ cbq_status cbq_batch_set_launch_config(cbq_batch* b, const cbq_batch_config* cfg
     if (st != CBQ_OK) return st;
     if (cfg->form == CBQ_FORM_SORTED && (st = ensure_sort_scratch(b)) != CBQ_OK) return st;
     b->cfg = *cfg;
+    b->own_shape = true;
     drop_graph(b);
     return CBQ_OK;
 }
@@ -602,18 +603,17 @@ cbq_status cbq_batch_autotune(cbq_batch* b, cbq_stream_t stream, int32_t repetit
     static const int blocks[] = {64, 128, 256};
     static const uint32_t refills[] = {4, 8, 12, 16};
     static const int32_t step_counts[] = {4, 8, 16};
-    // Kernel variants: local stack (64 registers), local stack held to 56
-    // registers, shared-memory stack; each with the rays in the order given or
+    // Descent stack in local or shared memory; the rays in the order given or
     // grouped by octant per job.
-    struct Variant { int32_t registers, stack, form; };
-    static const Variant variants[] = {
-        {0, CBQ_STACK_LOCAL, CBQ_FORM_PERSISTENT}, {56, CBQ_STACK_LOCAL, CBQ_FORM_PERSISTENT},
-        {0, CBQ_STACK_SHARED, CBQ_FORM_PERSISTENT}, {0, CBQ_STACK_LOCAL, CBQ_FORM_SORTED},
-        {56, CBQ_STACK_LOCAL, CBQ_FORM_SORTED}, {0, CBQ_STACK_SHARED, CBQ_FORM_SORTED}};
+    struct Variant { int32_t stack, form; };
+    static const Variant variants[] = {{CBQ_STACK_LOCAL, CBQ_FORM_PERSISTENT}, {CBQ_STACK_SHARED, CBQ_FORM_PERSISTENT},
+                                       {CBQ_STACK_LOCAL, CBQ_FORM_SORTED}, {CBQ_STACK_SHARED, CBQ_FORM_SORTED}};
     const bool can_sort = ensure_sort_scratch(b) == CBQ_OK;  // without the scratch, unsorted forms only
     cudaEvent_t e0, e1;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return CBQ_ERR_CUDA;
     const cbq_batch_config saved = b->cfg;
+    const bool saved_own = b->own_shape;
+    b->own_shape = true;
     cbq_batch_config best_cfg = saved;
     float best = 1e30f;
     cbq_status st = CBQ_OK;
@@ -622,7 +622,7 @@ cbq_status cbq_batch_autotune(cbq_batch* b, cbq_stream_t stream, int32_t repetit
             for (int32_t steps : step_counts) {
                 for (const Variant& v : variants) {
                     if (v.form == CBQ_FORM_SORTED && !can_sort) continue;
-                    b->cfg = cbq_batch_config{blk, rf, steps, v.registers, v.stack, v.form};
+                    b->cfg = cbq_batch_config{blk, rf, steps, 0, v.stack, v.form};
                     st = enqueue_batch(b, (cudaStream_t)stream);  // warm-up
                     if (st != CBQ_OK) break;
                     cudaEventRecord(e0, (cudaStream_t)stream);
@@ -645,12 +645,13 @@ cbq_status cbq_batch_autotune(cbq_batch* b, cbq_stream_t stream, int32_t repetit
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     b->cfg = st == CBQ_OK ? best_cfg : saved;
+    if (st != CBQ_OK) b->own_shape = saved_own;
     drop_graph(b);
     if (st == CBQ_OK)
         cbq::log(CBQ_LOG_INFO,
-                 "batch autotune: block %d, refill %u, %d steps per iteration, %d registers, %s stack, %s: "
+                 "batch autotune: block %d, refill %u, %d steps per check, %s stack, %s: "
                  "%.3f ms per launch",
-                 best_cfg.block, best_cfg.refill_min, best_cfg.steps, best_cfg.registers ? 56 : 64,
+                 best_cfg.block, best_cfg.refill_min, best_cfg.steps,
                  best_cfg.stack == CBQ_STACK_SHARED ? "shared" : "local",
                  best_cfg.form == CBQ_FORM_SORTED ? "octant-sorted" : "rays as given", best / (float)repetitions);
     return st;

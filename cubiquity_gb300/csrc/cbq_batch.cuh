@@ -34,10 +34,10 @@ struct BatchLaunch {
     int block = 128;
     uint32_t refill = 16;            // idle lanes that trigger a warp's refill
     uint32_t steps = 8;              // walk iterations between a warp's checks for idle lanes
-    bool registers56 = false;        // local-stack kernel held to 56 registers
     bool shared_stack = true;        // descent stack in shared memory (stack_rows rows) instead of local
     int stack_rows = 0;              // max SubDAG height over the jobs
     const uint32_t* perm = nullptr;  // octant order (launch_batch_octant_sort), or null
+    bool spread = false;             // a small launch may be spread over the chip (spread_warp_rays)
     bool counter_zeroed = false;     // the work counter is already zero, in stream order
 };
 

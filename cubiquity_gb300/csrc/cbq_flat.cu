@@ -12,7 +12,7 @@ namespace dev {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// PERSISTENT = false: one ray per thread (the drop-in form).
+// PERSISTENT = false: `refill_min` rays per warp (32: one per thread).
 // PERSISTENT = true : an SM-sized grid; when at least `refill_min` lanes of a
 //                     warp are idle, the warp takes that many new rays from
 //                     `counter` with one atomic and the idle lanes start them.
@@ -34,23 +34,26 @@ __device__ __forceinline__ void flat_body(const Ctx& c, uint64_t n, unsigned lon
     Lane L;
     L.mode = kLaneIdle;
     bool more = PERSISTENT;  // warp-uniform: the queue may still hold rays
+    WarpRefill refill(refill_min, steps);
     if (!PERSISTENT) {
-        const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-        if (i < n) lane_begin(L, c, SORTED ? (uint64_t)__ldg(perm + i) : c.ray_slot(i));
+        const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+        const uint64_t i = warp * refill_min + lane;
+        if (lane < refill_min && i < n) lane_begin(L, c, SORTED ? (uint64_t)__ldg(perm + i) : c.ray_slot(i));
     }
     for (;;) {
         if (PERSISTENT && more) {
             const uint32_t idle = __ballot_sync(kFull, L.mode == kLaneIdle);
             const uint32_t cnt = __popc(idle);
-            if (cnt == 32u || (cnt != 0u && cnt >= refill_min)) {
+            if (cnt == 32u || (cnt != 0u && cnt >= refill.idle_min)) {
                 const int leader = __ffs(idle) - 1;
                 unsigned long long base = 0;
                 if ((int)lane == leader) base = atomicAdd(counter, (unsigned long long)cnt);
                 base = __shfl_sync(kFull, base, leader);
-                if (L.mode == kLaneIdle) {
-                    const uint64_t i = base + __popc(idle & below);
-                    if (i < n) lane_begin(L, c, SORTED ? (uint64_t)__ldg(perm + i) : c.ray_slot(i));
-                }
+                const uint64_t i = base + __popc(idle & below);
+                const bool fresh = L.mode == kLaneIdle && i < n;
+                float4 d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (fresh) d = lane_begin(L, c, SORTED ? (uint64_t)__ldg(perm + i) : c.ray_slot(i));
+                refill.look(fresh, d);
                 if (base + cnt >= n) more = false;
             }
         }
@@ -62,12 +65,12 @@ __device__ __forceinline__ void flat_body(const Ctx& c, uint64_t n, unsigned lon
             lane_settle(L, c, sstack);
         else
             lane_settle(L, c, lstack);
-        // The walk goes on until refill_min lanes are idle (checked every
-        // `steps` iterations) or, with no rays left, until all are.
+        // The walk goes on until enough lanes are idle for a refill or, with no
+        // rays left, until all are.
         if (SHARED)
-            warp_walk_steps(L, c, sstack, steps, PERSISTENT && more ? refill_min : 32u);
+            warp_walk_steps(L, c, sstack, refill.steps, PERSISTENT && more ? refill.idle_min : 32u);
         else
-            warp_walk_steps(L, c, lstack, steps, PERSISTENT && more ? refill_min : 32u);
+            warp_walk_steps(L, c, lstack, refill.steps, PERSISTENT && more ? refill.idle_min : 32u);
     }
 }
 
@@ -77,18 +80,6 @@ __global__ void __launch_bounds__(256, 4) cbq_k_flat(Ctx c, uint64_t n, unsigned
                                                   uint32_t steps)
 {
     flat_body<PERSISTENT, SHARED, SORTED>(c, n, counter, refill_min, perm, steps);
-}
-
-// The persistent local-stack form held to 56 registers per thread: 36 resident
-// warps per SM instead of 32 with blocks of 64 or 128 threads.  Measured on
-// GB300 it is the faster choice for incoherent (bounce) rays, so the tuner
-// tries it (launch config `registers` = 56).
-template <bool SORTED, typename Ctx>
-__global__ void __maxnreg__(56) cbq_k_flat_r56(Ctx c, uint64_t n, unsigned long long* __restrict__ counter,
-                                               uint32_t refill_min, const uint32_t* __restrict__ perm,
-                                               uint32_t steps)
-{
-    flat_body<true, false, SORTED>(c, n, counter, refill_min, perm, steps);
 }
 
 // Octant of a ray: its direction sign bits (raytracing.cpp:416-417).
@@ -188,8 +179,8 @@ bool query_persistent_kernels()
            cudaFuncGetAttributes(&a, dev::cbq_k_flat<true, false, true, Ctx>) == cudaSuccess &&
            cudaFuncGetAttributes(&a, dev::cbq_k_flat<true, true, false, Ctx>) == cudaSuccess &&
            cudaFuncGetAttributes(&a, dev::cbq_k_flat<true, true, true, Ctx>) == cudaSuccess &&
-           cudaFuncGetAttributes(&a, dev::cbq_k_flat_r56<false, Ctx>) == cudaSuccess &&
-           cudaFuncGetAttributes(&a, dev::cbq_k_flat_r56<true, Ctx>) == cudaSuccess;
+           cudaFuncGetAttributes(&a, dev::cbq_k_flat<false, false, false, Ctx>) == cudaSuccess &&
+           cudaFuncGetAttributes(&a, dev::cbq_k_flat<false, true, false, Ctx>) == cudaSuccess;
 }
 
 }  // namespace
@@ -214,17 +205,15 @@ cbq_status launch_variant(const Ctx& c, uint64_t n, const FlatLaunch& fl, int ro
 {
     const size_t smem = S ? (size_t)rows * fl.block * sizeof(uint32_t) : 0;
     if (!P) {
-        const uint64_t blocks = (n + fl.block - 1) / fl.block;
+        const uint64_t per_block = (uint64_t)fl.block / 32u * fl.warp_rays;
+        const uint64_t blocks = (n + per_block - 1) / per_block;
         if (blocks > 0x7fffffffull) return CBQ_ERR_INVALID_ARGUMENT;
-        dev::cbq_k_flat<false, S, O, Ctx><<<(unsigned)blocks, fl.block, smem, stream>>>(c, n, nullptr, 0u, fl.perm,
-                                                                                     fl.steps ? fl.steps : 1u);
+        dev::cbq_k_flat<false, S, O, Ctx><<<(unsigned)blocks, fl.block, smem, stream>>>(
+            c, n, nullptr, fl.warp_rays, fl.perm, fl.steps ? fl.steps : 1u);
     } else {
         int sms = 0, per_sm = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return CBQ_ERR_CUDA;
         auto kernel = dev::cbq_k_flat<true, S, O, Ctx>;
-        if constexpr (!S) {
-            if (fl.registers56) kernel = dev::cbq_k_flat_r56<O, Ctx>;
-        }
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, fl.block, smem) != cudaSuccess)
             return CBQ_ERR_CUDA;
         per_sm = std::max(per_sm, 1);
@@ -283,6 +272,14 @@ Ctx make_ctx(const dev::DagParams& dp, const dev::QueryParams& q, const dev::Hit
     c.dir = dir;
     c.fetch_out = fetch_out;
     return c;
+}
+
+uint32_t spread_warp_rays(uint64_t n, int device)
+{
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0u;
+    const uint64_t warps = (uint64_t)sms * kSpreadWarpsPerSm;
+    return n <= warps * 32u ? (uint32_t)std::max<uint64_t>(1, (n + warps - 1) / warps) : 0u;
 }
 
 cbq_status launch_flat(const cbq_dag* dag, const dev::DagParams& dp, const dev::QueryParams& query,

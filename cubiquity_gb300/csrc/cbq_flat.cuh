@@ -209,8 +209,9 @@ struct OctantWalk {
 
 // Per-ray set-up: intersectVolume up to the octant loop (raytracing.cpp:409-434).
 // `ordered` false: by the reference form, whatever the ray.
+// Returns the ray's direction.
 template <typename Src>
-__device__ __forceinline__ void lane_begin(Lane& L, const Src& c, uint64_t i, bool ordered = true)
+__device__ __forceinline__ float4 lane_begin(Lane& L, const Src& c, uint64_t i, bool ordered = true)
 {
     L.ray = i;
     const float4 o = c.ray_origin(L, i);
@@ -252,6 +253,7 @@ __device__ __forceinline__ void lane_begin(Lane& L, const Src& c, uint64_t i, bo
     L.fetches = 0u;
     L.loads = 0u;
     L.mode = kLaneEnter;
+    return d;
 }
 
 // Completes a finished ray with the reference's operations and frees the lane:
@@ -768,6 +770,39 @@ __device__ __forceinline__ void warp_walk_steps(Lane& L, const Src& c, Stack& st
     flush_held(L, c);
 }
 
+// When a persistent warp refills: once `idle_min` lanes are idle, checked every
+// `steps` walk iterations.  A warp of coherent rays keeps its lanes in step
+// longest when nearly all of them start together, while one of incoherent rays
+// loses more to idle lanes than a refill costs.  So without a shape from the
+// caller (refill_min 0) each refill looks at its rays' directions: within a
+// quarter of their size of the first one's, the warp waits for 24 idle lanes
+// and checks every 16 iterations, else for 16 and every 8.  Both ways, us:
+// terrain-4096 camera rays 343 / 365, bounce rays 569 / 545.  The batch and
+// server launches keep 16 and 8: their small volumes' camera rays gain nothing
+// from waiting (12 volumes: 240 us, chosen by the rays 245).
+struct WarpRefill {
+    uint32_t idle_min, steps;
+    bool automatic;
+    __device__ __forceinline__ WarpRefill(uint32_t refill_min, uint32_t steps_)
+        : idle_min(refill_min ? refill_min : 16u), steps(refill_min ? steps_ : 8u), automatic(refill_min == 0u)
+    {
+    }
+    // After a refill (all 32 lanes call it): `fresh` lanes started rays of direction d.
+    __device__ __forceinline__ void look(bool fresh, float4 d)
+    {
+        if (!automatic) return;
+        const uint32_t mask = __ballot_sync(0xffffffffu, fresh);
+        const int first = __ffs(mask) - 1;  // (of -1, lane 31: no lane is fresh, the vote holds)
+        const float x = __shfl_sync(0xffffffffu, d.x, first), y = __shfl_sync(0xffffffffu, d.y, first),
+                    z = __shfl_sync(0xffffffffu, d.z, first);
+        const float near = 0.25f * fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z));
+        const float off = fmaxf(fmaxf(fabsf(d.x - x), fabsf(d.y - y)), fabsf(d.z - z));
+        const bool coherent = __all_sync(0xffffffffu, !fresh || off <= near);
+        idle_min = coherent ? 24u : 16u;
+        steps = coherent ? 16u : 8u;
+    }
+};
+
 // Octant transitions until the lane walks a SubDAG or has finished.  Bounded:
 // every kLaneNext raises `oct` (or finishes the ray), every kLaneEnter walks or
 // moves on, so at most 16 transitions happen.
@@ -791,8 +826,21 @@ struct FlatLaunch {
     bool local_stack = false;        // descent stack in local memory instead of shared
     const uint32_t* perm = nullptr;  // octant-sorted order (from launch_octant_sort), or null
     uint32_t steps = 1;              // ESVO steps per outer loop iteration
-    bool registers56 = false;        // persistent local-stack form held to 56 registers
+    uint32_t warp_rays = 32;         // plain form: rays per warp
 };
+
+// Rays per warp of a launch that the chip holds at once, 0 for a larger one.
+// A warp runs an iteration's advance and descent for any of its lanes, and a
+// small launch leaves most warp slots empty, so its rays are spread over all of
+// them: the call takes as long as its slowest ray, and a ray that shares its
+// warp with fewer others gets through its iterations sooner.  No work counter,
+// no atomics.  us per call, refilled from a counter / spread: 1,000 collision
+// rays 28.7 / 21.0, 12,000 33.4 / 28.4, 150,000 camera rays 37.7 / 32.1; one ray
+// per lane is reached at 32 rays a warp, where the two are alike (150,000
+// collision rays 46.6 / 43.4).  The server's launches run beside each other and
+// are not spread.
+constexpr int kSpreadWarpsPerSm = 32;
+uint32_t spread_warp_rays(uint64_t n, int device);
 
 }  // namespace cbq
 
@@ -806,6 +854,7 @@ cbq_status launch_flat(const cbq_dag* dag, const dev::DagParams& dp, const dev::
 cbq_status launch_octant_sort(const float4* dir, uint64_t n, uint32_t* counts16, uint32_t* perm, int device,
                               cudaStream_t stream);
 bool float_positions_exact(const cbq_dag* dag);
-// Loads every persistent flat traversal kernel on the current device.
+// Loads every flat traversal kernel that cbq_intersect_host_noalloc can launch
+// (persistent, or spread where the launch is small) on the current device.
 cbq_status preload_persistent_kernels();
 }  // namespace cbq

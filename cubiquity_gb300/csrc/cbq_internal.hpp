@@ -106,9 +106,9 @@ struct cbq_dag {
     int device = 0;
     bool flat_ok = false;          // float-position flat kernel applies (coordinates within +-2^21,
                                    // under 2^29 nodes); otherwise the integer-position form
-    // Defaults from GB300 sweeps of the ordered walk: persistent refill (block 128, 16 idle
-    // lanes), stack in shared memory, 8 iterations between the checks for idle lanes.
-    cbq_launch_config cfg{CBQ_KERNEL_AUTO, 0, 0, 0, CBQ_STACK_SHARED, CBQ_FORM_PERSISTENT, 8, 0};
+    // Persistent refill, block 128, stack in shared memory; refill and steps 0: chosen by the
+    // kernel from the rays (dev::WarpRefill).
+    cbq_launch_config cfg{CBQ_KERNEL_AUTO, 0, 0, 0, CBQ_STACK_SHARED, CBQ_FORM_PERSISTENT, 0, 0};
 
     // Staging sets of cbq_intersect_host, created as concurrent calls need them.
     std::mutex stages_lock;

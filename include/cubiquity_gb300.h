@@ -193,14 +193,14 @@ typedef struct cbq_launch_config {
     int32_t kernel;           /* cbq_kernel */
     int32_t block;            /* threads per block (multiple of 32, <= 256), 0 = default */
     uint32_t chunk;           /* nested persistent: rays per warp grab, 0 = default */
-    uint32_t refill_min;      /* flat persistent: idle lanes that trigger a refill, 0 = default */
+    uint32_t refill_min;      /* flat persistent: idle lanes that trigger a refill; 0 with
+                                 steps 0: both chosen from the rays, else 16 */
     int32_t stack;            /* CBQ_STACK_* (flat kernel; shared by default) */
     int32_t form;             /* CBQ_FORM_*, used by cbq_intersect_auto */
     int32_t steps;            /* flat kernel: walk iterations between a warp's checks for
-                                 idle lanes (1..32, 8 by default), 0 = 1 */
-    int32_t registers;        /* 0 (the default), or 56: the persistent local-stack
-                                 kernel held to 56 registers per thread (more
-                                 resident warps); other forms ignore it */
+                                 idle lanes (1..32), 0 = default (8, or from the rays) */
+    int32_t registers;        /* 0 (the default) or 56; every kernel of the walk takes
+                                 56 registers per thread now, so both are the same */
 } cbq_launch_config;
 
 cbq_status cbq_dag_set_launch_config(cbq_dag* dag, const cbq_launch_config* cfg);
@@ -216,10 +216,9 @@ uint64_t cbq_scratch_bytes(uint64_t n);
 cbq_status cbq_intersect_auto(const cbq_dag* dag, const cbq_rays* rays, uint64_t n, const cbq_query* query,
                               const cbq_hits* hits, void* scratch, uint64_t scratch_bytes, cbq_stream_t stream);
 
-/* Autotuner: times every form x block {64,128,256} x refill {4,8,16} x stack
- * {shared, local} x steps {2,4,8,16,32}, and the 56-register persistent
- * local-stack kernel, on these rays (synchronous; `repetitions` launches each),
- * stores the fastest in the DAG's launch config and returns it with its time. */
+/* Autotuner: times every form x block {64,128,256} x refill {8,16,24} x stack
+ * {shared, local} x steps {4,8,16,32} on these rays (synchronous; `repetitions`
+ * launches each), stores the fastest in the DAG's launch config and returns it with its time. */
 cbq_status cbq_autotune(cbq_dag* dag, const cbq_rays* rays, uint64_t n, const cbq_query* query,
                         const cbq_hits* hits, void* scratch, uint64_t scratch_bytes, int32_t repetitions,
                         cbq_launch_config* best, float* best_ms, cbq_stream_t stream);
@@ -324,7 +323,7 @@ typedef struct cbq_batch_config {
     int32_t block;            /* threads per block: 32..256, a multiple of 32 */
     uint32_t refill_min;      /* idle lanes that trigger a warp's refill: 1..32 */
     int32_t steps;            /* walk iterations between a warp's checks for idle lanes: 1..32 */
-    int32_t registers;        /* 0, or 56: the local-stack kernel held to 56 registers */
+    int32_t registers;        /* 0 or 56: the same (see cbq_launch_config) */
     int32_t stack;            /* CBQ_STACK_LOCAL or CBQ_STACK_SHARED (descent stack placement) */
     int32_t form;             /* CBQ_FORM_PERSISTENT: rays in the order given; CBQ_FORM_SORTED: each
                                  job's rays grouped by octant first (two small kernels per launch;
@@ -334,8 +333,8 @@ cbq_status cbq_batch_set_launch_config(cbq_batch* b, const cbq_batch_config* cfg
 cbq_status cbq_batch_get_launch_config(const cbq_batch* b, cbq_batch_config* cfg);
 
 /* Autotuner of the batched form: times block {64,128,256} x refill
- * {4,8,12,16} x steps {4,8,16} x {local stack, local stack at 56 registers,
- * shared-memory stack} x {rays as given, octant-sorted} on this batch
+ * {4,8,12,16} x steps {4,8,16} x {local stack, shared-memory stack} x {rays as
+ * given, octant-sorted} on this batch
  * (synchronous; `repetitions` launches each) and keeps the fastest. */
 cbq_status cbq_batch_autotune(cbq_batch* b, cbq_stream_t stream, int32_t repetitions);
 /* Replays the captured graph on `stream` (captures it first if needed). */
