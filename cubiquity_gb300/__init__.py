@@ -773,10 +773,7 @@ def pathtrace(dag: Dag, width: int, height: int, samples_per_pixel: int, bounces
     every traversal wave with device pointers (kind 0 extension, 1 shadow)."""
     import torch
     mats = np.ascontiguousarray(materials, dtype=np.float32).reshape(256, 2, 3)
-    arr = (_PtMaterial * 256)()
-    for m in range(256):
-        arr[m].albedo[:] = [float(v) for v in mats[m, 0]]
-        arr[m].emission[:] = [float(v) for v in mats[m, 1]]
+    arr = (_PtMaterial * 256).from_buffer_copy(mats)  # the same layout: albedo, emission
     cfg = _PtConfig(width, height, samples_per_pixel, bounces, (ctypes.c_double * 3)(*eye),
                     (ctypes.c_double * 3)(*target), tan_half_fov, max_footprint, (ctypes.c_float * 3)(*sun_direction),
                     (ctypes.c_float * 3)(*sun_colour), (ctypes.c_float * 3)(*sky_colour),

@@ -363,6 +363,7 @@ cbq_status cbq_dag_destroy(cbq_dag* dag)
     cudaFree(dag->d_nodes);
     if (dag->d_tagged) cudaFree(dag->d_tagged);
     for (auto& kv : dag->stream_counters) cudaFree(kv.second);
+    pt_workspace_release(dag->pt);
     for (auto& hs : dag->stages) {
         if (hs->d_stage) cudaFree(hs->d_stage);
         for (cudaStream_t& st : hs->pipe)
@@ -619,6 +620,28 @@ cbq_status cbq_intersect_persistent(const cbq_dag* dag, const cbq_rays* rays, ui
 }
 
 }  // extern "C"
+
+namespace cbq {
+
+bool takes_device_count(const cbq_dag* dag)
+{
+    return use_flat(dag) && dag->cfg.stack == CBQ_STACK_SHARED && dag->cfg.form == CBQ_FORM_PERSISTENT;
+}
+
+cbq_status intersect_device_count(const cbq_dag* dag, const cbq_rays* rays, uint64_t most, const uint32_t* n_dev,
+                                  const cbq_query* query, const cbq_hits* hits, uint64_t* zeroed_counter,
+                                  cbq_stream_t stream)
+{
+    const cbq_status st = check_rays(rays);
+    if (st != CBQ_OK || most == 0) return st;
+    FlatLaunch fl = flat_launch(dag, true, zeroed_counter, 0u);
+    fl.n_dev = n_dev;
+    return launch_flat(dag, make_dag_params(dag), make_query(query), make_hits(hits),
+                       (const float4*)rays->origin_tmax, (const float4*)rays->direction, most, nullptr, fl,
+                       (cudaStream_t)stream);
+}
+
+}  // namespace cbq
 
 namespace {
 

@@ -20,9 +20,13 @@ constexpr unsigned kFull = 0xffffffffu;
 //         per-thread local array.
 // SORTED: ray g of the launch is ray perm[g] of the input (octant order).
 // Ctx: FlatCtxT of the node store layout.
-template <bool PERSISTENT, bool SHARED, bool SORTED, typename Ctx>
+// COUNTED (persistent): the ray count, at most n, is at *n_dev, where an earlier
+// kernel on the stream left it.  A kernel of its own (cbq_k_flat_counted): the
+// two checks it needs cost the others 2-4%.
+template <bool PERSISTENT, bool SHARED, bool SORTED, typename Ctx, bool COUNTED = false>
 __device__ __forceinline__ void flat_body(const Ctx& c, uint64_t n, unsigned long long* __restrict__ counter,
-                                          uint32_t refill_min, const uint32_t* __restrict__ perm, uint32_t steps)
+                                          uint32_t refill_min, const uint32_t* __restrict__ perm, uint32_t steps,
+                                          const uint32_t* __restrict__ n_dev = nullptr)
 {
     extern __shared__ uint32_t smem_stack[];
     SharedStack sstack;
@@ -35,6 +39,12 @@ __device__ __forceinline__ void flat_body(const Ctx& c, uint64_t n, unsigned lon
     L.mode = kLaneIdle;
     bool more = PERSISTENT;  // warp-uniform: the queue may still hold rays
     WarpRefill refill(refill_min, steps);
+    uint32_t take = 32u;  // rays that a refill takes at most: fewer where the chip holds all rays at once
+    if constexpr (COUNTED) {
+        const uint32_t count = __ldg(n_dev), warps = gridDim.x * (blockDim.x >> 5);
+        if (count < n) n = count;
+        take = min(32u, max(1u, (count + warps - 1u) / warps));
+    }
     if (!PERSISTENT) {
         const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
         const uint64_t i = warp * refill_min + lane;
@@ -43,14 +53,16 @@ __device__ __forceinline__ void flat_body(const Ctx& c, uint64_t n, unsigned lon
     for (;;) {
         if (PERSISTENT && more) {
             const uint32_t idle = __ballot_sync(kFull, L.mode == kLaneIdle);
-            const uint32_t cnt = __popc(idle);
+            uint32_t cnt = __popc(idle);
             if (cnt == 32u || (cnt != 0u && cnt >= refill.idle_min)) {
                 const int leader = __ffs(idle) - 1;
                 unsigned long long base = 0;
+                if constexpr (COUNTED) cnt = min(cnt, take);
                 if ((int)lane == leader) base = atomicAdd(counter, (unsigned long long)cnt);
                 base = __shfl_sync(kFull, base, leader);
-                const uint64_t i = base + __popc(idle & below);
-                const bool fresh = L.mode == kLaneIdle && i < n;
+                const uint32_t rank = __popc(idle & below);
+                const uint64_t i = base + rank;
+                const bool fresh = L.mode == kLaneIdle && i < n && (!COUNTED || rank < cnt);
                 float4 d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 if (fresh) d = lane_begin(L, c, SORTED ? (uint64_t)__ldg(perm + i) : c.ray_slot(i));
                 refill.look(fresh, d);
@@ -80,6 +92,14 @@ __global__ void __launch_bounds__(256, 4) cbq_k_flat(Ctx c, uint64_t n, unsigned
                                                   uint32_t steps)
 {
     flat_body<PERSISTENT, SHARED, SORTED>(c, n, counter, refill_min, perm, steps);
+}
+
+template <typename Ctx>
+__global__ void __launch_bounds__(256, 4) cbq_k_flat_counted(Ctx c, uint64_t n, unsigned long long* __restrict__ counter,
+                                                             uint32_t refill_min, uint32_t steps,
+                                                             const uint32_t* __restrict__ n_dev)
+{
+    flat_body<true, true, false, Ctx, true>(c, n, counter, refill_min, nullptr, steps, n_dev);
 }
 
 // Octant of a ray: its direction sign bits (raytracing.cpp:416-417).
@@ -241,6 +261,22 @@ cbq_status launch_octant_sort(const float4* dir, uint64_t n, uint32_t* counts16,
     return cudaGetLastError() == cudaSuccess ? CBQ_OK : CBQ_ERR_CUDA;
 }
 
+// The counted launch: persistent, shared stack, rays in order, the work counter already zero.
+template <typename Ctx>
+cbq_status launch_counted(const Ctx& c, uint64_t n, const FlatLaunch& fl, int rows, cudaStream_t stream, int device)
+{
+    const size_t smem = (size_t)rows * fl.block * sizeof(uint32_t);
+    auto kernel = dev::cbq_k_flat_counted<Ctx>;
+    int sms = 0, per_sm = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, fl.block, smem) != cudaSuccess)
+        return CBQ_ERR_CUDA;
+    const uint64_t full = (uint64_t)sms * std::max(per_sm, 1);
+    const unsigned grid = (unsigned)std::min<uint64_t>(full, (n + 31) / 32);  // n may be far above the count
+    kernel<<<grid, fl.block, smem, stream>>>(c, n, (unsigned long long*)fl.counter, fl.refill_min, fl.steps, fl.n_dev);
+    return cudaGetLastError() == cudaSuccess ? CBQ_OK : CBQ_ERR_CUDA;
+}
+
 // The eight launch shapes of one context type.
 template <typename Ctx>
 cbq_status launch_ctx(const Ctx& c, uint64_t n, const FlatLaunch& fl, int rows, cudaStream_t stream, int dv)
@@ -274,6 +310,14 @@ Ctx make_ctx(const dev::DagParams& dp, const dev::QueryParams& q, const dev::Hit
     return c;
 }
 
+static dev::DagParams tagged_params(const cbq_dag* dag, const dev::DagParams& dp)
+{
+    dev::DagParams tagged = dp;
+    tagged.nodes = dag->d_tagged;
+    for (int k = 0; k < 8; k++) tagged.sd[k].node = dag->tagged_ref[k];
+    return tagged;
+}
+
 uint32_t spread_warp_rays(uint64_t n, int device)
 {
     int sms = 0;
@@ -286,6 +330,17 @@ cbq_status launch_flat(const cbq_dag* dag, const dev::DagParams& dp, const dev::
                        const dev::HitsOut& out, const float4* orig, const float4* dir, uint64_t n,
                        uint32_t* fetch_out, const FlatLaunch& fl, cudaStream_t stream)
 {
+    if (fl.n_dev) {  // contexts that take any query
+        const int rows = std::max(1, (int)dag->max_height), dv = dag->device;
+        if (dag->layout == CBQ_DAG_LAYOUT_COMPACT)
+            return launch_counted(make_ctx<CompactCtx<true>>(dp, query, out, orig, dir, nullptr), n, fl, rows, stream, dv);
+        if (!dag->flat_ok)
+            return launch_counted(make_ctx<IntCtx>(dp, query, out, orig, dir, nullptr), n, fl, rows, stream, dv);
+        if (dag->d_tagged)
+            return launch_counted(make_ctx<TaggedCtx<true>>(tagged_params(dag, dp), query, out, orig, dir, nullptr), n,
+                                  fl, rows, stream, dv);
+        return launch_counted(make_ctx<PlainCtx>(dp, query, out, orig, dir, nullptr), n, fl, rows, stream, dv);
+    }
     // The image order applies where it is a bijection of this launch's rays:
     // whole 8-row bands of a width that is a multiple of 4, 32-bit indices.
     dev::QueryParams q = query;
@@ -317,9 +372,7 @@ cbq_status launch_flat(const cbq_dag* dag, const dev::DagParams& dp, const dev::
     if (!dag->flat_ok)  // coordinates beyond +-2^21 or 2^29 nodes or more: integer positions
         return launch_ctx(make_ctx<IntCtx>(dp, q, out, orig, dir, nullptr), n, fl, rows, stream, dv);
     if (dag->d_tagged) {
-        dev::DagParams tagged = dp;
-        tagged.nodes = dag->d_tagged;
-        for (int k = 0; k < 8; k++) tagged.sd[k].node = dag->tagged_ref[k];
+        const dev::DagParams tagged = tagged_params(dag, dp);
         return lod ? launch_ctx(make_ctx<TaggedCtx<true>>(tagged, q, out, orig, dir, nullptr), n, fl, rows, stream, dv)
                    : launch_ctx(make_ctx<TaggedCtx<false>>(tagged, q, out, orig, dir, nullptr), n, fl, rows, stream,
                                 dv);

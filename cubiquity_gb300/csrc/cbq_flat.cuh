@@ -827,6 +827,9 @@ struct FlatLaunch {
     const uint32_t* perm = nullptr;  // octant-sorted order (from launch_octant_sort), or null
     uint32_t steps = 1;              // ESVO steps per outer loop iteration
     uint32_t warp_rays = 32;         // plain form: rays per warp
+    // Counted launches (always persistent, shared stack, in order): the device's ray count, at
+    // most the launch's n; the work counter is already zero, in stream order.
+    const uint32_t* n_dev = nullptr;
 };
 
 // Rays per warp of a launch that the chip holds at once, 0 for a larger one.

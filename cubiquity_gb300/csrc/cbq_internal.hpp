@@ -82,6 +82,29 @@ struct HostStage {
     struct CUevent_st* pipe_ev[2 * kHostChunksMax] = {};  // cudaEvent_t
 };
 
+// The pathtracer's device memory, streams and events.  A DAG keeps one set between
+// frames (at most kPtKeptBytes of memory); a frame that finds it in use by another
+// thread makes its own.
+constexpr uint64_t kPtKeptBytes = 1ull << 30;
+struct PtWorkspace {
+    char* base = nullptr;
+    uint64_t bytes = 0;
+    struct CUstream_st* wave = nullptr;    // extension waves and shading (higher priority)
+    struct CUstream_st* shadow = nullptr;  // shadow waves
+    struct CUevent_st* begin = nullptr;
+    struct CUevent_st* shaded[2] = {};     // a depth's shadow rays are written
+    struct CUevent_st* traced[2] = {};     // ... and traced (their set may be written again)
+};
+void pt_workspace_release(PtWorkspace& w);
+
+// Traversal of the rays that an earlier kernel on the stream counted at *n_dev (at
+// most `most`), with a work counter that is zero in stream order.  Where
+// takes_device_count(dag) is false the caller has to read the count itself.
+bool takes_device_count(const cbq_dag* dag);
+cbq_status intersect_device_count(const cbq_dag* dag, const cbq_rays* rays, uint64_t most, const uint32_t* n_dev,
+                                  const cbq_query* query, const cbq_hits* hits, uint64_t* zeroed_counter,
+                                  cbq_stream_t stream);
+
 }  // namespace cbq
 
 // The opaque DAG handle.
@@ -113,6 +136,8 @@ struct cbq_dag {
     // Staging sets of cbq_intersect_host, created as concurrent calls need them.
     std::mutex stages_lock;
     std::vector<std::unique_ptr<cbq::HostStage>> stages;
+    std::mutex pt_lock;  // held by the frame that uses `pt`
+    cbq::PtWorkspace pt;
     // Work counters of cbq_intersect's persistent form, one per stream id (ids are unique
     // for the context's lifetime, so launches sharing a counter are ordered by their stream).
     std::mutex counter_lock;

@@ -24,6 +24,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <vector>
 
 namespace {
@@ -142,7 +143,8 @@ __device__ __forceinline__ void reserve_slots(unsigned long long* counts, bool h
     b = (uint32_t)(base >> 32) + (uint32_t)__popc(cm & below);
 }
 
-__global__ void cbq_k_pt_shade(const Shading* __restrict__ sh, uint32_t n, uint32_t depth, uint64_t seed, int last, const PathState* __restrict__ st,
+__global__ void cbq_k_pt_shade(const Shading* __restrict__ sh, uint32_t n, const uint32_t* __restrict__ n_dev,
+                               uint32_t depth, uint64_t seed, int last, const PathState* __restrict__ st,
                                const uint8_t* __restrict__ hit, const uint32_t* __restrict__ material,
                                const float* __restrict__ position, const float* __restrict__ normal,
                                float* __restrict__ image, float4* __restrict__ so, float4* __restrict__ sd,
@@ -150,6 +152,7 @@ __global__ void cbq_k_pt_shade(const Shading* __restrict__ sh, uint32_t n, uint3
                                float4* __restrict__ no, float4* __restrict__ nd, PathState* __restrict__ nst)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n_dev) n = __ldg(n_dev);  // the count of an earlier wave's shading; n otherwise
     const bool live = i < n;
     PathState p{0u, 0u, 0.0f, 0.0f, 0.0f};
     bool h = false;
@@ -202,10 +205,11 @@ __global__ void cbq_k_pt_shade(const Shading* __restrict__ sh, uint32_t n, uint3
     }
 }
 
-__global__ void cbq_k_pt_shadow_add(uint32_t n, const uint8_t* __restrict__ hit, const float4* __restrict__ sw,
-                                    float* __restrict__ image)
+__global__ void cbq_k_pt_shadow_add(uint32_t n, const uint32_t* __restrict__ n_dev, const uint8_t* __restrict__ hit,
+                                    const float4* __restrict__ sw, float* __restrict__ image)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n_dev) n = __ldg(n_dev);
     if (i >= n || hit[i]) return;
     const float4 w = sw[i];
     add_pixel(image, __float_as_uint(w.w), w.x, w.y, w.z);
@@ -217,6 +221,39 @@ __global__ void cbq_k_pt_scale(float* image, size_t count, float scale)
     if (i < count) image[i] *= scale;
 }
 
+void release_memory(cbq::PtWorkspace& w)
+{
+    if (w.base) cudaFree(w.base);
+    w.base = nullptr;
+    w.bytes = 0;
+}
+
+// Streams, events and at least `bytes` of device memory in `w`.
+cbq_status prepare_workspace(cbq::PtWorkspace& w, uint64_t bytes)
+{
+    if (!w.wave) {
+        int low = 0, high = 0;
+        bool ok = cudaDeviceGetStreamPriorityRange(&low, &high) == cudaSuccess &&
+                  cudaStreamCreateWithPriority(&w.wave, cudaStreamNonBlocking, high) == cudaSuccess &&
+                  cudaStreamCreateWithPriority(&w.shadow, cudaStreamNonBlocking, low) == cudaSuccess;
+        cudaEvent_t* events[] = {&w.begin, &w.shaded[0], &w.shaded[1], &w.traced[0], &w.traced[1]};
+        for (cudaEvent_t* ev : events) ok = ok && cudaEventCreateWithFlags(ev, cudaEventDisableTiming) == cudaSuccess;
+        if (!ok) {
+            cudaGetLastError();
+            return CBQ_ERR_CUDA;
+        }
+    }
+    if (w.bytes >= bytes) return CBQ_OK;
+    release_memory(w);
+    if (cudaMalloc((void**)&w.base, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        w.base = nullptr;
+        return CBQ_ERR_OUT_OF_MEMORY;
+    }
+    w.bytes = bytes;
+    return CBQ_OK;
+}
+
 template <typename T>
 T* carve(char*& p, size_t count)
 {
@@ -226,6 +263,19 @@ T* carve(char*& p, size_t count)
 }
 
 }  // namespace
+
+void cbq::pt_workspace_release(PtWorkspace& w)
+{
+    release_memory(w);
+    for (cudaStream_t* q : {&w.wave, &w.shadow}) {
+        if (*q) cudaStreamDestroy(*q);
+        *q = nullptr;
+    }
+    for (cudaEvent_t* ev : {&w.begin, &w.shaded[0], &w.shaded[1], &w.traced[0], &w.traced[1]}) {
+        if (*ev) cudaEventDestroy(*ev);
+        *ev = nullptr;
+    }
+}
 
 extern "C" cbq_status cbq_copy_to_host(void* host_dst, const void* device_src, uint64_t bytes)
 {
@@ -272,21 +322,30 @@ extern "C" cbq_status cbq_pathtrace(const cbq_dag* dag, const cbq_pt_config* cfg
             host_sh.emission[m][a] = cfg->materials[m].emission[a];
         }
 
-    // Buffers for one pass: two extension sets (ping-pong) and the shadow set.
+    // Buffers for one pass: two extension sets (ping-pong) and two shadow sets (a depth's
+    // shadow wave runs beside the next depth's extension wave).
     const uint64_t per_pass = std::max<uint64_t>(
         1, std::min<uint64_t>((uint64_t)cfg->samples_per_pixel, kPtRaysPerPass / npix));
     const size_t ext = npix * per_pass, sha = 2 * ext;
+    const size_t passes = ((size_t)cfg->samples_per_pixel + per_pass - 1) / per_pass;
+    const size_t waves = passes * ((size_t)cfg->bounces + 1);
     const size_t per_ext = 2 * 16 + sizeof(PathState) + 1 + 4 + 12 + 12;
-    const size_t bytes = 2 * (ext * per_ext) + sha * (16 * 3 + 1) + sizeof(Shading) + 32 * 256;  // + carve padding
-    char* base = nullptr;
-    if (cudaMalloc((void**)&base, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        return CBQ_ERR_OUT_OF_MEMORY;
+    const size_t control = waves * (8 + 2 * 8);  // per wave: shadow and next count, two work counters
+    const size_t bytes = 2 * (ext * per_ext + sha * (16 * 3 + 1)) + control + sizeof(Shading) + 40 * 256;  // + carve padding
+
+    // The DAG's workspace, or one of this frame's own where another frame has it.
+    cbq_dag* owner = const_cast<cbq_dag*>(dag);
+    std::unique_lock<std::mutex> lock(owner->pt_lock, std::try_to_lock);
+    cbq::PtWorkspace own;
+    cbq::PtWorkspace& ws = lock.owns_lock() ? owner->pt : own;
+    cbq_status st = prepare_workspace(ws, bytes);
+    if (st != CBQ_OK) {
+        cbq::pt_workspace_release(ws);
+        return st;
     }
-    char* p = base;
+    char* p = ws.base;
     Shading* d_sh = carve<Shading>(p, 1);
-    uint32_t* counters = carve<uint32_t>(p, 8);           // [0] shadow count, [1] next count (one 64-bit word)
-    uint64_t* work = carve<uint64_t>(p, 4);
+    uint64_t* counts = carve<uint64_t>(p, 3 * waves);  // per wave: [shadow count, next count], extension and shadow work
     struct Ext {
         float4 *o, *d;
         PathState* st;
@@ -294,6 +353,10 @@ extern "C" cbq_status cbq_pathtrace(const cbq_dag* dag, const cbq_pt_config* cfg
         uint32_t* material;
         float *position, *normal;
     } e[2];
+    struct Sha {
+        float4 *o, *d, *w;
+        uint8_t* hit;
+    } s2[2];
     for (int k = 0; k < 2; k++) {
         e[k].o = carve<float4>(p, ext);
         e[k].d = carve<float4>(p, ext);
@@ -302,24 +365,33 @@ extern "C" cbq_status cbq_pathtrace(const cbq_dag* dag, const cbq_pt_config* cfg
         e[k].material = carve<uint32_t>(p, ext);
         e[k].position = carve<float>(p, 3 * ext);
         e[k].normal = carve<float>(p, 3 * ext);
+        s2[k].o = carve<float4>(p, sha);
+        s2[k].d = carve<float4>(p, sha);
+        s2[k].w = carve<float4>(p, sha);
+        s2[k].hit = carve<uint8_t>(p, sha);
     }
-    float4* so = carve<float4>(p, sha);
-    float4* sd = carve<float4>(p, sha);
-    float4* sw = carve<float4>(p, sha);
-    uint8_t* shit = carve<uint8_t>(p, sha);
-    if ((size_t)(p - base) > bytes) {
-        cudaFree(base);
-        return CBQ_ERR_INVALID_ARGUMENT;
-    }
+    if ((size_t)(p - ws.base) > bytes) return CBQ_ERR_INVALID_ARGUMENT;
 
-    cbq_status st = CBQ_OK;
+    // Without a wave callback the host reads nothing until the frame is done: a wave's ray
+    // count stays on the device (the shading that compacts the next wave's rays leaves it
+    // there), and shadow waves run on a stream of their own beside the next extension wave,
+    // each filling the SMs that the other's last rays leave.
+    const bool ahead = !on_wave && cbq::takes_device_count(dag);
+    const cudaStream_t sw = ahead ? (cudaStream_t)ws.wave : s;
+    const cudaStream_t ss = ahead ? (cudaStream_t)ws.shadow : s;
     uint64_t ext_rays = 0, shadow_rays = 0, launches = 0;
     auto fail = [&](cbq_status code) {
         st = code;
         cudaGetLastError();
     };
-    if (cudaMemcpyAsync(d_sh, &host_sh, sizeof(Shading), cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        cudaMemsetAsync(device_image, 0, npix * 3 * sizeof(float), s) != cudaSuccess)
+    auto ok = [](cudaError_t e) { return e == cudaSuccess; };
+    if (!ok(cudaMemcpyAsync(d_sh, &host_sh, sizeof(Shading), cudaMemcpyHostToDevice, s)) ||
+        !ok(cudaMemsetAsync(counts, 0, 3 * waves * sizeof(uint64_t), s)) ||
+        !ok(cudaMemsetAsync(device_image, 0, npix * 3 * sizeof(float), s)))
+        fail(CBQ_ERR_CUDA);
+    if (st == CBQ_OK && ahead &&
+        (!ok(cudaEventRecord(ws.begin, s)) || !ok(cudaStreamWaitEvent(sw, ws.begin, 0)) ||
+         !ok(cudaStreamWaitEvent(ss, ws.begin, 0))))
         fail(CBQ_ERR_CUDA);
 
     const cbq_query qext{1, cfg->max_footprint, 0u, 0u};
@@ -327,6 +399,8 @@ extern "C" cbq_status cbq_pathtrace(const cbq_dag* dag, const cbq_pt_config* cfg
     // The camera wave's paths are the pass's samples' images stacked in row-major
     // order: the traversal may deal them to warps in image tiles.
     const cbq_query qcam{1, cfg->max_footprint, 0u, (uint32_t)cfg->width};
+    size_t wave = 0;  // over the frame's passes and depths
+    bool set_used[2] = {false, false};
     for (int sample = 0; sample < cfg->samples_per_pixel && st == CBQ_OK; sample += (int)per_pass) {
         const uint32_t samples = (uint32_t)std::min<uint64_t>(per_pass, (uint64_t)(cfg->samples_per_pixel - sample));
         Frame fr;
@@ -343,64 +417,111 @@ extern "C" cbq_status cbq_pathtrace(const cbq_dag* dag, const cbq_pt_config* cfg
         fr.ux = (float)u[0]; fr.uy = (float)u[1]; fr.uz = (float)u[2];
         fr.tan_half = (float)cfg->tan_half_fov;
         fr.aspect = (float)cfg->width / (float)cfg->height;
-        const uint64_t paths = npix * samples;
-        cbq_k_pt_camera<<<(unsigned)((paths + 255) / 256), 256, 0, s>>>(fr, e[0].o, e[0].d, e[0].st);
+        const uint32_t paths = (uint32_t)(npix * samples);
+        cbq_k_pt_camera<<<(paths + 255) / 256, 256, 0, sw>>>(fr, e[0].o, e[0].d, e[0].st);
         launches++;
-        uint32_t n = (uint32_t)paths;
+        uint32_t n = paths;                  // this wave's rays, or (ahead, depth > 0) at most that
+        const uint32_t* n_dev = nullptr;     // ... and their count on the device
         int cur = 0;
-        for (int depth = 0; depth <= cfg->bounces && n > 0 && st == CBQ_OK; depth++) {
+        ext_rays += paths;
+        for (int depth = 0; depth <= cfg->bounces && n > 0 && st == CBQ_OK; depth++, wave++) {
             Ext& E = e[cur];
             Ext& N = e[cur ^ 1];
+            const int set = (int)(wave & 1u);
+            Sha& S = s2[set];
+            uint32_t* count = (uint32_t*)(counts + wave);                 // [0] shadow rays, [1] next extension rays
+            uint64_t* work = counts + waves + 2 * wave;                   // extension and shadow work counters
             cbq_rays rays{(const float*)E.o, (const float*)E.d};
             cbq_hits hits{E.hit, nullptr, E.material, E.position, E.normal, nullptr, nullptr};
             const cbq_query* qe = depth == 0 ? &qcam : &qext;
-            cbq_status ts = cbq_intersect_persistent(dag, &rays, n, qe, &hits, work, 0u, (cbq_stream_t)s);
+            cbq_status ts = n_dev ? cbq::intersect_device_count(dag, &rays, n, n_dev, qe, &hits, work, (cbq_stream_t)sw)
+                                  : cbq_intersect_persistent(dag, &rays, n, qe, &hits, work, 0u, (cbq_stream_t)sw);
             if (ts != CBQ_OK) { fail(ts); break; }
-            ext_rays += n;
             launches++;
             if (on_wave) {
-                if (cudaStreamSynchronize(s) != cudaSuccess) { fail(CBQ_ERR_CUDA); break; }
+                if (!ok(cudaStreamSynchronize(s))) { fail(CBQ_ERR_CUDA); break; }
                 on_wave(user, 0, depth, sample, (const float*)E.o, (const float*)E.d, n, &hits, qe);
             }
-            if (cudaMemsetAsync(counters, 0, 8 * sizeof(uint32_t), s) != cudaSuccess) { fail(CBQ_ERR_CUDA); break; }
+            if (ahead && set_used[set] && !ok(cudaStreamWaitEvent(sw, ws.traced[set], 0))) { fail(CBQ_ERR_CUDA); break; }
             const int last = depth == cfg->bounces;
-            cbq_k_pt_shade<<<(n + 255) / 256, 256, 0, s>>>(d_sh, n, (uint32_t)depth, cfg->seed, last,
-                                                          E.st, E.hit, E.material, E.position, E.normal, device_image,
-                                                          so, sd, sw, (unsigned long long*)counters, N.o, N.d, N.st);
+            cbq_k_pt_shade<<<(n + 255) / 256, 256, 0, sw>>>(d_sh, n, n_dev, (uint32_t)depth, cfg->seed, last, E.st, E.hit,
+                                                            E.material, E.position, E.normal, device_image, S.o, S.d,
+                                                            S.w, (unsigned long long*)count, N.o, N.d, N.st);
             launches++;
-            uint32_t h_counts[2] = {0, 0};
-            if (cudaMemcpyAsync(h_counts, counters, sizeof(h_counts), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-                cudaStreamSynchronize(s) != cudaSuccess) {
+            uint32_t ns = 2u * n, next = n;
+            if (!ahead) {
+                uint32_t h_counts[2] = {0, 0};
+                if (!ok(cudaMemcpyAsync(h_counts, count, sizeof(h_counts), cudaMemcpyDeviceToHost, s)) ||
+                    !ok(cudaStreamSynchronize(s))) {
+                    fail(CBQ_ERR_CUDA);
+                    break;
+                }
+                ns = h_counts[0];
+                next = h_counts[1];
+                shadow_rays += ns;
+                ext_rays += next;
+            } else if (!ok(cudaEventRecord(ws.shaded[set], sw)) || !ok(cudaStreamWaitEvent(ss, ws.shaded[set], 0))) {
                 fail(CBQ_ERR_CUDA);
                 break;
             }
-            const uint32_t ns = h_counts[0];
             if (ns > 0) {
-                cbq_rays srays{(const float*)so, (const float*)sd};
-                cbq_hits shits{shit, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-                ts = cbq_intersect_persistent(dag, &srays, ns, &qsh, &shits, work + 1, 0u, (cbq_stream_t)s);
+                cbq_rays srays{(const float*)S.o, (const float*)S.d};
+                cbq_hits shits{S.hit, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+                ts = ahead ? cbq::intersect_device_count(dag, &srays, ns, count, &qsh, &shits, work + 1, (cbq_stream_t)ss)
+                           : cbq_intersect_persistent(dag, &srays, ns, &qsh, &shits, work + 1, 0u, (cbq_stream_t)ss);
                 if (ts != CBQ_OK) { fail(ts); break; }
-                shadow_rays += ns;
                 launches++;
                 if (on_wave) {
-                    if (cudaStreamSynchronize(s) != cudaSuccess) { fail(CBQ_ERR_CUDA); break; }
-                    on_wave(user, 1, depth, sample, (const float*)so, (const float*)sd, ns, &shits, &qsh);
+                    if (!ok(cudaStreamSynchronize(s))) { fail(CBQ_ERR_CUDA); break; }
+                    on_wave(user, 1, depth, sample, (const float*)S.o, (const float*)S.d, ns, &shits, &qsh);
                 }
-                cbq_k_pt_shadow_add<<<(ns + 255) / 256, 256, 0, s>>>(ns, shit, sw, device_image);
+                cbq_k_pt_shadow_add<<<(ns + 255) / 256, 256, 0, ss>>>(ns, ahead ? count : nullptr, S.hit, S.w,
+                                                                      device_image);
                 launches++;
             }
-            n = h_counts[1];
+            if (ahead) {
+                if (!ok(cudaEventRecord(ws.traced[set], ss))) { fail(CBQ_ERR_CUDA); break; }
+                set_used[set] = true;
+                n_dev = count + 1;
+            }
+            n = next;
             cur ^= 1;
         }
     }
+    if (ahead) {  // both streams' work ends before the caller's goes on, errors or not
+        for (cudaStream_t q : {sw, ss})
+            if (!ok(cudaEventRecord(ws.begin, q)) || !ok(cudaStreamWaitEvent(s, ws.begin, 0))) fail(CBQ_ERR_CUDA);
+    }
+    std::vector<uint64_t> h_counts;
     if (st == CBQ_OK) {
         const size_t cnt = npix * 3;
         cbq_k_pt_scale<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(device_image, cnt,
-                                                                       1.0f / (float)cfg->samples_per_pixel);
+                                                                     1.0f / (float)cfg->samples_per_pixel);
         launches++;
-        if (cudaStreamSynchronize(s) != cudaSuccess) fail(CBQ_ERR_CUDA);
+        if (ahead) {
+            try {
+                h_counts.resize(waves);
+            } catch (const std::exception&) {  // nothing may throw across the C ABI
+                fail(CBQ_ERR_OUT_OF_MEMORY);
+            }
+            if (st == CBQ_OK &&
+                !ok(cudaMemcpyAsync(h_counts.data(), counts, waves * sizeof(uint64_t), cudaMemcpyDeviceToHost, s)))
+                fail(CBQ_ERR_CUDA);
+        }
     }
-    cudaFree(base);
+    // The workspace is this frame's until everything on it is done.
+    if (!ok(cudaStreamSynchronize(s))) fail(CBQ_ERR_CUDA);
+    if (ahead && st != CBQ_OK) {
+        cudaStreamSynchronize(sw);
+        cudaStreamSynchronize(ss);
+        cudaGetLastError();
+    }
+    for (size_t w = 0; w < h_counts.size() && st == CBQ_OK; w++) {
+        shadow_rays += (uint32_t)h_counts[w];
+        ext_rays += h_counts[w] >> 32;
+    }
+    if (!lock.owns_lock()) cbq::pt_workspace_release(own);
+    else if (ws.bytes > cbq::kPtKeptBytes) release_memory(ws);
     if (stats) {
         stats->extension_rays = ext_rays;
         stats->shadow_rays = shadow_rays;
