@@ -1,12 +1,12 @@
 // Device-side C ABI: DAG upload, traversal launches (plain and persistent).
 #include "cbq_flat.cuh"
 #include "cbq_internal.hpp"
+#include "cbq_stage.cuh"
 #include "cbq_traverse.cuh"
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstring>
 #include <exception>
 #include <new>
@@ -97,58 +97,82 @@ dev::HitsOut make_hits(const cbq_hits* h)
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-// One chunk of a cbq_intersect_host call.  The call's rays are cut into blocks of
-// `block` consecutive rays dealt round-robin to the chunks (block b to chunk
-// b % chunks), so that every chunk samples the whole batch: a camera batch whose
-// first rows are sky and whose middle rows are terrain gives chunks of equal work,
-// and the copies and traversals of consecutive chunks stay balanced.  On the
-// device a chunk's rays and hits are contiguous, from ray `start`; on the host its
-// full blocks are the rows of a pitched array, and the batch's last, partial block
-// (if this chunk has it) is copied on its own.
+// One chunk of a cbq_intersect_host call.  The call's rays are cut into
+// kHostBlocksPerChunk blocks of `pitch` consecutive rays, and every chunk takes
+// `width` rays of each (its rows), from `offset` in the block: so every chunk
+// samples the whole batch (a camera batch whose first rows are sky and whose
+// middle rows are terrain), and the copies and traversals of consecutive chunks
+// stay in proportion.  The rays after the last block go to the last chunk.  On
+// the device a chunk's rays and hits are contiguous, from ray `start`; on the
+// host its rows are those of a pitched array.
 struct HostChunk {
-    uint64_t block = 1;    // rays per block
-    uint64_t start = 0;    // first ray of the chunk in the device staging
-    uint64_t rows = 0;     // full blocks: host blocks k, k + chunks, ...
-    uint64_t tail = 0;     // rays of the batch's partial last block, if this chunk has it
-    uint64_t tail_at = 0;  // host index of that block's first ray
-    uint64_t rays() const { return rows * block + tail; }
+    uint64_t start = 0, width = 0, offset = 0, pitch = 0, rows = 0;
+    uint64_t tail = 0, tail_at = 0;  // rays after the last block, and the host index of the first
+    uint64_t rays() const { return rows * width + tail; }
 };
 
-HostChunk host_chunk(uint64_t n, uint64_t chunks, uint64_t block, uint64_t k, uint64_t start)
-{
-    const uint64_t full = n / block, rem = n % block;
-    HostChunk c;
-    c.block = block;
-    c.start = start;
-    c.rows = full > k ? (full - k + chunks - 1) / chunks : 0;
-    if (rem != 0 && full % chunks == k) {
-        c.tail = rem;
-        c.tail_at = full * block;
-    }
-    return c;
-}
-
-// Copies `width` bytes per ray of chunk k between the host array (every ray of the
+// Copies `bytes` per ray of a chunk between the host array (every ray of the
 // call) and the device array (the chunk's rays from c.start).
-bool copy_chunk(void* host, void* dev, size_t width, const HostChunk& c, uint64_t k, uint64_t chunks,
-                cudaMemcpyKind kind, cudaStream_t s)
+bool copy_chunk(void* host, void* dev, size_t bytes, const HostChunk& c, cudaMemcpyKind kind, cudaStream_t s)
 {
-    char* h = (char*)host;
-    char* d = (char*)dev + c.start * width;
-    const size_t row = c.block * width;
+    char* h = (char*)host + c.offset * bytes;
+    char* d = (char*)dev + c.start * bytes;
+    const size_t row = c.width * bytes, pitch = c.pitch * bytes;
     const bool in = kind == cudaMemcpyHostToDevice;
-    if (c.rows != 0) {
-        char* hr = h + k * row;
-        const cudaError_t e = in ? cudaMemcpy2DAsync(d, row, hr, chunks * row, row, c.rows, kind, s)
-                                 : cudaMemcpy2DAsync(hr, chunks * row, d, row, row, c.rows, kind, s);
+    if (row != 0) {
+        const cudaError_t e = in ? cudaMemcpy2DAsync(d, row, h, pitch, row, c.rows, kind, s)
+                                 : cudaMemcpy2DAsync(h, pitch, d, row, row, c.rows, kind, s);
         if (e != cudaSuccess) return false;
     }
     if (c.tail != 0) {
-        char* ht = h + c.tail_at * width;
+        char* ht = (char*)host + c.tail_at * bytes;
         char* dt = d + c.rows * row;
-        const cudaError_t e = in ? cudaMemcpyAsync(dt, ht, c.tail * width, kind, s)
-                                 : cudaMemcpyAsync(ht, dt, c.tail * width, kind, s);
+        const cudaError_t e = in ? cudaMemcpyAsync(dt, ht, c.tail * bytes, kind, s)
+                                 : cudaMemcpyAsync(ht, dt, c.tail * bytes, kind, s);
         if (e != cudaSuccess) return false;
+    }
+    return true;
+}
+
+// The copies of a call in one chunk with page-locked buffers: one kernel each way.
+struct HostOut {
+    StageOut row[kHitFields];
+};
+__global__ void __launch_bounds__(kStageBlock) cbq_k_host_in(const __grid_constant__ StageIn in)
+{
+    dev::stage_in(in, (uint64_t)blockIdx.x * kStageBlock + threadIdx.x, (uint64_t)gridDim.x * kStageBlock);
+}
+// Row y of the grid copies out.row[y].
+__global__ void __launch_bounds__(kStageBlock) cbq_k_host_out(const __grid_constant__ HostOut out)
+{
+    dev::stage_out(out.row[blockIdx.y], (uint64_t)blockIdx.x * kStageBlock + threadIdx.x,
+                   (uint64_t)gridDim.x * kStageBlock);
+}
+
+// The two copies of a call of n rays, where all its buffers are page-locked (and the rays
+// 16-byte aligned); false otherwise.
+bool host_staging(const float* o, const float* d, uint64_t n, const cbq_hits& h, float* d_o, float* d_d,
+                  const cbq_hits& dh, StageIn* in, HostOut* out, int* rows)
+{
+    if (!aligned16(o) || !aligned16(d)) return false;
+    const void *ao = device_alias(o), *ad = ao ? device_alias(d) : nullptr;
+    if (!ad) return false;
+    *in = StageIn{(const float4*)ao, (const float4*)ad, (float4*)d_o, (float4*)d_d, n, 0};
+    struct Field {
+        void* host;
+        const void* dev;
+        uint64_t width;
+    };
+    const Field fields[kHitFields] = {{h.hit, dh.hit, 1},           {h.distance, dh.distance, 4},
+                                      {h.material, dh.material, 4}, {h.position, dh.position, 12},
+                                      {h.normal, dh.normal, 12},    {h.voxel, dh.voxel, 12},
+                                      {h.status, dh.status, 1}};
+    *rows = 0;
+    for (const Field& f : fields) {
+        if (!f.host) continue;
+        char* host = (char*)device_alias(f.host);
+        if (!host) return false;
+        out->row[(*rows)++] = StageOut{(const char*)f.dev, host, n * f.width};
     }
     return true;
 }
@@ -645,13 +669,6 @@ cbq_status intersect_device_count(const cbq_dag* dag, const cbq_rays* rays, uint
 
 namespace {
 
-// cbq_intersect_host calls in flight in this process (any DAG).
-std::atomic<int> g_host_calls{0};
-struct HostCallCount {
-    HostCallCount() { g_host_calls.fetch_add(1, std::memory_order_relaxed); }
-    ~HostCallCount() { g_host_calls.fetch_sub(1, std::memory_order_relaxed); }
-};
-
 // Takes a staging set of `dag` for one call, locked: a free one, else a new
 // one while fewer than kHostStagesMax exist, else the first (waiting for it).
 std::unique_lock<std::mutex> take_stage(cbq_dag* dag, HostStage** out)
@@ -697,7 +714,6 @@ extern "C" cbq_status cbq_intersect_host(const cbq_dag* cdag, const float* host_
 {
     if (!cdag || !host_origin_tmax || !host_direction || !host_hits) return CBQ_ERR_INVALID_ARGUMENT;
     if (n == 0) return CBQ_OK;
-    const HostCallCount in_flight;
     cbq_dag* dag = const_cast<cbq_dag*>(cdag);
     HostStage* hs = nullptr;
     std::unique_lock<std::mutex> lock = take_stage(dag, &hs);
@@ -746,17 +762,6 @@ extern "C" cbq_status cbq_intersect_host(const cbq_dag* cdag, const float* host_
     p += n;
     // Work counters, one 64-byte line per chunk.
     uint64_t* d_counters = (uint64_t*)(((uintptr_t)p + 255u) & ~(uintptr_t)255u);
-    // Chunks pipeline the copies with the traversal: while chunk k is traversed, chunk k + 1 is
-    // copied in and chunk k - 1 copied out.  Consecutive chunks are traversed on alternating
-    // streams, so the next chunk's blocks fill the SMs while the previous launch drains (a
-    // persistent launch ends with a tail of few busy warps).  Events order each chunk's copy in,
-    // traversal and copy out.  Chunks interleave blocks of the batch (HostChunk).  Measured on
-    // terrain-4096 (primary and bounce calls, 4 Mi rays each): alone, 8 chunks per call (3.0
-    // Grays/s end to end; 2.9 with 4); with the two batches' calls from two threads, 4 chunks
-    // (4.25 against 3.9 with 8).
-    const uint64_t cmax =
-        g_host_calls.load(std::memory_order_relaxed) > 1 ? kHostChunksConcurrent : kHostChunksMax;
-    const uint64_t chunks = std::min<uint64_t>(cmax, std::max<uint64_t>(1, n / kHostChunkMin));
     cudaStream_t s_in = hs->pipe[0], s_out = hs->pipe[1];
     // Every queued copy and launch ends before the call returns (the staging buffers are reused).
     auto drain = [&](cbq_status st) {
@@ -764,17 +769,65 @@ extern "C" cbq_status cbq_intersect_host(const cbq_dag* cdag, const float* host_
         for (cudaStream_t s : hs->pipe) ok = cudaStreamSynchronize(s) == cudaSuccess && ok;
         return ok ? st : CBQ_ERR_CUDA;
     };
-    const uint64_t block = std::max<uint64_t>(kHostBlockMin, n / (chunks * kHostBlocksPerChunk));
-    uint64_t start = 0;
+    // Chunks pipeline the copies with the traversal: while chunk k is traversed, chunk k + 1 is
+    // copied in and chunk k - 1 copied out.  Consecutive chunks are traversed on alternating
+    // streams, so the next chunk's blocks fill the SMs while the previous launch drains (a
+    // persistent launch ends with a tail of few busy warps).  Events order each chunk's copy in,
+    // traversal and copy out.  The copies out take longest, so the first chunks are the smallest:
+    // the copies out then begin early and the larger chunks are traversed under them.  us per
+    // call of 300 Ki / 1 Mi / 4 Mi bounce rays: chunks of 1:2:3:4 238 / 494 / 1,399; up to 8 equal
+    // ones of 256 Ki rays or more 259 / 528 / 1,498, up to 8 of 1:2:3:4:4:.. 235 / 507 / 1,450.
+    static const unsigned weights[kHostChunksMax] = {1, 2, 3, 4};
+    uint64_t chunks = 1, sum = weights[0];
+    while (chunks < kHostChunksMax && n >= kHostChunkMin * (sum + weights[chunks])) sum += weights[chunks++];
+    StageIn stage_rays;
+    HostOut stage_hits;
+    int stage_rows = 0;
+    if (chunks == 1 && host_staging(host_origin_tmax, host_direction, n, *host_hits, d_o, d_d, dh, &stage_rays,
+                                    &stage_hits, &stage_rows)) {
+        // One chunk of page-locked buffers: a copy kernel in, the traversal and a copy kernel out
+        // in a row on one stream.
+        cudaStream_t s = hs->pipe[2];
+        cbq_k_host_in<<<stage_blocks(2 * n), kStageBlock, 0, s>>>(stage_rays);
+        if (cudaGetLastError() != cudaSuccess) return drain(CBQ_ERR_CUDA);
+        cbq_rays rays{d_o, d_d};
+        cbq_hits launch = dh;
+        if (!host_hits->hit) launch.hit = nullptr;
+        if (!host_hits->distance) launch.distance = nullptr;
+        if (!host_hits->material) launch.material = nullptr;
+        if (!host_hits->position) launch.position = nullptr;
+        if (!host_hits->normal) launch.normal = nullptr;
+        if (!host_hits->voxel) launch.voxel = nullptr;
+        if (!host_hits->status) launch.status = nullptr;
+        const cbq_status st = cbq_intersect_persistent(dag, &rays, n, query, &launch, d_counters, 0u, (cbq_stream_t)s);
+        if (st != CBQ_OK) return drain(st);
+        if (stage_rows != 0) {
+            cbq_k_host_out<<<dim3(stage_blocks(n * 12 / 16), stage_rows), kStageBlock, 0, s>>>(stage_hits);
+            if (cudaGetLastError() != cudaSuccess) return drain(CBQ_ERR_CUDA);
+        }
+        return cudaStreamSynchronize(s) == cudaSuccess ? CBQ_OK : CBQ_ERR_CUDA;
+    }
+    const uint64_t blocks = chunks == 1 ? 1 : kHostBlocksPerChunk, pitch = n / blocks;
+    uint64_t offset = 0, start = 0;
     for (uint64_t k = 0; k < chunks; k++) {
-        const HostChunk hc = host_chunk(n, chunks, block, k, start);
+        HostChunk hc;
+        hc.start = start;
+        hc.offset = offset;
+        hc.pitch = pitch;
+        hc.rows = blocks;
+        hc.width = k + 1 < chunks ? pitch * weights[k] / sum / 32 * 32 : pitch - offset;
+        if (k + 1 == chunks) {
+            hc.tail_at = blocks * pitch;
+            hc.tail = n - hc.tail_at;
+        }
+        offset += hc.width;
         const uint64_t a = start, m = hc.rays();
         start += m;
         if (m == 0) continue;
         cudaStream_t s_run = hs->pipe[2 + (k & 1)];
         cudaEvent_t copied = hs->pipe_ev[2 * k], traversed = hs->pipe_ev[2 * k + 1];
-        if (!copy_chunk((void*)host_origin_tmax, d_o, 16, hc, k, chunks, cudaMemcpyHostToDevice, s_in) ||
-            !copy_chunk((void*)host_direction, d_d, 16, hc, k, chunks, cudaMemcpyHostToDevice, s_in) ||
+        if (!copy_chunk((void*)host_origin_tmax, d_o, 16, hc, cudaMemcpyHostToDevice, s_in) ||
+            !copy_chunk((void*)host_direction, d_d, 16, hc, cudaMemcpyHostToDevice, s_in) ||
             cudaEventRecord(copied, s_in) != cudaSuccess || cudaStreamWaitEvent(s_run, copied, 0) != cudaSuccess)
             return drain(CBQ_ERR_CUDA);
         cbq_hits launch;
@@ -803,8 +856,7 @@ extern "C" cbq_status cbq_intersect_host(const cbq_dag* cdag, const float* host_
                                {host_hits->status, dh.status, 1}};
         for (const Copy& c : copies) {
             if (!c.host) continue;
-            if (!copy_chunk(c.host, c.dev, c.width, hc, k, chunks, cudaMemcpyDeviceToHost, s_out))
-                return drain(CBQ_ERR_CUDA);
+            if (!copy_chunk(c.host, c.dev, c.width, hc, cudaMemcpyDeviceToHost, s_out)) return drain(CBQ_ERR_CUDA);
         }
     }
     return drain(CBQ_OK);

@@ -59,17 +59,12 @@ cbq_status noalloc_prepare(int device);
 // beyond that they queue for one.
 constexpr int kHostStagesMax = 4;
 
-// cbq_intersect_host splits a call into at most kHostChunksMax chunks of at
-// least kHostChunkMin rays; kHostChunksConcurrent while another call is in
-// flight in the process (its copies and traversals fill the gaps that smaller
-// chunks would, so fewer persistent-launch tails pay more).
-constexpr uint64_t kHostChunksMax = 8;
-constexpr uint64_t kHostChunksConcurrent = 4;
-constexpr uint64_t kHostChunkMin = 1ull << 18;
-// ... each made of about kHostBlocksPerChunk blocks of consecutive rays (at least
-// kHostBlockMin) dealt round-robin.
+// cbq_intersect_host splits a call into at most kHostChunksMax chunks, the first
+// of at least kHostChunkMin rays.
+constexpr uint64_t kHostChunksMax = 4;
+constexpr uint64_t kHostChunkMin = 1ull << 16;
+// Blocks of the batch that every chunk takes a part of.
 constexpr uint64_t kHostBlocksPerChunk = 4;
-constexpr uint64_t kHostBlockMin = 4096;
 
 // Device staging and streams of one cbq_intersect_host call at a time: rays and
 // hits, copied in and out in chunks on four streams (copy in, copy out, two for

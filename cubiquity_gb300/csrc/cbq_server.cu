@@ -18,6 +18,7 @@
 // Nothing on the device waits on the host: every launch finishes on its own,
 // and host waits are on CUDA events or condition variables.
 #include "cbq_batch.cuh"
+#include "cbq_stage.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -63,20 +64,6 @@ struct Request {
     cbq_status status = CBQ_OK;
 };
 
-// The device address of host memory the GPU can use directly (page-locked and
-// mapped, or managed), or nullptr when the buffer has to be staged.
-const void* device_alias(const void* p)
-{
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (a.type == cudaMemoryTypeHost && a.devicePointer) return a.devicePointer;
-    if (a.type == cudaMemoryTypeManaged) return p;
-    return nullptr;
-}
-
 // True when a device-to-host copy into `p` is asynchronous: page-locked or
 // managed host memory (into pageable memory the copy blocks the calling thread).
 bool copy_into_is_async(const void* p)
@@ -116,28 +103,11 @@ void resolve_buffers(Request& rq)
     }
 }
 
-// Copies of a launch between its requests' page-locked buffers and the pool.
-// The copy engine took two copies in, the job table, the counter's memset and
-// up to seven copies out per request, each a call of 2-4 us on the launching
-// thread and a few us of the stream's time.  Two kernels do all of it for
-// every request of a launch: 24 requests of 1 Ki to 64 Ki rays submitted from
-// one Python thread 1,040 -> 828 us (median latency of one 136 -> 107 us).
-// They are bound by the host link and their launches; 16-byte accesses by whole
-// warps on the host side, so that the link carries full lines.
-struct StageIn {
-    const float4 *o, *d;   // host rays
-    float4 *dst_o, *dst_d;
-    uint64_t count;
-    uint64_t pad;
-};
-struct StageOut {
-    const char* src;       // pool, 4-byte aligned
-    char* dst;             // host, any alignment
-    uint64_t bytes;
-};
-constexpr int kStageBlock = 256;
+// Copies of a launch between its requests' page-locked buffers and the pool, two
+// kernels for every request of a launch (cbq_stage.cuh): 24 requests of 1 Ki to
+// 64 Ki rays submitted from one Python thread 1,040 -> 828 us (median latency of
+// one 136 -> 107 us) against the copy engine's calls.
 constexpr uint64_t kStageRequestsMax = 4096;  // per launch: seven times that are grid rows
-constexpr int kHitFields = 7;
 
 // Row y of the grid copies the rays of in[y]; the last row the job table (in
 // 8-byte words) and the zero of the work counter.
@@ -153,47 +123,14 @@ __global__ void __launch_bounds__(kStageBlock) cbq_k_stage_in(const StageIn* __r
         for (uint64_t i = first; i < table_words; i += stride) d_table[i] = __ldcs(h_table + i);
         return;
     }
-    const StageIn s = in[blockIdx.y];
-    for (uint64_t i = first; i < s.count; i += stride) {
-        const float4 o = __ldcs(s.o + i), d = __ldcs(s.d + i);
-        s.dst_o[i] = o;
-        s.dst_d[i] = d;
-    }
+    dev::stage_in(in[blockIdx.y], first, stride);
 }
 
-// Row y copies out[y]: 16-byte stores to the host side, the source words
-// shifted into place where the two sides' alignments differ; the unaligned
-// ends byte by byte.  Reads at most 3 bytes beyond the source's end, which the
-// pool's padding covers.
+// Row y copies out[y].  (The pool's padding covers the reads beyond a source's end.)
 __global__ void __launch_bounds__(kStageBlock) cbq_k_stage_out(const StageOut* __restrict__ out)
 {
-    const StageOut s = out[blockIdx.y];
-    const uint64_t first = (uint64_t)blockIdx.x * kStageBlock + threadIdx.x;
-    const uint64_t stride = (uint64_t)gridDim.x * kStageBlock;
-    const uint64_t lead = (16u - ((uintptr_t)s.dst & 15u)) & 15u, head = lead < s.bytes ? lead : s.bytes;
-    const uint64_t body = (s.bytes - head) / 16u, tail = head + body * 16u;
-    if (first < head) s.dst[first] = s.src[first];
-    if (first < s.bytes - tail) s.dst[tail + first] = s.src[tail + first];
-    const uint32_t* words = (const uint32_t*)(s.src + (head & ~(uint64_t)3u));
-    const uint32_t shift = (uint32_t)(head & 3u) * 8u;
-    uint4* dst = (uint4*)(s.dst + head);
-    for (uint64_t i = first; i < body; i += stride) {
-        const uint32_t* w = words + 4 * i;
-        uint4 v = make_uint4(__ldcs(w), __ldcs(w + 1), __ldcs(w + 2), __ldcs(w + 3));
-        if (shift != 0u) {
-            const uint32_t next = __ldcs(w + 4);
-            v = make_uint4(__funnelshift_r(v.x, v.y, shift), __funnelshift_r(v.y, v.z, shift),
-                           __funnelshift_r(v.z, v.w, shift), __funnelshift_r(v.w, next, shift));
-        }
-        dst[i] = v;
-    }
-}
-
-// Blocks per row for rows of up to `items` 16-byte accesses: two per thread,
-// at most 64 (16,384 threads keep enough lines in flight for the host link).
-unsigned stage_blocks(uint64_t items)
-{
-    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(64, (items + 2 * kStageBlock - 1) / (2 * kStageBlock)));
+    dev::stage_out(out[blockIdx.y], (uint64_t)blockIdx.x * kStageBlock + threadIdx.x,
+                   (uint64_t)gridDim.x * kStageBlock);
 }
 
 // First-fit allocator over [0, size).

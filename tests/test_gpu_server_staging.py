@@ -85,3 +85,21 @@ def test_mixed_buffers_in_one_server(scene):
         assert server.wait(ticket, 20_000_000) == 0
         _check(whole, shift, want)
     server.close()
+
+
+@pytest.mark.parametrize("n", [1, 3, 16, 33, 65536, 196607, 196608, 393216, 655359, 655360, 655361])
+def test_host_call_chunks(scene, n):
+    """The host entry point around the sizes where its chunk count changes (the first of chunks
+    1:2:3:4 has 65,536 rays at least), with page-locked and pageable buffers, all fields and two."""
+    dag, co, cd = scene
+    o = np.resize(co, (n, 4)).astype(np.float32)
+    d = np.resize(cd, (n, 4)).astype(np.float32)
+    o[:, 3] += np.arange(n, dtype=np.float32) % 7  # rays that differ from one copy to the next
+    dev = cbq.intersect_volume(dag, torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda(), use_tmax=True)
+    want = {k: v.cpu().numpy() for k, v in dev.items()}
+    want["material"] = want["material"].astype(np.uint32)
+    for pinned, shift, fields in ((True, 0, cbq.HIT_FIELDS), (True, 5, ("hit", "position")), (False, 0, cbq.HIT_FIELDS)):
+        whole, out = _buffers(n, shift, fields, pinned)
+        po, pd = (_pin(o), _pin(d)) if pinned else (o, d)
+        cbq.intersect_volume_host(dag, po, pd, use_tmax=True, out=out)
+        _check(whole, shift, want)
