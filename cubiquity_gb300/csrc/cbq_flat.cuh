@@ -377,6 +377,80 @@ __device__ __forceinline__ uint32_t walk_child(const uint32_t* __restrict__ node
     }
 }
 
+// An ordered ray enters SubDAG `s`, whose reflected corner is (px, py, pz) and
+// whose size is ns.
+//
+// Origin inside (entry <= 0 < exit): descend to the cell that holds it here,
+// with all of a refill's lanes in step.  Every cell on the way has entry <= 0 <
+// tChildExit, so the first child is the one that holds the origin: its slot is a
+// bit of each of the origin's voxel coordinates, and no distance is needed
+// (terrain-4096 bounce rays make 8.1 of their 17.2 descents here; by distances
+// and positions as in the walk the descent took a third more instructions:
+// bounce rays 550 -> 536 us, 1.5 M shadow rays 134 -> 129, a path-traced frame
+// 900 -> 878).  Origin outside: the slab test, and the first child by one
+// compare per axis.
+template <typename Src, typename Stack>
+__device__ __forceinline__ void enter_ordered(Lane& L, const Src& c, Stack& stack, const SubDag& s, int32_t px,
+                                              int32_t py, int32_t pz, uint32_t ns)
+{
+    constexpr Store S = Src::kStore;
+    constexpr uint32_t kBiasBits = 0x4B400000u;  // of kPosBias
+    const uint32_t mx = (uint32_t)(__float2int_rd(L.rox) - px), my = (uint32_t)(__float2int_rd(L.roy) - py),
+                   mz = (uint32_t)(__float2int_rd(L.roz) - pz);
+    L.node = S == Store::kPlain ? s.node * 8u : s.node;  // plain: the word index of its children
+    // With LOD, a cell of size s that holds the origin has tChildExit <= s * min(1 / |dir|):
+    // where that minimum is within footprint_tmax all of them are large.
+    bool inside = (mx | my | mz) < ns && s.height > 0;
+    if constexpr (Src::kLod) inside = inside && fminf(fminf(L.ix, L.iy), L.iz) <= c.query(L).footprint_tmax;
+    if (inside) {
+        const uint32_t* nodes = c.nodes(L);
+        int l = s.height - 1;  // the cell's size is 1 << l
+        uint32_t slot;
+        L.h = (int)stack.at(s.height);
+        stack.store((uint32_t)L.h, L.node);
+        for (;;) {
+            const uint32_t m = 1u << l;
+            slot = (((mx & m) + ((my & m) << 1) + ((mz & m) << 2)) >> l) ^ L.sign;
+            if (!walk_occupied<S>(nodes, L.node, slot)) break;
+            const uint32_t child = walk_child<S>(nodes, L.node, slot);
+            if (child < kMaterialCount) break;  // fetched again by the walk
+            L.node = S == Store::kPlain ? child * 8u : child;
+            L.h = (int)stack.below((uint32_t)L.h);
+            stack.store((uint32_t)L.h, L.node);
+            l--;
+        }
+        const uint32_t keep = 0u - (1u << l);
+        L.cid = slot;
+        L.fcns = __uint_as_float((uint32_t)(127 + l) << 23);  // 2^l
+        L.fx = __uint_as_float(kBiasBits + (uint32_t)px + (mx & keep));
+        L.fy = __uint_as_float(kBiasBits + (uint32_t)py + (my & keep));
+        L.fz = __uint_as_float(kBiasBits + (uint32_t)pz + (mz & keep));
+        L.last_exit = 0.0f;  // an entry at or behind the origin
+    } else {
+        const float fpx = (float)px, fpy = (float)py, fpz = (float)pz, fns = (float)ns;
+        const float entry = fmaxf(fmaxf((fpx - L.rox) * L.ix, (fpy - L.roy) * L.iy), (fpz - L.roz) * L.iz);
+        const float exit_ = fminf(fminf(((fpx + fns) - L.rox) * L.ix, ((fpy + fns) - L.roy) * L.iy),
+                                  ((fpz + fns) - L.roz) * L.iz);
+        if (!(entry < exit_)) {
+            L.mode = kLaneNext;
+            return;
+        }
+        L.fcns = (float)(ns >> 1);
+        const float te = fmaxf(entry, FLT_MIN);
+        const float cx = fpx + L.fcns, cy = fpy + L.fcns, cz = fpz + L.fcns;
+        const bool bx = (cx - L.rox) * L.ix < te, by = (cy - L.roy) * L.iy < te, bz = (cz - L.roz) * L.iz < te;
+        L.cid = ((uint32_t)bx | ((uint32_t)by << 1) | ((uint32_t)bz << 2)) ^ L.sign;
+        L.fx = (bx ? cx : fpx) + kPosBias;
+        L.fy = (by ? cy : fpy) + kPosBias;
+        L.fz = (bz ? cz : fpz) + kPosBias;
+        L.last_exit = entry;
+        L.h = (int)stack.at(s.height);
+        if (s.height > 0) stack.store((uint32_t)L.h, L.node);
+    }
+    L.fetches += 64u;  // more than were made here
+    L.mode = kLaneWalk;
+}
+
 // Enters the SubDAG of the current octant: the slab test and set-up at the top
 // of intersectRayNodeESVO (raytracing.cpp:218-250, 443-460).
 template <typename Src, typename Stack>
@@ -392,6 +466,13 @@ __device__ __forceinline__ void lane_enter(Lane& L, const Src& c, Stack& stack)
     const int32_t px = (int32_t)((sbx ? 0u - (uint32_t)s.lx : (uint32_t)s.lx) - (sbx ? ns : 0u));
     const int32_t py = (int32_t)((sby ? 0u - (uint32_t)s.ly : (uint32_t)s.ly) - (sby ? ns : 0u));
     const int32_t pz = (int32_t)((sbz ? 0u - (uint32_t)s.lz : (uint32_t)s.lz) - (sbz ? ns : 0u));
+    L.limit = ns;
+    if constexpr (!Src::kIntPos) {
+        if (L.fast) {
+            enter_ordered(L, c, stack, s, px, py, pz, ns);
+            return;
+        }
+    }
     const float fpx = (float)px, fpy = (float)py, fpz = (float)pz, fns = (float)ns;
     const float t0x = (fpx - L.rox) * L.ix;
     const float t0y = (fpy - L.roy) * L.iy;
@@ -406,67 +487,23 @@ __device__ __forceinline__ void lane_enter(Lane& L, const Src& c, Stack& stack)
         return;
     }
     L.node = s.node;
-    L.limit = ns;
     L.mode = kLaneWalk;
+    L.h = s.height;
+    L.last_exit = exit_;
     if constexpr (Src::kIntPos) {
-        L.h = s.height;
         L.cns = (int32_t)(ns >> 1);
         L.cid = first_child_f(L, entry, (float)wadd(px, L.cns), (float)wadd(py, L.cns), (float)wadd(pz, L.cns));
         L.px = wadd(px, (L.cid & 1u) ? L.cns : 0);
         L.py = wadd(py, (L.cid & 2u) ? L.cns : 0);
         L.pz = wadd(pz, (L.cid & 4u) ? L.cns : 0);
-        L.last_exit = exit_;
-        stack.clear(s.height);
     } else {
         L.fcns = (float)(ns >> 1);
         L.cid = first_child_f(L, entry, fpx + L.fcns, fpy + L.fcns, fpz + L.fcns);
         L.fx = fpx + ((L.cid & 1u) ? L.fcns : 0.0f);
         L.fy = fpy + ((L.cid & 2u) ? L.fcns : 0.0f);
         L.fz = fpz + ((L.cid & 4u) ? L.fcns : 0.0f);
-        if (L.fast) {
-            L.last_exit = entry;
-            L.cid ^= L.sign;
-            L.fx += kPosBias;
-            L.fy += kPosBias;
-            L.fz += kPosBias;
-            if (Src::kStore == Store::kPlain) L.node *= 8u;  // the word index of its children
-            L.h = (int)stack.at(s.height);
-            if (s.height > 0) stack.store((uint32_t)L.h, L.node);
-            // Origin inside the SubDAG: descend to the cell that holds it here,
-            // with all of a refill's lanes in step.  Every cell on the way has
-            // entry <= 0 < tChildExit, so the first child is the one that holds
-            // the origin and no distance is needed (terrain-4096 bounce rays:
-            // 8.9 of 18 descents; 774 -> 744 us when it was added).
-            if (entry <= 0.0f && exit_ > 0.0f) {
-                const uint32_t* nodes = c.nodes(L);
-                while (walk_occupied<Src::kStore>(nodes, L.node, L.cid)) {
-                    if constexpr (Src::kLod) {
-                        const float sb = L.fcns - kPosBias;
-                        const float tcx = fminf(fminf(((L.fx + sb) - L.rox) * L.ix, ((L.fy + sb) - L.roy) * L.iy),
-                                                ((L.fz + sb) - L.roz) * L.iz);
-                        if (!(tcx <= L.fcns * c.query(L).footprint_tmax)) break;
-                    }
-                    const uint32_t child = walk_child<Src::kStore>(nodes, L.node, L.cid);
-                    if (child < kMaterialCount) break;  // fetched again by the walk
-                    L.node = Src::kStore == Store::kPlain ? child * 8u : child;
-                    L.h = (int)stack.below((uint32_t)L.h);
-                    stack.store((uint32_t)L.h, L.node);
-                    L.fcns *= 0.5f;
-                    const float sb = L.fcns - kPosBias;
-                    const bool bx = L.rox >= L.fx + sb, by = L.roy >= L.fy + sb, bz = L.roz >= L.fz + sb;
-                    L.cid = ((uint32_t)bx | ((uint32_t)by << 1) | ((uint32_t)bz << 2)) ^ L.sign;
-                    if (bx) L.fx += L.fcns;
-                    if (by) L.fy += L.fcns;
-                    if (bz) L.fz += L.fcns;
-                }
-            }
-            L.fetches += 64u;  // more than were made here
-        } else {
-            L.last_exit = exit_;
-            L.h = s.height;
-            stack.clear(s.height);
-        }
     }
+    stack.clear(s.height);
 }
 
 // min3/max3 of slab distances: the reference's NaN-ordered forms, or (FAST,
