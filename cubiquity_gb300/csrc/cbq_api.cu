@@ -59,6 +59,7 @@ dev::DagParams make_dag_params(const cbq_dag* dag)
     dev::DagParams p;
     p.nodes = dag->d_nodes;
     p.occupied = 0u;
+    p.top = (const uint4*)dag->d_top;
     for (int i = 0; i < 8; i++) {
         if (dag->sd_ref[i] != 0u) p.occupied |= 1u << i;
         p.sd[i].lx = dag->subdags[i].lower_bound[0];
@@ -66,7 +67,8 @@ dev::DagParams make_dag_params(const cbq_dag* dag)
         p.sd[i].lz = dag->subdags[i].lower_bound[2];
         p.sd[i].height = dag->subdags[i].node_height;
         p.sd[i].node = dag->sd_ref[i];
-        p.sd[i].pad[0] = p.sd[i].pad[1] = p.sd[i].pad[2] = 0;
+        p.sd[i].top = dag->top_index[i];
+        p.sd[i].pad[0] = p.sd[i].pad[1] = 0;
     }
     return p;
 }
@@ -279,7 +281,60 @@ __global__ void __launch_bounds__(256) cbq_k_tag_nodes(const uint4* __restrict__
     }
 }
 
+// The table of upper cells of the SubDAG with root reference `root`: one cell per thread.
+template <dev::Store S>
+__global__ void __launch_bounds__(256) cbq_k_top_table(const uint32_t* __restrict__ nodes, uint32_t root,
+                                                       uint4* __restrict__ table)
+{
+    const uint32_t cell = blockIdx.x * 256u + threadIdx.x;
+    uint32_t path[dev::kTopLevels] = {0u, 0u, 0u, 0u, 0u};
+    uint32_t ref = root, count = 0u, loads = 0u;
+#pragma unroll
+    for (int d = 0; d < dev::kTopLevels; d++) {
+        const int b = dev::kTopLevels - 1 - d;
+        const uint32_t slot = ((cell >> b) & 1u) | (((cell >> (b + 5)) & 1u) << 1) | (((cell >> (b + 10)) & 1u) << 2);
+        const uint32_t child = (int)count == d ? dev::child_of<S>(nodes, ref, slot, loads) : 0u;
+        if (child >= dev::kMaterialCount) {
+            path[d] = ref = child;
+            count++;
+        }
+    }
+    table[2u * cell] = make_uint4(path[0], path[1], path[2], path[3]);
+    table[2u * cell + 1u] = make_uint4(path[4], count, ref, 0u);
+}
+
 namespace {
+
+// Builds the tables of a DAG whose walk store carries masks; without memory for them there
+// are none, and rays descend level by level.
+cbq_status build_top_tables(cbq_dag* dag)
+{
+    uint32_t tables = 0;
+    for (int k = 0; k < 8; k++) {
+        const cbq_subdag& s = dag->subdags[k];
+        const bool has = s.node_index >= dev::kMaterialCount && s.node_height > dev::kTopLevels;
+        dag->top_index[k] = has ? ++tables : 0u;
+    }
+    if (tables == 0) return CBQ_OK;
+    if (cudaMalloc((void**)&dag->d_top, (size_t)tables * dev::kTopCells * 32u) != cudaSuccess) {
+        cudaGetLastError();
+        dag->d_top = nullptr;
+        for (uint32_t& t : dag->top_index) t = 0u;
+        return CBQ_OK;
+    }
+    for (int k = 0; k < 8; k++) {
+        if (!dag->top_index[k]) continue;
+        uint4* table = (uint4*)dag->d_top + 2ull * (dag->top_index[k] - 1u) * dev::kTopCells;
+        if (dag->layout == CBQ_DAG_LAYOUT_COMPACT)
+            cbq_k_top_table<dev::Store::kCompact><<<dev::kTopCells / 256u, 256, 0, cudaStreamLegacy>>>(
+                dag->walk_nodes(), dag->walk_root(k), table);
+        else
+            cbq_k_top_table<dev::Store::kTagged><<<dev::kTopCells / 256u, 256, 0, cudaStreamLegacy>>>(
+                dag->walk_nodes(), dag->walk_root(k), table);
+    }
+    return cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess ? CBQ_OK
+                                                                                                    : CBQ_ERR_CUDA;
+}
 
 cbq_status preload_nested_persistent()
 {
@@ -372,6 +427,10 @@ cbq_status cbq_dag_create_ex(const uint32_t* host_nodes, uint64_t node_count, ui
             dag->tagged_ref[i] = r == 0u ? 0u : (r << 8) | mask;
         }
     }
+    if (dag->batch_ok() && build_top_tables(dag) != CBQ_OK) {
+        cbq_dag_destroy(dag);
+        return CBQ_ERR_CUDA;
+    }
     cbq::log(CBQ_LOG_INFO,
              "DAG uploaded to device %d: %llu nodes, %s layout (%.1f MB), root %u, max sub-DAG height %d, %s kernel",
              dag->device, (unsigned long long)node_count,
@@ -386,6 +445,7 @@ cbq_status cbq_dag_destroy(cbq_dag* dag)
     if (!dag) return CBQ_ERR_INVALID_ARGUMENT;
     cudaFree(dag->d_nodes);
     if (dag->d_tagged) cudaFree(dag->d_tagged);
+    if (dag->d_top) cudaFree(dag->d_top);
     for (auto& kv : dag->stream_counters) cudaFree(kv.second);
     pt_workspace_release(dag->pt);
     for (auto& hs : dag->stages) {

@@ -29,6 +29,7 @@ struct BatchSrc {
     __device__ __forceinline__ const QueryParams& query(const Lane& L) const { return jobs[L.job].q; }
     __device__ __forceinline__ const uint32_t* nodes(const Lane& L) const { return L.nodes; }
     __device__ __forceinline__ uint32_t occupied(const Lane& L) const { return jobs[L.job].occupied; }
+    __device__ __forceinline__ const uint4* top(const Lane& L) const { return jobs[L.job].top; }
     __device__ __forceinline__ const SubDag& subdag(const Lane& L, uint32_t k) const { return jobs[L.job].sd[k]; }
     // Rays are read once (from device or page-locked host memory): streaming loads.
     __device__ __forceinline__ float4 ray_origin(const Lane& L, uint64_t i) const { return __ldcs(jobs[L.job].orig + i); }
@@ -197,6 +198,7 @@ void fill_job_volume(dev::JobDesc& d, const cbq_dag* dag)
 {
     d.nodes = dag->walk_nodes();
     d.occupied = 0u;
+    d.top = (const uint4*)dag->d_top;
     for (int k = 0; k < 8; k++) {
         if (dag->walk_root(k) != 0u) d.occupied |= 1u << k;
         const cbq_subdag& s = dag->subdags[k];
@@ -205,7 +207,8 @@ void fill_job_volume(dev::JobDesc& d, const cbq_dag* dag)
         d.sd[k].lz = s.lower_bound[2];
         d.sd[k].height = s.node_height;
         d.sd[k].node = dag->walk_root(k);
-        d.sd[k].pad[0] = d.sd[k].pad[1] = d.sd[k].pad[2] = 0;
+        d.sd[k].top = dag->top_index[k];
+        d.sd[k].pad[0] = d.sd[k].pad[1] = 0;
     }
 }
 

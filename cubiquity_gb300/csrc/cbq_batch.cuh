@@ -21,6 +21,7 @@ struct JobDesc {
     uint64_t count;
     QueryParams q;
     uint32_t occupied;  // bit k: SubDAG k is not empty
+    const uint4* top;   // the volume's tables of upper cells
     SubDag sd[8];
 };
 

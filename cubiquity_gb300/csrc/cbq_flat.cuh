@@ -124,6 +124,7 @@ struct FlatCtxT {
         return (uint64_t)(band * 8u + (k >> 2)) * w + col * 4u + (k & 3u);
     }
     __device__ __forceinline__ uint32_t occupied(const Lane&) const { return dag.occupied; }
+    __device__ __forceinline__ const uint4* top(const Lane&) const { return dag.top; }
     __device__ __forceinline__ const SubDag& subdag(const Lane&, uint32_t k) const { return dag.sd[k]; }
     // Rays are read once: streaming loads (evict-first) leave L2 to the node store.
     __device__ __forceinline__ float4 ray_origin(const Lane&, uint64_t i) const { return __ldcs(orig + i); }
@@ -408,6 +409,27 @@ __device__ __forceinline__ void enter_ordered(Lane& L, const Src& c, Stack& stac
         uint32_t slot;
         L.h = (int)stack.at(s.height);
         stack.store((uint32_t)L.h, L.node);
+        if (S != Store::kPlain && s.top != 0u) {
+            // The first five levels at once, from the table: two loads instead of a
+            // chain of five (bounce rays 536 -> 519 us, shadow rays 129 -> 124, the
+            // compact store 152 -> 146).  Slots below the last node get the row's
+            // empty entries: they are stored again before they are read.
+            const uint32_t flip = ns - 1u;
+            const int sh = s.height - kTopLevels;
+            const uint32_t ux = (mx ^ ((L.sign & 1u) ? flip : 0u)) >> sh, uy = (my ^ ((L.sign & 2u) ? flip : 0u)) >> sh,
+                           uz = (mz ^ ((L.sign & 4u) ? flip : 0u)) >> sh;
+            const uint4* row = c.top(L) + 2u * ((s.top - 1u) * kTopCells + (ux | (uy << 5) | (uz << 10)));
+            const uint4 a = __ldg(row), b = __ldg(row + 1);
+            uint32_t at = stack.below((uint32_t)L.h);
+            stack.store(at, a.x);
+            stack.store(at = stack.below(at), a.y);
+            stack.store(at = stack.below(at), a.z);
+            stack.store(at = stack.below(at), a.w);
+            stack.store(at = stack.below(at), b.x);
+            if (b.y != 0u) L.node = b.z;
+            l -= (int)b.y;
+            L.h = (int)stack.at(l + 1);
+        }
         for (;;) {
             const uint32_t m = 1u << l;
             slot = (((mx & m) + ((my & m) << 1) + ((mz & m) << 2)) >> l) ^ L.sign;

@@ -115,6 +115,10 @@ struct cbq_dag {
     uint32_t tagged_ref[8] = {};
     const uint32_t* walk_nodes() const { return d_tagged ? d_tagged : d_nodes; }
     uint32_t walk_root(int k) const { return d_tagged ? tagged_ref[k] : sd_ref[k]; }
+    // Tables of the upper cells of SubDAGs of height 6 or more, in the walk's references
+    // (dev::SubDag::top); null where there are none.
+    uint32_t* d_top = nullptr;
+    uint32_t top_index[8] = {};
     // The batch kernel takes tagged and compact stores; other DAGs are launched on their own.
     bool batch_ok() const { return flat_ok && (d_tagged || layout == CBQ_DAG_LAYOUT_COMPACT); }
     uint64_t node_count = 0;

@@ -29,11 +29,20 @@ struct SubDag {
     int32_t lx, ly, lz;   // lower bound (signed voxel coordinates)
     int32_t height;
     uint32_t node;
-    uint32_t pad[3];
+    uint32_t top;         // ordered walk: 1 + its table of upper cells (kTopLevels), 0 without one
+    uint32_t pad[2];
 };
+
+// A SubDAG's table of upper cells: for each of its 32^3 cells (five levels
+// below the root; x + 32 y + 1024 z, by voxel coordinate), a row of eight words:
+// the references of the internal nodes on the way to the cell, how many there
+// are, and the last one.
+constexpr int kTopLevels = 5;
+constexpr uint32_t kTopCells = 1u << (3 * kTopLevels);
 
 struct DagParams {
     const uint32_t* __restrict__ nodes;
+    const uint4* __restrict__ top;  // tables of upper cells, kTopCells rows each
     uint32_t occupied;  // bit k: SubDAG k is not empty
     SubDag sd[8];
 };

@@ -212,3 +212,38 @@ def test_store_beyond_the_tagged_range(orc):
                 g = res[k] if isinstance(res[k], np.ndarray) else res[k].cpu().numpy()
                 assert oracle.same_bits_nan_equal(g.astype(want[k].dtype) if k == "material" else g, want[k]), (k, mf)
         server.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("log2", [1, 4, 5, 6, 7])
+def test_origins_inside_around_the_table_s_height(log2, orc):
+    """Rays from inside volumes whose SubDAG has no table of upper cells (height 5 and below),
+    ends right below it (6) and goes on (7), in one octant and in three, both layouts."""
+    torch = pytest.importorskip("torch")
+    torch.cuda.set_device(0)
+    rng = np.random.default_rng(70 + log2)
+    edge = 1 << log2
+    for places in (((0, 0, 0),), ((-edge, 0, 0), (0, -edge, -edge), (0, 0, 0)), ((-(1 << 21),) * 3,)):
+        nodes, root = _join([build_dag(random_voxels(rng, edge) if log2 > 1 else
+                                       rng.integers(0, 2, (2, 2, 2)).astype(np.uint8) * 7, p) for p in places])
+        sd = orc.find_subdags(nodes, root)
+        n = 4000
+        at = np.array(places, np.float64)[rng.integers(0, len(places), n)]
+        o = np.zeros((n, 4), np.float32)
+        d = rng.normal(size=(n, 4)).astype(np.float32)
+        o[:, :3] = at + rng.uniform(-0.5, edge - 0.5, (n, 3))
+        snap = rng.random(n) < 0.3
+        o[snap, :3] = np.round(o[snap, :3] * 2.0) / 2.0
+        o[:, 3] = np.inf
+        to, td = torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda()
+        for mf in (-1.0, 0.0035, 0.4, 3.0):
+            want = orc.intersect(nodes, sd, o, d, True, mf)
+            for layout in (cbq.LAYOUT_REFERENCE, cbq.LAYOUT_COMPACT):
+                dag = cbq.Dag(nodes, root, layout)
+                for stack in (cbq.STACK_SHARED, cbq.STACK_LOCAL):
+                    dag.set_launch_config(stack=stack)
+                    got = cbq.intersect_volume(dag, to, td, True, mf)
+                    for k in FIELDS:
+                        g = got[k].cpu().numpy()
+                        assert oracle.same_bits_nan_equal(g.astype(want[k].dtype) if k == "material" else g,
+                                                          want[k]), (k, mf, layout, stack, places)
