@@ -253,7 +253,7 @@ __device__ __forceinline__ float4 lane_begin(Lane& L, const Src& c, uint64_t i, 
     }
     L.fetches = 0u;
     L.loads = 0u;
-    L.mode = kLaneEnter;
+    L.mode = ((c.occupied(L) >> ((L.oct ^ L.sign) & 7u)) & 1u) ? kLaneEnter : kLaneNext;
     return d;
 }
 
@@ -326,9 +326,33 @@ template <typename Src>
 __device__ __forceinline__ void lane_next(Lane& L, const Src& c)
 {
     const uint32_t occupied = c.occupied(L);
-    if (!Src::kIntPos && L.fast && (occupied & octants_ahead(L.oct, L.sign)) == 0u) {
-        L.mode = kLaneMiss;
-        return;
+    if (!Src::kIntPos && L.fast) {
+        const uint32_t ahead = occupied & octants_ahead(L.oct, L.sign);
+        if (ahead == 0u) {
+            L.mode = kLaneMiss;
+            return;
+        }
+        if ((ahead & (ahead - 1u)) == 0u) {
+            // One octant with a SubDAG ahead.  The walk comes to it exactly when it crosses all
+            // the planes between (`need`) before any other (`rest`).  Products with 1/|dir| are
+            // within 2^-22 of the quotients that decide; only closer calls take the walk itself,
+            // with its three divisions (camera rays 345 -> 334 us, spheres-256 72 -> 69.5).
+            const uint32_t k = (31u - __clz(ahead)) ^ L.sign, need = k & ~L.oct, rest = ~k;
+            const float tx = -L.rox * L.ix, ty = -L.roy * L.iy, tz = -L.roz * L.iz;
+            const float last = fmaxf(fmaxf((need & 1u) ? tx : 0.0f, (need & 2u) ? ty : 0.0f), (need & 4u) ? tz : 0.0f);
+            const float first = fminf(fminf((rest & 1u) ? tx : FLT_MAX, (rest & 2u) ? ty : FLT_MAX),
+                                      (rest & 4u) ? tz : FLT_MAX);
+            const float slack = first * 9.5367431640625e-07f;  // 2^-20
+            if (last < first - slack) {
+                L.oct = k;
+                L.mode = kLaneEnter;
+                return;
+            }
+            if (last > first + slack) {
+                L.mode = kLaneMiss;
+                return;
+            }
+        }
     }
     OctantWalk w;
     w.begin(L, c.ray_direction(L, L.ray));

@@ -247,3 +247,34 @@ def test_origins_inside_around_the_table_s_height(log2, orc):
                         g = got[k].cpu().numpy()
                         assert oracle.same_bits_nan_equal(g.astype(want[k].dtype) if k == "material" else g,
                                                           want[k]), (k, mf, layout, stack, places)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("places", [((0, 0, 0),), ((-32, 0, -32),), ((0, 0, 0), (-32, -32, 0)),
+                                    ((0, 0, 0), (0, -32, 0), (-32, -32, -32), (-32, 0, 0))])
+def test_rays_from_other_octants(places, orc):
+    """Volumes in one, two and four octants met from all the others, with crossings of the
+    planes between that tie exactly or differ by a few units in the last place."""
+    torch = pytest.importorskip("torch")
+    torch.cuda.set_device(0)
+    rng = np.random.default_rng(len(places))
+    nodes, root = _join([build_dag(random_voxels(rng, 32), p) for p in places])
+    sd = orc.find_subdags(nodes, root)
+    n = 60000
+    o = np.zeros((n, 4), np.float32)
+    d = np.zeros((n, 4), np.float32)
+    o[:, :3] = rng.integers(-128, 129, (n, 3)) * 0.5 - 0.5
+    d[:, :3] = rng.choice(np.array([-2.0, -1.0, -0.5, -0.75, 0.25, 0.75, 1.0, 3.0], np.float32), (n, 3))
+    toward = rng.random(n) < 0.5  # through a point near the origin's planes: close calls of their order
+    d[toward, :3] = -(o[toward, :3] + np.float32(0.5)) + rng.integers(-1, 2, (int(toward.sum()), 3)) * np.float32(1e-5)
+    for a in range(3):
+        bump = rng.random(n) < 0.3
+        d[bump, a] = np.nextafter(d[bump, a], rng.choice(np.array([-9.0, 9.0], np.float32), int(bump.sum())))
+    o[:, 3] = np.inf
+    dag = cbq.Dag(nodes, root)
+    got = cbq.intersect_volume(dag, torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda())
+    want = orc.intersect(nodes, sd, o, d)
+    assert 0 < int(want["hit"].sum()) < n
+    for k in FIELDS:
+        g = got[k].cpu().numpy()
+        assert oracle.same_bits_nan_equal(g.astype(want[k].dtype) if k == "material" else g, want[k]), k
