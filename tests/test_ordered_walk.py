@@ -278,3 +278,48 @@ def test_rays_from_other_octants(places, orc):
     for k in FIELDS:
         g = got[k].cpu().numpy()
         assert oracle.same_bits_nan_equal(g.astype(want[k].dtype) if k == "material" else g, want[k]), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("places", [((1 << 23, 0, 0),), ((1 << 23, 0, 1 << 22), (-32, -32, 0), (-32, 0, -32)),
+                                    ((0, 0, 0), (-(1 << 22), 0, 0), (-(1 << 31), -32, -32))])
+def test_rays_between_octants_of_far_volumes(places, orc):
+    """Integer positions: volumes beyond +-2^21 and around the origin met from all octants, from
+    origins up to 2^31, directions on both sides of the octant rules' range, and close calls."""
+    torch = pytest.importorskip("torch")
+    torch.cuda.set_device(0)
+    rng = np.random.default_rng(len(places))
+    nodes, root = _join([build_dag(random_voxels(rng, 32), p) for p in places])
+    sd = orc.find_subdags(nodes, root)
+    n = 60000
+    o = np.zeros((n, 4), np.float32)
+    d = np.zeros((n, 4), np.float32)
+    target = np.array(places, np.float64)[rng.integers(0, len(places), n)] + rng.uniform(0.0, 32.0, (n, 3))
+    away = np.exp2(rng.uniform(3.0, 31.0, n))[:, None]
+    way = rng.normal(size=(n, 3))
+    way /= np.linalg.norm(way, axis=1, keepdims=True)
+    o[:, :3] = np.clip(target - way * away, -(2.0 ** 31), 2.0 ** 31)
+    d[:, :3] = way
+    near = rng.random(n) < 0.4
+    o[near, :3] = rng.integers(-128, 129, (int(near.sum()), 3)) * 0.5 - 0.5
+    toward = rng.random(n) < 0.3  # through a point near the origin's planes: close calls of their order
+    d[toward, :3] = -(o[toward, :3] + np.float32(0.5)) + rng.integers(-1, 2, (int(toward.sum()), 3)) * np.float32(1e-5)
+    odd = np.nonzero(rng.random(n) < 0.1)[0]
+    vals = np.array([DIR_MIN, np.nextafter(DIR_MIN, np.float32(0)), DIR_MAX,
+                     np.nextafter(DIR_MAX, np.float32(np.inf)), 0.0, 1e-38, 1e-30, 1e30], np.float32)
+    d[odd, rng.integers(0, 3, odd.size)] = rng.choice(vals, odd.size) * rng.choice((-1.0, 1.0), odd.size)
+    beyond = np.nonzero(rng.random(n) < 0.02)[0]
+    o[beyond, rng.integers(0, 3, beyond.size)] = rng.choice(
+        np.array([2.0 ** 32, -(2.0 ** 32), 4.3e9, -1e12, 1e30], np.float32), beyond.size)
+    o[:, 3] = np.inf
+    to, td = torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda()
+    dag = cbq.Dag(nodes, root)
+    for mf in (-1.0, 0.02):
+        want = orc.intersect(nodes, sd, o, d, True, mf)
+        assert 0 < int(want["hit"].sum()) < n
+        for stack, form in ((cbq.STACK_SHARED, cbq.FORM_PERSISTENT), (cbq.STACK_LOCAL, cbq.FORM_PLAIN)):
+            dag.set_launch_config(stack=stack, form=form)
+            got = cbq.intersect_volume(dag, to, td, True, mf)
+            for k in FIELDS:
+                g = got[k].cpu().numpy()
+                assert oracle.same_bits_nan_equal(g.astype(want[k].dtype) if k == "material" else g, want[k]), (k, mf)
