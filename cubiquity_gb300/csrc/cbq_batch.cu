@@ -18,10 +18,13 @@
 namespace cbq {
 namespace dev {
 
-template <Store STORE>
+// LOD: some job's query may stop at a footprint (each job has its own query).
+// Without any, the walk leaves out the test, nine instructions of each
+// iteration (12 volumes, 2.2 M rays: 227 -> 208 us).
+template <Store STORE, bool LOD>
 struct BatchSrc {
     static constexpr Store kStore = STORE;
-    static constexpr bool kLod = true;      // each job has its own query
+    static constexpr bool kLod = LOD;
     static constexpr bool kOrdered = true;
     static constexpr bool kIntPos = false;  // such jobs run on their own (cbq_dag::batch_ok)
     const JobDesc* __restrict__ jobs;
@@ -59,7 +62,7 @@ __device__ __forceinline__ uint32_t job_of(const uint64_t* prefix, uint32_t njob
 // instead of a per-thread local array.  SORTED: global ray g of the launch is
 // ray perm[g], a ray of the same job (launch_batch_octant_sort).  Every job of
 // one launch has the node store layout COMPACT.
-template <bool COMPACT, bool SHARED, bool SORTED>
+template <bool COMPACT, bool SHARED, bool SORTED, bool LOD>
 __device__ __forceinline__ void batch_body(const JobDesc* __restrict__ jobs, uint32_t njobs, uint64_t total,
                                            unsigned long long* __restrict__ counter, uint32_t refill_min,
                                            uint32_t steps, const uint32_t* __restrict__ perm, uint32_t warp_rays)
@@ -71,7 +74,7 @@ __device__ __forceinline__ void batch_body(const JobDesc* __restrict__ jobs, uin
     SharedStack sstack;
     sstack.init((uint32_t*)(prefix + njobs + 1) + threadIdx.x, blockDim.x);
 
-    BatchSrc<COMPACT ? Store::kCompact : Store::kTagged> c;
+    BatchSrc<COMPACT ? Store::kCompact : Store::kTagged, LOD> c;
     c.jobs = jobs;
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t below = (1u << lane) - 1u;
@@ -125,13 +128,13 @@ __device__ __forceinline__ void batch_body(const JobDesc* __restrict__ jobs, uin
     }
 }
 
-template <bool COMPACT, bool SHARED, bool SORTED>
+template <bool COMPACT, bool SHARED, bool SORTED, bool LOD>
 __global__ void __launch_bounds__(256, 4) cbq_k_flat_batch(const JobDesc* __restrict__ jobs, uint32_t njobs,
                                                         uint64_t total, unsigned long long* __restrict__ counter,
                                                         uint32_t refill_min, uint32_t steps,
                                                         const uint32_t* __restrict__ perm, uint32_t warp_rays)
 {
-    batch_body<COMPACT, SHARED, SORTED>(jobs, njobs, total, counter, refill_min, steps, perm, warp_rays);
+    batch_body<COMPACT, SHARED, SORTED, LOD>(jobs, njobs, total, counter, refill_min, steps, perm, warp_rays);
 }
 
 // Octant of a ray: its direction sign bits (raytracing.cpp:416-417).
@@ -214,11 +217,11 @@ void fill_job_volume(dev::JobDesc& d, const cbq_dag* dag)
 
 namespace {
 
-template <bool COMPACT, bool SHARED, bool SORTED>
+template <bool COMPACT, bool SHARED, bool SORTED, bool LOD>
 cbq_status launch_batch_variant(const dev::JobDesc* d_jobs, uint32_t njobs, uint64_t total, uint64_t* counter,
                                 int device, cudaStream_t s, const BatchLaunch& bl)
 {
-    auto kernel = dev::cbq_k_flat_batch<COMPACT, SHARED, SORTED>;
+    auto kernel = dev::cbq_k_flat_batch<COMPACT, SHARED, SORTED, LOD>;
     const uint32_t warp_rays = bl.spread ? spread_warp_rays(total, device) : 0u;
     if (!warp_rays && !bl.counter_zeroed && cudaMemsetAsync(counter, 0, sizeof(uint64_t), s) != cudaSuccess)
         return CBQ_ERR_CUDA;
@@ -243,16 +246,16 @@ cbq_status launch_batch_variant(const dev::JobDesc* d_jobs, uint32_t njobs, uint
     return cudaGetLastError() == cudaSuccess ? CBQ_OK : CBQ_ERR_CUDA;
 }
 
-template <bool COMPACT>
+template <bool COMPACT, bool LOD>
 cbq_status launch_batch_layout(const dev::JobDesc* d_jobs, uint32_t njobs, uint64_t total, uint64_t* counter,
                                int device, cudaStream_t s, const BatchLaunch& bl)
 {
     const bool sorted = bl.perm != nullptr;
     if (bl.shared_stack)
-        return sorted ? launch_batch_variant<COMPACT, true, true>(d_jobs, njobs, total, counter, device, s, bl)
-                      : launch_batch_variant<COMPACT, true, false>(d_jobs, njobs, total, counter, device, s, bl);
-    return sorted ? launch_batch_variant<COMPACT, false, true>(d_jobs, njobs, total, counter, device, s, bl)
-                  : launch_batch_variant<COMPACT, false, false>(d_jobs, njobs, total, counter, device, s, bl);
+        return sorted ? launch_batch_variant<COMPACT, true, true, LOD>(d_jobs, njobs, total, counter, device, s, bl)
+                      : launch_batch_variant<COMPACT, true, false, LOD>(d_jobs, njobs, total, counter, device, s, bl);
+    return sorted ? launch_batch_variant<COMPACT, false, true, LOD>(d_jobs, njobs, total, counter, device, s, bl)
+                  : launch_batch_variant<COMPACT, false, false, LOD>(d_jobs, njobs, total, counter, device, s, bl);
 }
 
 }  // namespace
@@ -261,8 +264,11 @@ cbq_status launch_batch_kernel(const dev::JobDesc* d_jobs, uint32_t njobs, uint6
                                bool compact, int device, cudaStream_t s, const BatchLaunch& bl)
 {
     if (total == 0 || njobs == 0) return CBQ_OK;
-    return compact ? launch_batch_layout<true>(d_jobs, njobs, total, counter, device, s, bl)
-                   : launch_batch_layout<false>(d_jobs, njobs, total, counter, device, s, bl);
+    if (bl.lod)
+        return compact ? launch_batch_layout<true, true>(d_jobs, njobs, total, counter, device, s, bl)
+                       : launch_batch_layout<false, true>(d_jobs, njobs, total, counter, device, s, bl);
+    return compact ? launch_batch_layout<true, false>(d_jobs, njobs, total, counter, device, s, bl)
+                   : launch_batch_layout<false, false>(d_jobs, njobs, total, counter, device, s, bl);
 }
 
 cbq_status launch_batch_octant_sort(const dev::JobDesc* d_jobs, uint32_t njobs, uint64_t total, uint32_t* scratch,
@@ -328,6 +334,7 @@ BatchLaunch batch_launch(const cbq_batch* b, const uint32_t* perm)
     bl.shared_stack = b->cfg.stack == CBQ_STACK_SHARED;
     bl.stack_rows = b->stack_rows;
     bl.spread = !b->own_shape;
+    bl.lod = !(b->query.max_footprint < 0.0f);
     bl.perm = perm;
     return bl;
 }

@@ -38,6 +38,7 @@ struct BatchLaunch {
     bool shared_stack = true;        // descent stack in shared memory (stack_rows rows) instead of local
     int stack_rows = 0;              // max SubDAG height over the jobs
     const uint32_t* perm = nullptr;  // octant order (launch_batch_octant_sort), or null
+    bool lod = true;                 // some job's query may stop at a footprint (max_footprint >= 0)
     bool spread = false;             // a small launch may be spread over the chip (spread_warp_rays)
     bool counter_zeroed = false;     // the work counter is already zero, in stream order
 };

@@ -287,6 +287,7 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
     uint32_t njobs = 0, rows_in = 0, rows_out = 0;
     uint64_t total = 0, most_rays = 0, most_bytes = 0;
     int stack_rows = 1;
+    bool lod = false;
     // First pass: where every request's rays and hits are on the device, the job and
     // staging tables, and the copies in that the staging kernel does not make.
     for (Request* rq : group) {
@@ -343,6 +344,7 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
         s.h_table[njobs++] = jd;
         total += n;
         stack_rows = std::max(stack_rows, (int)rq->r.dag->max_height);
+        lod = lod || !(jd.q.max_footprint < 0.0f);
     }
     static_assert(sizeof(dev::JobDesc) % 8 == 0, "the job table is copied in 8-byte words");
     if (rows_in || njobs) {
@@ -367,6 +369,7 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
         bl.block = cfg.block;
         bl.refill = cfg.refill_min;
         bl.counter_zeroed = true;
+        bl.lod = lod;
         bl.stack_rows = stack_rows;
         bl.shared_stack = batch_stack_in_shared(njobs, stack_rows, cfg.block);
         cbq_status st = launch_batch_kernel(s.d_table, njobs, total, s.d_counter,

@@ -323,3 +323,25 @@ def test_rays_between_octants_of_far_volumes(places, orc):
             for k in FIELDS:
                 g = got[k].cpu().numpy()
                 assert oracle.same_bits_nan_equal(g.astype(want[k].dtype) if k == "material" else g, want[k]), (k, mf)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("footprints", [(-1.0,), (0.02,), (-1.0, 0.02, 0.0, -1.0, 1.0, float("inf"), float("nan"))])
+def test_requests_with_and_without_lod(footprints, orc):
+    """Server groups of requests with and without a footprint, in both layouts, against the oracle."""
+    torch = pytest.importorskip("torch")
+    torch.cuda.set_device(0)
+    nodes, root, centre, edge = _volume(3)
+    sd = orc.find_subdags(nodes, root)
+    o, d = _rays(3, centre, edge, 3000)
+    for layout in (cbq.LAYOUT_REFERENCE, cbq.LAYOUT_COMPACT):
+        dag = cbq.Dag(nodes, root, layout)
+        server = cbq.Server(device_memory_budget=64 << 20)
+        asked = [(mf, *server.submit(dag, o, d, cbq.Query(True, mf))) for mf in footprints * 12]
+        for mf, ticket, got in asked:
+            assert server.wait(ticket, 20_000_000) == 0
+            want = orc.intersect(nodes, sd, o, d, True, mf)
+            for k in FIELDS:
+                g = got[k].astype(want[k].dtype) if k == "material" else got[k]
+                assert oracle.same_bits_nan_equal(g, want[k]), (k, mf, layout)
+        server.close()
