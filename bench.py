@@ -452,8 +452,7 @@ def run_gpu(args, world, rank, local):
         c = tuned.get(label, cfg)
         per_batch[label] = {
             "rays": n, "launch_ms": ms, "fetches_per_ray": f, "bytes_per_ray": bpr,
-            "kernel": ("cbq_k_flat_r56" if c.get("registers") == 56 and c.get("form") != 0 and c.get("stack") == 1
-                       else kernel_name),
+            "kernel": kernel_name,
             "achieved_gbs": achieved, "frac_l2_stream": achieved / l2_stream,
             "sector_rate_gsps": sectors, "frac_l2_sector": sectors / l2_rand,
             "dram_bytes_per_launch": None if dram is None else dram * n,

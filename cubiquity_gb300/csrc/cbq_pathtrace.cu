@@ -35,7 +35,7 @@ struct PathState {
 };
 
 // Paths traced together in one pass: the samples of a pass share each wave's
-// launches (fewer, larger launches; one host round trip per depth and pass).
+// launches (fewer, larger launches).
 constexpr uint64_t kPtRaysPerPass = 1ull << 24;
 
 struct Frame {

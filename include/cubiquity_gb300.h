@@ -199,8 +199,8 @@ typedef struct cbq_launch_config {
     int32_t form;             /* CBQ_FORM_*, used by cbq_intersect_auto */
     int32_t steps;            /* flat kernel: walk iterations between a warp's checks for
                                  idle lanes (1..32), 0 = default (8, or from the rays) */
-    int32_t registers;        /* 0 (the default) or 56; every kernel of the walk takes
-                                 56 registers per thread now, so both are the same */
+    int32_t registers;        /* 0 (the default) or 56: the same, there is one kernel of
+                                 each form */
 } cbq_launch_config;
 
 cbq_status cbq_dag_set_launch_config(cbq_dag* dag, const cbq_launch_config* cfg);
