@@ -186,6 +186,20 @@ __device__ __forceinline__ bool ordered_axis(float rd, float ro)
     return rd >= kOrderedDirMin && rd <= kOrderedDirMax && fabsf(ro) <= (INT ? kIntOrigin : kOrderedOrigin);
 }
 
+// Rays parallel to one or two of the axes (a component of exactly 0) are
+// ordered too where the origin lies on no plane of those axes (not an integer):
+// there 1/|dir| is infinite, a plane behind the origin lies at -inf and one
+// ahead at +inf, never NaN.  Such an axis never bounds a cell's distances,
+// since the other axes' are finite, and of two halves the walk takes the one
+// that holds the origin, as the reference does.  1 Mi rays on terrain-1024: an
+// orthographic view along an axis 161 -> 92 us, bounce rays with one in sixteen
+// parallel to a plane 221 -> 136.
+constexpr uint32_t kParallelMoves = 16u;  // such a ray's mark in Lane::moves
+__device__ __forceinline__ bool parallel_axis(float rd, float ro)
+{
+    return rd == 0.0f && truncf(ro) != ro && fabsf(ro) <= kOrderedOrigin;
+}
+
 // The walk over the octants around the origin (raytracing.cpp:424-434,
 // :469-475).  A lane keeps only its octant and the transitions made: the
 // distances are computed again where a transition is due, which most rays
@@ -242,9 +256,15 @@ __device__ __forceinline__ float4 lane_begin(Lane& L, const Src& c, uint64_t i, 
     // the reference's std::min/std::max compositions.
     L.fast = (Src::kOrdered || Src::kIntPos) && ordered && ordered_axis<Src::kIntPos>(rdx, L.rox) &&
              ordered_axis<Src::kIntPos>(rdy, L.roy) && ordered_axis<Src::kIntPos>(rdz, L.roz);
+    L.moves = 0u;
+    if (Src::kOrdered && ordered && !L.fast) {
+        const bool px = parallel_axis(rdx, L.rox), py = parallel_axis(rdy, L.roy), pz = parallel_axis(rdz, L.roz);
+        L.fast = (px || ordered_axis(rdx, L.rox)) && (py || ordered_axis(rdy, L.roy)) &&
+                 (pz || ordered_axis(rdz, L.roz)) && !(px && py && pz);
+        L.moves = kParallelMoves;
+    }
     // The octant of the origin: distToOrigin = -o' / |dir| below 0
     // (raytracing.cpp:424-434), which is o' > 0 for a ray within the range.
-    L.moves = 0u;
     if (L.fast) {
         L.oct = (L.rox > 0.0f ? 1u : 0u) | (L.roy > 0.0f ? 2u : 0u) | (L.roz > 0.0f ? 4u : 0u);
     } else {
@@ -327,7 +347,9 @@ template <typename Src>
 __device__ __forceinline__ void lane_next(Lane& L, const Src& c)
 {
     const uint32_t occupied = c.occupied(L);
-    if (L.fast) {
+    // (A ray parallel to an axis takes the reference's own transitions: a distance of -inf
+    // plus FLT_MAX stays -inf, and is crossed again.)
+    if (L.fast && L.moves < kParallelMoves) {
         const uint32_t ahead = occupied & octants_ahead(L.oct, L.sign);
         if (ahead == 0u) {
             L.mode = kLaneMiss;
@@ -357,7 +379,7 @@ __device__ __forceinline__ void lane_next(Lane& L, const Src& c)
     }
     OctantWalk w;
     w.begin(L, c.ray_direction(L, L.ray));
-    for (uint32_t k = 0; k < L.moves; k++) w.next();
+    for (uint32_t k = 0; k < (L.moves & (kParallelMoves - 1u)); k++) w.next();
     do {
         if (!w.next()) {  // the reference would revisit this octant forever
             L.mode = kLaneStuck;

@@ -345,3 +345,75 @@ def test_requests_with_and_without_lod(footprints, orc):
                 g = got[k].astype(want[k].dtype) if k == "material" else got[k]
                 assert oracle.same_bits_nan_equal(g, want[k]), (k, mf, layout)
         server.close()
+
+
+def _parallel_rays(seed, centre, edge, n=6000):
+    """Rays with one, two or three components of exactly 0 (or -0), origins on voxel faces and off them."""
+    rng = np.random.default_rng(600 + seed)
+    o, d = _rays(seed, centre, edge, n)
+    for a in range(3):
+        zero = rng.random(n) < 0.45
+        d[zero, a] = rng.choice(np.array([0.0, -0.0], np.float32), int(zero.sum()))
+    aim = rng.random(n) < 0.6  # along the zero axes the origin lies within the volume
+    within = (centre + rng.uniform(-0.5, 0.5, (n, 3)) * edge).astype(np.float32)
+    o[:, :3] = np.where(aim[:, None] & (d[:, :3] == 0), within, o[:, :3])
+    snap = rng.random(n) < 0.3
+    o[snap, :3] = np.round(o[snap, :3] * 4.0) / 4.0
+    return o, d
+
+
+def _parallel(o, d):
+    """The rays that the ordered walk takes beside those of _ordered."""
+    sign = np.where(d[:, :3] < 0, np.float32(-1), np.float32(1))
+    ro = (o[:, :3] + np.float32(0.5)) * sign
+    rd = np.abs(d[:, :3])
+    zero = (rd == 0) & (np.trunc(ro) != ro)
+    ok = (np.abs(ro) <= ORIGIN_MAX) & (zero | ((rd >= DIR_MIN) & (rd <= DIR_MAX)))
+    return ok.all(axis=1) & ~zero.all(axis=1) & zero.any(axis=1)
+
+
+@pytest.mark.parametrize("seed", range(12))
+@pytest.mark.filterwarnings("ignore:divide by zero")
+def test_rules_of_parallel_rays(seed, orc, walk):
+    nodes, root, centre, edge = _volume(seed)
+    sd = orc.find_subdags(nodes, root)
+    o, d = _parallel_rays(seed, centre, edge)
+    keep = _parallel(o, d)
+    assert keep.sum() > 200
+    o, d = np.ascontiguousarray(o[keep]), np.ascontiguousarray(d[keep])
+    for mf in FOOTPRINTS:
+        want = orc.intersect(nodes, sd, o, d, False, mf)
+        fetches = orc.count_fetches(nodes, sd, o, d, False, mf)
+        got = walk(nodes, sd, o, d, mf)
+        assert not (got["status"] > 3).any()
+        own = got["status"] == 0
+        assert own.mean() > 0.5
+        for k in ("hit", "distance"):
+            assert np.array_equal(got[k][own].view(np.uint8), want[k][own].view(np.uint8)), (k, mf)
+        assert np.array_equal(got["fetches"][own], fetches[own]), mf
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("seed", range(8))
+def test_kernels_on_parallel_rays(seed, orc):
+    torch = pytest.importorskip("torch")
+    torch.cuda.set_device(0)
+    nodes, root, centre, edge = _volume(seed)
+    sd = orc.find_subdags(nodes, root)
+    o, d = _parallel_rays(seed, centre, edge)
+    to, td = torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda()
+    for mf in (-1.0, 0.0035, 0.3):
+        want = orc.intersect(nodes, sd, o, d, True, mf)
+        for layout in (cbq.LAYOUT_REFERENCE, cbq.LAYOUT_COMPACT):
+            dag = cbq.Dag(nodes, root, layout)
+            for stack, form in ((cbq.STACK_SHARED, cbq.FORM_PERSISTENT), (cbq.STACK_LOCAL, cbq.FORM_PLAIN)):
+                dag.set_launch_config(stack=stack, form=form)
+                got = cbq.intersect_volume(dag, to, td, True, mf)
+                batch = cbq.Batch([(dag, to, td)], True, mf)
+                batch.launch()
+                torch.cuda.synchronize()
+                for what, res in (("call", got), ("batch", batch.outputs[0])):
+                    for k in FIELDS:
+                        g = res[k].cpu().numpy()
+                        assert oracle.same_bits_nan_equal(g.astype(want[k].dtype) if k == "material" else g,
+                                                          want[k]), (what, k, mf, layout, stack)
