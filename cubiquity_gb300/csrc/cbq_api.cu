@@ -19,6 +19,15 @@ namespace {
 constexpr int kFlatBlockDefault = 128;  // GB300, terrain-4096: 64, 128 and 256 threads within 1-3%
 constexpr uint32_t kRefillDefault = 16;
 constexpr uint32_t kStepsDefault = 8;
+// One thread per ray: a warp walks until all its lanes have stopped, so a check for idle lanes
+// only costs (camera rays of spheres-256, 1 Mi: every 16 iterations 64.0 us, every 32 63.3).
+constexpr uint32_t kStepsPlain = 32;
+// An image of up to this many rays takes one thread per ray: its warps stay full to the end, so
+// refilling them gains less than the counter's zeroing and the refills cost (about 8 us a call).
+// Larger ones gain from refills.  us, one thread per ray / refilled: spheres 0.26 Mi 26 / 33, 1 Mi
+// 63 / 70, terrain 1 Mi 85 / 92, city with LOD 1 Mi 105 / 108, 2 Mi 152 / 149, terrain 2.25 Mi
+// 187 / 186, 4 Mi 345 / 329.
+constexpr uint64_t kPlainImageRays = 3ull << 19;
 
 bool use_flat(const cbq_dag* dag)
 {
@@ -38,15 +47,18 @@ FlatLaunch flat_launch(const cbq_dag* dag, bool persistent, uint64_t* counter, u
     fl.steps = (uint32_t)dag->cfg.steps;
     // Either alone takes the other's default; neither leaves both to the kernel (WarpRefill).
     if (fl.steps && !fl.refill_min) fl.refill_min = kRefillDefault;
-    if (!fl.steps) fl.steps = kStepsDefault;
+    if (!fl.steps) fl.steps = persistent ? kStepsDefault : kStepsPlain;
     return fl;
 }
 
-// Rays per warp where a launch without a shape of the caller's is spread (spread_warp_rays), else 0.
-uint32_t spread_rays(const cbq_dag* dag, uint64_t n)
+// Rays per warp where a launch without a shape of the caller's is spread (spread_warp_rays) or
+// takes one thread per ray (kPlainImageRays), else 0.
+uint32_t spread_rays(const cbq_dag* dag, uint64_t n, const cbq_query* query)
 {
     const bool own = dag->cfg.refill_min != 0 || dag->cfg.steps != 0 || dag->cfg.form != CBQ_FORM_PERSISTENT;
-    return own ? 0u : spread_warp_rays(n, dag->device);
+    if (own) return 0u;
+    const uint32_t spread = spread_warp_rays(n, dag->device);
+    return !spread && query && query->image_width && n <= kPlainImageRays ? 32u : spread;
 }
 
 constexpr uint64_t kTaggedMaxNodes = 1ull << 24;  // a tagged reference holds 24 bits of node index
@@ -524,7 +536,7 @@ cbq_status cbq_intersect(const cbq_dag* dag, const cbq_rays* rays, uint64_t n, c
     if (st != CBQ_OK) return st;
     if (use_flat(dag)) {
         // The DAG's form: persistent (the default, with this stream's work counter) or plain.
-        const uint32_t spread = spread_rays(dag, n);
+        const uint32_t spread = spread_rays(dag, n, query);
         uint64_t* counter =
             dag->cfg.form != CBQ_FORM_PLAIN && !spread ? stream_counter(dag, (cudaStream_t)stream) : nullptr;
         FlatLaunch fl = counter ? flat_launch(dag, true, counter, 0u) : flat_launch(dag, false, nullptr, 0u);
@@ -690,7 +702,7 @@ cbq_status cbq_intersect_persistent(const cbq_dag* dag, const cbq_rays* rays, ui
     cbq_status st = check_rays(rays);
     if (st != CBQ_OK) return st;
     if (use_flat(dag)) {
-        const uint32_t spread = chunk == 0 ? spread_rays(dag, n) : 0u;
+        const uint32_t spread = chunk == 0 ? spread_rays(dag, n, query) : 0u;
         FlatLaunch fl = flat_launch(dag, !spread, spread ? nullptr : work_counter, std::min<uint32_t>(chunk, 32u));
         if (spread) fl.warp_rays = spread;
         return launch_flat(dag, make_dag_params(dag), make_query(query), make_hits(hits),

@@ -883,8 +883,10 @@ __device__ __forceinline__ void warp_walk_steps(Lane& L, const Src& c, Stack& st
 // loses more to idle lanes than a refill costs.  So without a shape from the
 // caller (refill_min 0) each refill looks at its rays' directions: within a
 // quarter of their size of the first one's, the warp waits for 24 idle lanes
-// and checks every 16 iterations, else for 16 and every 8.  Both ways, us:
-// terrain-4096 camera rays 343 / 365, bounce rays 569 / 545.  The batch and
+// and checks every 32 iterations, else for 16 and every 8.  Both ways, us:
+// terrain-4096 camera rays 331 / 365, bounce rays 569 / 545 (camera rays checked
+// every 16 iterations 333).  Equal directions (sun rays from scattered surfaces)
+// tell less: every 16 (1.5 M shadow rays 123, every 32 125).  The batch and
 // server launches keep 16 and 8: their small volumes' camera rays gain nothing
 // from waiting (12 volumes: 240 us, chosen by the rays 245).
 struct WarpRefill {
@@ -905,8 +907,9 @@ struct WarpRefill {
         const float near = 0.25f * fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z));
         const float off = fmaxf(fmaxf(fabsf(d.x - x), fabsf(d.y - y)), fabsf(d.z - z));
         const bool coherent = __all_sync(0xffffffffu, !fresh || off <= near);
+        const bool beam = !__any_sync(0xffffffffu, fresh && off > 0.0f);
         idle_min = coherent ? 24u : 16u;
-        steps = coherent ? 16u : 8u;
+        steps = !coherent ? 8u : beam ? 16u : 32u;
     }
 };
 

@@ -67,3 +67,19 @@ def test_spread_launch_in_a_capture(scene):
     graph.replay()
     torch.cuda.synchronize()
     _same(out, cbq.intersect_volume(shaped, o, d), "capture")
+
+
+@pytest.mark.parametrize("n", [(3 << 19) - 4096, 3 << 19, (3 << 19) + 1, (3 << 19) + 4096])
+def test_image_sizes(scene, n):
+    """Around the size up to which an image takes one thread per ray: whole bands, ragged ends, host calls."""
+    dag, shaped, _, _ = scene
+    o, d = W.camera_scaled(8, 512, -(-n // 512)).rays()
+    to, td = torch.from_numpy(o[:n]).cuda(), torch.from_numpy(d[:n]).cuda()
+    for kw in ({}, {"max_footprint": 0.01}):
+        want = cbq.intersect_volume(shaped, to, td, **kw)
+        for width in (512, 513):
+            _same(cbq.intersect_volume(dag, to, td, image_width=width, **kw), want, f"{n} {kw} width {width}")
+    host = cbq.intersect_volume_host(dag, o[:n], d[:n], image_width=512)
+    want = cbq.intersect_volume(shaped, to, td)
+    for k in want:
+        assert want[k].cpu().numpy().tobytes() == host[k].tobytes(), k
