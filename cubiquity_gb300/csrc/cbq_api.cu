@@ -327,9 +327,8 @@ __global__ void __launch_bounds__(256) cbq_k_top_table(const uint32_t* __restric
 
 namespace {
 
-// Builds the tables of a DAG whose walk store carries masks; without memory for them there
-// are none, and rays descend level by level.
-cbq_status build_top_tables(cbq_dag* dag)
+// Numbers the tables of a DAG whose walk store carries masks; returns how many there are.
+uint32_t number_top_tables(cbq_dag* dag)
 {
     uint32_t tables = 0;
     for (int k = 0; k < 8; k++) {
@@ -337,13 +336,12 @@ cbq_status build_top_tables(cbq_dag* dag)
         const bool has = s.node_index >= dev::kMaterialCount && s.node_height > dev::kTopLevels;
         dag->top_index[k] = has ? ++tables : 0u;
     }
-    if (tables == 0) return CBQ_OK;
-    if (cudaMalloc((void**)&dag->d_top, (size_t)tables * dev::kTopCells * 32u) != cudaSuccess) {
-        cudaGetLastError();
-        dag->d_top = nullptr;
-        for (uint32_t& t : dag->top_index) t = 0u;
-        return CBQ_OK;
-    }
+    return tables;
+}
+
+// Queues the kernels that fill them.
+cbq_status build_top_tables(const cbq_dag* dag)
+{
     for (int k = 0; k < 8; k++) {
         if (!dag->top_index[k]) continue;
         uint4* table = (uint4*)dag->d_top + 2ull * (dag->top_index[k] - 1u) * dev::kTopCells;
@@ -354,8 +352,7 @@ cbq_status build_top_tables(cbq_dag* dag)
             cbq_k_top_table<dev::Store::kTagged><<<dev::kTopCells / 256u, 256, 0, cudaStreamLegacy>>>(
                 dag->walk_nodes(), dag->walk_root(k), table);
     }
-    return cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess ? CBQ_OK
-                                                                                                    : CBQ_ERR_CUDA;
+    return cudaGetLastError() == cudaSuccess ? CBQ_OK : CBQ_ERR_CUDA;
 }
 
 cbq_status preload_nested_persistent()
@@ -424,24 +421,30 @@ cbq_status cbq_dag_create_ex(const uint32_t* host_nodes, uint64_t node_count, ui
     }
     dag->device_bytes = bytes;
     const bool tag = dag->flat_ok && dag->layout == CBQ_DAG_LAYOUT_REFERENCE && node_count <= kTaggedMaxNodes;
-    cudaError_t e = cudaMalloc((void**)&dag->d_nodes, bytes);
-    if (e != cudaSuccess) { cudaGetLastError(); delete dag; return CBQ_ERR_OUT_OF_MEMORY; }
-    e = cudaMemcpy(dag->d_nodes, src, bytes, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) { cudaFree(dag->d_nodes); delete dag; return CBQ_ERR_CUDA; }
-    if (tag && cudaMalloc((void**)&dag->d_tagged, bytes) != cudaSuccess) {
-        cudaGetLastError();  // without it the walk takes the reference layout
-        dag->d_tagged = nullptr;
+    // One allocation: the node array, its tagged copy and the tables of upper cells (a cudaMalloc
+    // takes 70 us).  Without memory for all of it there is the node array alone, and the walk
+    // takes that.
+    const bool masks = tag || dag->layout == CBQ_DAG_LAYOUT_COMPACT;
+    const size_t part = (bytes + 255u) & ~(size_t)255u;
+    const size_t top_bytes = masks ? (size_t)number_top_tables(dag) * dev::kTopCells * 32u : 0u;
+    const size_t total = part + (tag ? part : 0u) + top_bytes;
+    const bool whole = cudaMalloc((void**)&dag->d_nodes, total) == cudaSuccess;
+    if (!whole) {
+        cudaGetLastError();
+        for (uint32_t& t : dag->top_index) t = 0u;
+        if (cudaMalloc((void**)&dag->d_nodes, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            delete dag;
+            return CBQ_ERR_OUT_OF_MEMORY;
+        }
     }
-    if (dag->d_tagged) {
+    cudaError_t e = cudaMemcpy(dag->d_nodes, src, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && whole && tag) {
+        dag->d_tagged = dag->d_nodes + part / 4u;
         const uint64_t words = node_count * 8u;
         cbq_k_tag_nodes<<<(unsigned)std::min<uint64_t>((words + 255) / 256, 1u << 20), 256, 0, cudaStreamLegacy>>>(
             (const uint4*)dag->d_nodes, words, dag->d_tagged);
-        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
-            cudaFree(dag->d_nodes);
-            cudaFree(dag->d_tagged);
-            delete dag;
-            return CBQ_ERR_CUDA;
-        }
+        e = cudaGetLastError();
         for (int i = 0; i < 8; i++) {
             const uint32_t r = dag->subdags[i].node_index;
             uint32_t mask = 0;
@@ -449,8 +452,13 @@ cbq_status cbq_dag_create_ex(const uint32_t* host_nodes, uint64_t node_count, ui
             dag->tagged_ref[i] = r == 0u ? 0u : (r << 8) | mask;
         }
     }
-    if (dag->batch_ok() && build_top_tables(dag) != CBQ_OK) {
-        cbq_dag_destroy(dag);
+    if (e == cudaSuccess && whole && top_bytes != 0u) {
+        dag->d_top = dag->d_nodes + (total - top_bytes) / 4u;
+        if (build_top_tables(dag) != CBQ_OK) e = cudaErrorUnknown;
+    }
+    if (e != cudaSuccess || cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
+        cudaFree(dag->d_nodes);
+        delete dag;
         return CBQ_ERR_CUDA;
     }
     cbq::log(CBQ_LOG_INFO,
@@ -466,8 +474,6 @@ cbq_status cbq_dag_destroy(cbq_dag* dag)
 {
     if (!dag) return CBQ_ERR_INVALID_ARGUMENT;
     cudaFree(dag->d_nodes);
-    if (dag->d_tagged) cudaFree(dag->d_tagged);
-    if (dag->d_top) cudaFree(dag->d_top);
     for (auto& kv : dag->stream_counters) cudaFree(kv.second);
     pt_workspace_release(dag->pt);
     for (auto& hs : dag->stages) {

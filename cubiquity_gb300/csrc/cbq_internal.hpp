@@ -104,7 +104,8 @@ cbq_status intersect_device_count(const cbq_dag* dag, const cbq_rays* rays, uint
 
 // The opaque DAG handle.
 struct cbq_dag {
-    uint32_t* d_nodes = nullptr;   // device: node_count * 8 words, or the compact store
+    uint32_t* d_nodes = nullptr;   // device: node_count * 8 words, or the compact store; in the same
+                                   // allocation d_tagged and d_top
     uint32_t layout = CBQ_DAG_LAYOUT_REFERENCE;
     uint64_t device_bytes = 0;     // size of the device node store
     uint32_t sd_ref[8] = {};       // SubDAG roots as the device store refers to them
