@@ -198,7 +198,8 @@ typedef struct cbq_launch_config {
     int32_t stack;            /* CBQ_STACK_* (flat kernel; shared by default) */
     int32_t form;             /* CBQ_FORM_*, used by cbq_intersect_auto */
     int32_t steps;            /* flat kernel: walk iterations between a warp's checks for
-                                 idle lanes (1..32), 0 = default (8, or from the rays) */
+                                 idle lanes (1..32), 0 = default (8, plain 32, or from
+                                 the rays) */
     int32_t registers;        /* 0 (the default) or 56: the same, there is one kernel of
                                  each form */
 } cbq_launch_config;
