@@ -201,10 +201,13 @@ bool host_staging(const float* o, const float* d, uint64_t n, const cbq_hits& h,
     return true;
 }
 
-// The persistent form's work counter for launches on `stream` (one per stream,
-// allocated on first use), or nullptr where none can be had: the id query
-// fails, or the stream is being captured (no allocation inside a capture).
-uint64_t* stream_counter(const cbq_dag* cdag, cudaStream_t stream)
+// A zeroed work counter of the persistent form for the next launch on `stream`
+// (from the stream's ring, allocated on first use), or nullptr where none can be
+// had: the id query fails, or the stream is being captured (no allocation inside
+// a capture).  The launch is queued while `lk` holds counter_lock.  A memset
+// before every launch took 2 us of the stream (1.5 M shadow rays 123.4 us,
+// without 121.4; city camera with LOD 150.5, 148.7).
+uint64_t* stream_counter(const cbq_dag* cdag, cudaStream_t stream, std::unique_lock<std::mutex>& lk)
 {
     cbq_dag* dag = const_cast<cbq_dag*>(cdag);
     // Only the capture query is legal while a capture is under way: ask it first.
@@ -219,16 +222,24 @@ uint64_t* stream_counter(const cbq_dag* cdag, cudaStream_t stream)
         cudaGetLastError();
         return nullptr;
     }
-    std::lock_guard<std::mutex> lk(dag->counter_lock);
-    auto it = dag->stream_counters.find(id);
-    if (it != dag->stream_counters.end()) return it->second;
-    uint64_t* p = nullptr;
-    if (cudaMalloc((void**)&p, 256) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
+    lk = std::unique_lock<std::mutex>(dag->counter_lock);
+    cbq_dag::CounterRing& ring = dag->stream_counters[id];
+    if (!ring.at) {
+        if (cudaMalloc((void**)&ring.at, cbq_dag::kCounterRing * sizeof(uint64_t)) != cudaSuccess) {
+            cudaGetLastError();
+            ring.at = nullptr;
+            return nullptr;
+        }
+        ring.used = cbq_dag::kCounterRing;
     }
-    dag->stream_counters[id] = p;
-    return p;
+    if (ring.used == cbq_dag::kCounterRing) {
+        if (cudaMemsetAsync(ring.at, 0, cbq_dag::kCounterRing * sizeof(uint64_t), stream) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        ring.used = 0;
+    }
+    return ring.at + ring.used++;
 }
 
 cbq_status check_rays(const cbq_rays* rays)
@@ -474,7 +485,8 @@ cbq_status cbq_dag_destroy(cbq_dag* dag)
 {
     if (!dag) return CBQ_ERR_INVALID_ARGUMENT;
     cudaFree(dag->d_nodes);
-    for (auto& kv : dag->stream_counters) cudaFree(kv.second);
+    for (auto& kv : dag->stream_counters)
+        if (kv.second.at) cudaFree(kv.second.at);
     pt_workspace_release(dag->pt);
     for (auto& hs : dag->stages) {
         if (hs->d_stage) cudaFree(hs->d_stage);
@@ -543,9 +555,11 @@ cbq_status cbq_intersect(const cbq_dag* dag, const cbq_rays* rays, uint64_t n, c
     if (use_flat(dag)) {
         // The DAG's form: persistent (the default, with this stream's work counter) or plain.
         const uint32_t spread = spread_rays(dag, n, query);
-        uint64_t* counter =
-            dag->cfg.form != CBQ_FORM_PLAIN && !spread ? stream_counter(dag, (cudaStream_t)stream) : nullptr;
+        std::unique_lock<std::mutex> queueing;
+        uint64_t* counter = dag->cfg.form != CBQ_FORM_PLAIN && !spread
+                                ? stream_counter(dag, (cudaStream_t)stream, queueing) : nullptr;
         FlatLaunch fl = counter ? flat_launch(dag, true, counter, 0u) : flat_launch(dag, false, nullptr, 0u);
+        fl.counter_zeroed = counter != nullptr;
         if (spread) fl.warp_rays = spread;
         return launch_flat(dag, make_dag_params(dag), make_query(query), make_hits(hits),
                            (const float4*)rays->origin_tmax, (const float4*)rays->direction, n, nullptr, fl,

@@ -237,7 +237,8 @@ cbq_status launch_variant(const Ctx& c, uint64_t n, const FlatLaunch& fl, int ro
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, fl.block, smem) != cudaSuccess)
             return CBQ_ERR_CUDA;
         per_sm = std::max(per_sm, 1);
-        if (cudaMemsetAsync(fl.counter, 0, sizeof(uint64_t), stream) != cudaSuccess) return CBQ_ERR_CUDA;
+        if (!fl.counter_zeroed && cudaMemsetAsync(fl.counter, 0, sizeof(uint64_t), stream) != cudaSuccess)
+            return CBQ_ERR_CUDA;
         // No more blocks than the rays fill.
         const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sms * per_sm, (n + fl.block - 1) / fl.block);
         kernel<<<grid, fl.block, smem, stream>>>(c, n, (unsigned long long*)fl.counter, fl.refill_min,

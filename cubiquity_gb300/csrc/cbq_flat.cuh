@@ -931,6 +931,7 @@ __device__ __forceinline__ void lane_settle(Lane& L, const Src& c, Stack& stack)
 struct FlatLaunch {
     bool persistent = false;
     uint64_t* counter = nullptr;     // persistent: work counter (zeroed by the launch)
+    bool counter_zeroed = false;     // ... unless it is already zero, in stream order
     int block = 64;
     uint32_t refill_min = 8;
     bool local_stack = false;        // descent stack in local memory instead of shared

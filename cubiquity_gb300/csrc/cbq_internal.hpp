@@ -141,5 +141,13 @@ struct cbq_dag {
     // Work counters of cbq_intersect's persistent form, one per stream id (ids are unique
     // for the context's lifetime, so launches sharing a counter are ordered by their stream).
     std::mutex counter_lock;
-    std::map<unsigned long long, uint64_t*> stream_counters;
+    // Each launch takes the next counter of its stream's ring, which is zeroed as a whole when it
+    // has been used up: one memset in kCounterRing launches.  Taking a counter and queueing its
+    // launch happen under counter_lock.
+    struct CounterRing {
+        uint64_t* at = nullptr;
+        uint32_t used = 0;
+    };
+    static constexpr uint32_t kCounterRing = 256;
+    std::map<unsigned long long, CounterRing> stream_counters;
 };

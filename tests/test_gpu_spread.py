@@ -83,3 +83,36 @@ def test_image_sizes(scene, n):
     want = cbq.intersect_volume(shaped, to, td)
     for k in want:
         assert want[k].cpu().numpy().tobytes() == host[k].tobytes(), k
+
+
+@pytest.mark.parametrize("shared_stream", [False, True])
+def test_launches_beyond_the_counter_ring(scene, shared_stream):
+    """600 persistent launches (a stream's ring holds 256 work counters) from three threads, on streams of
+    their own or all on one: every launch traverses all its rays."""
+    import threading
+    dag, shaped, warps, pools = scene
+    o, d = pools["collision"]
+    cuts = [o.shape[0] - k for k in (0, 1, 777)]  # beyond the spread sizes
+    want = cbq.intersect_volume(shaped, o, d)
+    torch.cuda.synchronize()
+    one, bad = torch.cuda.Stream(), []
+
+    def run(k):
+        torch.cuda.set_device(0)
+        stream = one if shared_stream else torch.cuda.Stream()
+        n = cuts[k]
+        for i in range(200):
+            with torch.cuda.stream(stream):
+                out = cbq.alloc_hits(n, fields=("hit", "distance"))
+                out["distance"].fill_(-1.0)
+                cbq.intersect_volume(dag, o[:n], d[:n], out=out, stream=stream)
+                same = torch.equal(out["hit"], want["hit"][:n]) and torch.equal(out["distance"], want["distance"][:n])
+            if not same:
+                bad.append((k, i))
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
