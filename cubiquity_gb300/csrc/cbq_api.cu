@@ -165,11 +165,15 @@ __global__ void __launch_bounds__(kStageBlock) cbq_k_host_out(const __grid_const
 
 // Whether all of a call's host buffers are page-locked (or managed): copies from and to them
 // are asynchronous.
-bool page_locked(const float* o, const float* d, const cbq_hits& h)
+bool page_locked(const float* o, const float* d, uint64_t n, const cbq_hits& h)
 {
-    const void* const buffers[] = {o, d, h.hit, h.distance, h.material, h.position, h.normal, h.voxel, h.status};
-    for (const void* p : buffers)
-        if (p && !device_alias(p)) return false;
+    const struct {
+        const void* p;
+        uint64_t width;
+    } buffers[] = {{o, 16},          {d, 16},       {h.hit, 1},    {h.distance, 4}, {h.material, 4},
+                   {h.position, 12}, {h.normal, 12}, {h.voxel, 12}, {h.status, 1}};
+    for (const auto& b : buffers)
+        if (b.p && !device_alias(b.p, n * b.width)) return false;
     return true;
 }
 
@@ -179,7 +183,7 @@ bool host_staging(const float* o, const float* d, uint64_t n, const cbq_hits& h,
                   const cbq_hits& dh, StageIn* in, HostOut* out, int* rows)
 {
     if (!aligned16(o) || !aligned16(d)) return false;
-    const void *ao = device_alias(o), *ad = ao ? device_alias(d) : nullptr;
+    const void *ao = device_alias(o, n * 16), *ad = ao ? device_alias(d, n * 16) : nullptr;
     if (!ad) return false;
     *in = StageIn{(const float4*)ao, (const float4*)ad, (float4*)d_o, (float4*)d_d, n, 0};
     struct Field {
@@ -194,7 +198,7 @@ bool host_staging(const float* o, const float* d, uint64_t n, const cbq_hits& h,
     *rows = 0;
     for (const Field& f : fields) {
         if (!f.host) continue;
-        char* host = (char*)device_alias(f.host);
+        char* host = (char*)device_alias(f.host, n * f.width);
         if (!host) return false;
         out->row[(*rows)++] = StageOut{(const char*)f.dev, host, n * f.width};
     }
@@ -884,7 +888,7 @@ extern "C" cbq_status cbq_intersect_host(const cbq_dag* cdag, const float* host_
     // and every chunk adds nine copies (300 K / 1 M bounce rays 434 -> 310 us, 1,015 -> 637).
     uint64_t chunks = 1, sum = weights[0];
     const bool overlaps = n >= kHostChunkMin * (sum + weights[1]) &&
-                          page_locked(host_origin_tmax, host_direction, *host_hits);
+                          page_locked(host_origin_tmax, host_direction, n, *host_hits);
     while (overlaps && chunks < kHostChunksMax && n >= kHostChunkMin * (sum + weights[chunks])) sum += weights[chunks++];
     StageIn stage_rays;
     HostOut stage_hits;

@@ -64,42 +64,31 @@ struct Request {
     cbq_status status = CBQ_OK;
 };
 
-// True when a device-to-host copy into `p` is asynchronous: page-locked or
-// managed host memory (into pageable memory the copy blocks the calling thread).
-bool copy_into_is_async(const void* p)
-{
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return a.type != cudaMemoryTypeUnregistered;
-}
-
 // Finds the device aliases of a request's buffers (rays_mapped, hits_mapped)
 // and whether copies into its hit buffers are asynchronous (out_async).
 void resolve_buffers(Request& rq)
 {
     const cbq_request& r = rq.r;
     if (!((uintptr_t)r.host_origin_tmax & 15u) && !((uintptr_t)r.host_direction & 15u)) {
-        rq.d_o = (const float*)device_alias(r.host_origin_tmax);
-        rq.d_d = rq.d_o ? (const float*)device_alias(r.host_direction) : nullptr;
+        rq.d_o = (const float*)device_alias(r.host_origin_tmax, r.ray_count * 16);
+        rq.d_d = rq.d_o ? (const float*)device_alias(r.host_direction, r.ray_count * 16) : nullptr;
         rq.rays_mapped = rq.d_o && rq.d_d;
     }
     const cbq_hits& h = r.host_hits;
     cbq_hits& d = rq.d_hits;
-    struct F { void* host; void** dev; };
-    const F fields[] = {{h.hit, (void**)&d.hit}, {h.distance, (void**)&d.distance}, {h.material, (void**)&d.material},
-                        {h.position, (void**)&d.position}, {h.normal, (void**)&d.normal},
-                        {h.voxel, (void**)&d.voxel}, {h.status, (void**)&d.status}};
+    struct F { void* host; void** dev; uint64_t width; };
+    const F fields[] = {{h.hit, (void**)&d.hit, 1}, {h.distance, (void**)&d.distance, 4},
+                        {h.material, (void**)&d.material, 4}, {h.position, (void**)&d.position, 12},
+                        {h.normal, (void**)&d.normal, 12}, {h.voxel, (void**)&d.voxel, 12},
+                        {h.status, (void**)&d.status, 1}};
     rq.hits_mapped = true;
     for (const F& f : fields) {
         *f.dev = nullptr;
         if (!f.host) continue;
-        if (rq.hits_mapped) *f.dev = (void*)device_alias(f.host);
-        if (*f.dev) continue;
-        rq.hits_mapped = false;
-        rq.out_async = rq.out_async && copy_into_is_async(f.host);
+        const HostRange range = host_range(f.host, r.ray_count * f.width);
+        *f.dev = (void*)range.device;
+        rq.hits_mapped = rq.hits_mapped && range.device;
+        rq.out_async = rq.out_async && range.whole;
     }
 }
 

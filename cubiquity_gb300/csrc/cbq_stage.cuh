@@ -8,6 +8,8 @@
 // so that the link carries full lines.
 #pragma once
 
+#include "cbq_hostmem.hpp"
+
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -75,20 +77,6 @@ __device__ __forceinline__ void stage_out(const StageOut& s, uint64_t first, uin
 inline unsigned stage_blocks(uint64_t items)
 {
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(64, (items + 2 * kStageBlock - 1) / (2 * kStageBlock)));
-}
-
-// The device address of host memory the GPU can use directly (page-locked and
-// mapped, or managed), or nullptr when the buffer has to be copied.
-inline const void* device_alias(const void* p)
-{
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (a.type == cudaMemoryTypeHost && a.devicePointer) return a.devicePointer;
-    if (a.type == cudaMemoryTypeManaged) return p;
-    return nullptr;
 }
 
 }  // namespace cbq
