@@ -1,5 +1,6 @@
 // Device-side C ABI: DAG upload, traversal launches (plain and persistent).
 #include "cbq_flat.cuh"
+#include "cbq_hostcopy.hpp"
 #include "cbq_internal.hpp"
 #include "cbq_stage.cuh"
 #include "cbq_traverse.cuh"
@@ -111,41 +112,19 @@ dev::HitsOut make_hits(const cbq_hits* h)
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-// One chunk of a cbq_intersect_host call.  The call's rays are cut into
-// kHostBlocksPerChunk blocks of `pitch` consecutive rays, and every chunk takes
-// `width` rays of each (its rows), from `offset` in the block: so every chunk
-// samples the whole batch (a camera batch whose first rows are sky and whose
-// middle rows are terrain), and the copies and traversals of consecutive chunks
-// stay in proportion.  The rays after the last block go to the last chunk.  On
-// the device a chunk's rays and hits are contiguous, from ray `start`; on the
-// host its rows are those of a pitched array.
-struct HostChunk {
-    uint64_t start = 0, width = 0, offset = 0, pitch = 0, rows = 0;
-    uint64_t tail = 0, tail_at = 0;  // rays after the last block, and the host index of the first
-    uint64_t rays() const { return rows * width + tail; }
-};
-
 // Copies `bytes` per ray of a chunk between the host array (every ray of the
 // call) and the device array (the chunk's rays from c.start).
-bool copy_chunk(void* host, void* dev, size_t bytes, const HostChunk& c, cudaMemcpyKind kind, cudaStream_t s)
+bool copy_chunk(void* host, void* dev, size_t bytes, const HostChunk& c, cudaMemcpyKind kind, uint64_t max_pitch,
+                cudaStream_t s)
 {
-    char* h = (char*)host + c.offset * bytes;
-    char* d = (char*)dev + c.start * bytes;
-    const size_t row = c.width * bytes, pitch = c.pitch * bytes;
     const bool in = kind == cudaMemcpyHostToDevice;
-    if (row != 0) {
-        const cudaError_t e = in ? cudaMemcpy2DAsync(d, row, h, pitch, row, c.rows, kind, s)
-                                 : cudaMemcpy2DAsync(h, pitch, d, row, row, c.rows, kind, s);
-        if (e != cudaSuccess) return false;
-    }
-    if (c.tail != 0) {
-        char* ht = (char*)host + c.tail_at * bytes;
-        char* dt = d + c.rows * row;
-        const cudaError_t e = in ? cudaMemcpyAsync(dt, ht, c.tail * bytes, kind, s)
-                                 : cudaMemcpyAsync(ht, dt, c.tail * bytes, kind, s);
-        if (e != cudaSuccess) return false;
-    }
-    return true;
+    return for_each_copy(c, bytes, max_pitch, [&](const HostCopy& x) {
+        char *h = (char*)host + x.host, *d = (char*)dev + x.dev;
+        if (x.rows == 1)
+            return (in ? cudaMemcpyAsync(d, h, x.width, kind, s) : cudaMemcpyAsync(h, d, x.width, kind, s)) == cudaSuccess;
+        return (in ? cudaMemcpy2DAsync(d, x.width, h, x.pitch, x.width, x.rows, kind, s)
+                   : cudaMemcpy2DAsync(h, x.pitch, d, x.width, x.width, x.rows, kind, s)) == cudaSuccess;
+    });
 }
 
 // The copies of a call in one chunk with page-locked buffers: one kernel each way.
@@ -883,13 +862,11 @@ extern "C" cbq_status cbq_intersect_host(const cbq_dag* cdag, const float* host_
     // the copies out then begin early and the larger chunks are traversed under them.  us per
     // call of 300 Ki / 1 Mi / 4 Mi bounce rays: chunks of 1:2:3:4 238 / 494 / 1,399; up to 8 equal
     // ones of 256 Ki rays or more 259 / 528 / 1,498, up to 8 of 1:2:3:4:4:.. 235 / 507 / 1,450.
-    static const unsigned weights[kHostChunksMax] = {1, 2, 3, 4};
     // Pageable buffers take one chunk: their copies block the calling thread, so nothing overlaps
     // and every chunk adds nine copies (300 K / 1 M bounce rays 434 -> 310 us, 1,015 -> 637).
-    uint64_t chunks = 1, sum = weights[0];
-    const bool overlaps = n >= kHostChunkMin * (sum + weights[1]) &&
-                          page_locked(host_origin_tmax, host_direction, n, *host_hits);
-    while (overlaps && chunks < kHostChunksMax && n >= kHostChunkMin * (sum + weights[chunks])) sum += weights[chunks++];
+    HostChunk plan[kHostChunksMax];
+    const bool overlaps = host_chunks(n) > 1 && page_locked(host_origin_tmax, host_direction, n, *host_hits);
+    const uint64_t chunks = plan_host_chunks(n, overlaps, plan);
     StageIn stage_rays;
     HostOut stage_hits;
     int stage_rows = 0;
@@ -917,27 +894,16 @@ extern "C" cbq_status cbq_intersect_host(const cbq_dag* cdag, const float* host_
         }
         return cudaStreamSynchronize(s) == cudaSuccess ? CBQ_OK : CBQ_ERR_CUDA;
     }
-    const uint64_t blocks = chunks == 1 ? 1 : kHostBlocksPerChunk, pitch = n / blocks;
-    uint64_t offset = 0, start = 0;
+    int max_pitch = 0;
+    if (cudaDeviceGetAttribute(&max_pitch, cudaDevAttrMaxPitch, dag->device) != cudaSuccess) return CBQ_ERR_CUDA;
     for (uint64_t k = 0; k < chunks; k++) {
-        HostChunk hc;
-        hc.start = start;
-        hc.offset = offset;
-        hc.pitch = pitch;
-        hc.rows = blocks;
-        hc.width = k + 1 < chunks ? pitch * weights[k] / sum / 32 * 32 : pitch - offset;
-        if (k + 1 == chunks) {
-            hc.tail_at = blocks * pitch;
-            hc.tail = n - hc.tail_at;
-        }
-        offset += hc.width;
-        const uint64_t a = start, m = hc.rays();
-        start += m;
+        const HostChunk& hc = plan[k];
+        const uint64_t a = hc.start, m = hc.rays();
         if (m == 0) continue;
         cudaStream_t s_run = hs->pipe[2 + (k & 1)];
         cudaEvent_t copied = hs->pipe_ev[2 * k], traversed = hs->pipe_ev[2 * k + 1];
-        if (!copy_chunk((void*)host_origin_tmax, d_o, 16, hc, cudaMemcpyHostToDevice, s_in) ||
-            !copy_chunk((void*)host_direction, d_d, 16, hc, cudaMemcpyHostToDevice, s_in) ||
+        if (!copy_chunk((void*)host_origin_tmax, d_o, 16, hc, cudaMemcpyHostToDevice, max_pitch, s_in) ||
+            !copy_chunk((void*)host_direction, d_d, 16, hc, cudaMemcpyHostToDevice, max_pitch, s_in) ||
             cudaEventRecord(copied, s_in) != cudaSuccess || cudaStreamWaitEvent(s_run, copied, 0) != cudaSuccess)
             return drain(CBQ_ERR_CUDA);
         cbq_hits launch;
@@ -966,7 +932,7 @@ extern "C" cbq_status cbq_intersect_host(const cbq_dag* cdag, const float* host_
                                {host_hits->status, dh.status, 1}};
         for (const Copy& c : copies) {
             if (!c.host) continue;
-            if (!copy_chunk(c.host, c.dev, c.width, hc, cudaMemcpyDeviceToHost, s_out)) return drain(CBQ_ERR_CUDA);
+            if (!copy_chunk(c.host, c.dev, c.width, hc, cudaMemcpyDeviceToHost, max_pitch, s_out)) return drain(CBQ_ERR_CUDA);
         }
     }
     return drain(CBQ_OK);

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "../../include/cubiquity_gb300.h"
+#include "cbq_hostcopy.hpp"
 
 #include <cstdint>
 #include <map>
@@ -58,13 +59,6 @@ cbq_status noalloc_prepare(int device);
 // host threads) each take their own staging set, up to kHostStagesMax of them;
 // beyond that they queue for one.
 constexpr int kHostStagesMax = 4;
-
-// cbq_intersect_host splits a call into at most kHostChunksMax chunks, the first
-// of at least kHostChunkMin rays.
-constexpr uint64_t kHostChunksMax = 4;
-constexpr uint64_t kHostChunkMin = 1ull << 16;
-// Blocks of the batch that every chunk takes a part of.
-constexpr uint64_t kHostBlocksPerChunk = 4;
 
 // Device staging and streams of one cbq_intersect_host call at a time: rays and
 // hits, copied in and out in chunks on four streams (copy in, copy out, two for
