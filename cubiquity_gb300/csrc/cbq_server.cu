@@ -40,7 +40,11 @@ namespace {
 using Clock = std::chrono::steady_clock;
 
 constexpr uint64_t kAlign = 256;
-constexpr size_t kInlineMaxInflight = 2;  // submit launches by itself below this many launches in flight
+// Submit launches by itself below this many launches in flight: when the server is idle.  A
+// launch costs the submitting thread 8 us beside a request's 1 us, so that with 2 a client
+// that submits in a row (every 12 us, from Python) launched nearly every request itself: 24
+// requests of 16 Ki rays 525 us, 256 of 2 Ki 5.4 ms; with 1, 470 us and 3.7 ms.
+constexpr size_t kInlineMaxInflight = 1;
 constexpr uint64_t kBytesPerRay = 16 + 16 + 12 + 12 + 12 + 4 + 4 + 1 + 1;  // rays in, all hit fields out
 
 uint64_t align_up(uint64_t v) { return (v + kAlign - 1) & ~(kAlign - 1); }
@@ -65,7 +69,10 @@ struct Request {
 };
 
 // Finds the device aliases of a request's buffers (rays_mapped, hits_mapped)
-// and whether copies into its hit buffers are asynchronous (out_async).
+// and whether copies into its hit buffers are asynchronous (out_async).  Nine
+// driver queries, which wait for the other threads' launches: made by the thread
+// that launches the request, not by the one that submits it (256 requests of 2 Ki
+// rays submitted natively 1,300 -> 730 us).
 void resolve_buffers(Request& rq)
 {
     const cbq_request& r = rq.r;
@@ -280,6 +287,7 @@ cbq_status cbq_server::enqueue(Slot& s, const std::vector<Request*>& group)
     // First pass: where every request's rays and hits are on the device, the job and
     // staging tables, and the copies in that the staging kernel does not make.
     for (Request* rq : group) {
+        if (!(cfg.flags & CBQ_SERVER_IN_PLACE)) resolve_buffers(*rq);
         const uint64_t n = rq->r.ray_count;
         dev::JobDesc jd;
         std::memset(&jd, 0, sizeof(jd));
@@ -578,7 +586,7 @@ cbq_status cbq_server_submit(cbq_server* s, const cbq_request* r, uint64_t* tick
     if (!rq) return CBQ_ERR_OUT_OF_MEMORY;
     rq->submitted = Clock::now();
     rq->r = *r;
-    if (r->ray_count > 0) resolve_buffers(*rq);
+    if (r->ray_count > 0 && (s->cfg.flags & CBQ_SERVER_IN_PLACE)) resolve_buffers(*rq);
     rq->direct = (s->cfg.flags & CBQ_SERVER_IN_PLACE) && rq->rays_mapped && rq->hits_mapped;
     rq->bytes = rq->direct ? 0 : request_bytes(r->ray_count);
     if (rq->bytes > s->cfg.device_memory_budget) {
@@ -599,9 +607,9 @@ cbq_status cbq_server_submit(cbq_server* s, const cbq_request* r, uint64_t* tick
         return CBQ_OK;
     }
     s->live[rq->ticket] = 1;
-    // A lightly loaded device (nothing queued, under two launches in flight), a slot and
-    // memory free: launch from this thread, one thread hand-off fewer than through the
-    // scheduler (arrival order is kept).  Under load, requests queue and leave in groups.
+    // An idle server (nothing queued or in flight), a slot and memory free: launch from this
+    // thread, one thread hand-off fewer than through the scheduler (arrival order is kept).
+    // Otherwise requests queue and leave in groups.
     uint64_t off = 0;
     if (s->queue.empty() && s->inflight.size() + s->inline_pending < kInlineMaxInflight &&
         !s->free_slots.empty() && (rq->bytes == 0 || s->pool.alloc(rq->bytes, &off))) {
