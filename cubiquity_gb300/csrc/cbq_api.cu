@@ -669,8 +669,7 @@ cbq_status cbq_dag_get_launch_config(const cbq_dag* dag, cbq_launch_config* cfg)
     if (cfg->kernel == CBQ_KERNEL_AUTO) cfg->kernel = CBQ_KERNEL_FLAT;
     if (cfg->block == 0) cfg->block = use_flat(dag) ? kFlatBlockDefault : kPlainBlock;
     if (cfg->chunk == 0) cfg->chunk = kDefaultChunk;
-    if (cfg->refill_min == 0) cfg->refill_min = kRefillDefault;
-    if (cfg->steps == 0) cfg->steps = kStepsDefault;
+    // refill_min and steps stay 0 where they are automatic: no fixed value gives the same launches.
     return CBQ_OK;
 }
 

@@ -205,6 +205,9 @@ typedef struct cbq_launch_config {
 } cbq_launch_config;
 
 cbq_status cbq_dag_set_launch_config(cbq_dag* dag, const cbq_launch_config* cfg);
+/* The configuration in use: setting it (on this or another DAG) gives the same
+ * launches.  Defaults that are one value come as that value; refill_min and
+ * steps are 0 where they are automatic. */
 cbq_status cbq_dag_get_launch_config(const cbq_dag* dag, cbq_launch_config* cfg);
 
 /* Device scratch cbq_intersect_auto needs for n rays (work counter, octant
