@@ -56,8 +56,7 @@ FlatLaunch flat_launch(const cbq_dag* dag, bool persistent, uint64_t* counter, u
 // takes one thread per ray (kPlainImageRays), else 0.
 uint32_t spread_rays(const cbq_dag* dag, uint64_t n, const cbq_query* query)
 {
-    const bool own = dag->cfg.refill_min != 0 || dag->cfg.steps != 0 || dag->cfg.form != CBQ_FORM_PERSISTENT;
-    if (own) return 0u;
+    if (own_shape(dag->cfg)) return 0u;
     const uint32_t spread = spread_warp_rays(n, dag->device);
     return !spread && query && query->image_width && n <= kPlainImageRays ? 32u : spread;
 }

@@ -294,8 +294,6 @@ using namespace cbq;
 
 namespace {
 constexpr int kBatchBlockDefault = 128;
-constexpr uint32_t kBatchRefillDefault = 16;
-constexpr int32_t kBatchStepsDefault = 8;
 }  // namespace
 
 struct cbq_batch {
@@ -311,11 +309,9 @@ struct cbq_batch {
     uint64_t* d_counter = nullptr;
     uint32_t* d_sort = nullptr;             // octant order: 16 uint32 per job, then one index per ray
     cbq_query query{1, CBQ_MAX_FOOTPRINT_DISABLED, 0u, 0u};
-    // 12 volumes, 2.2 M rays, shared stack: refill 16 at 8 iterations 264 us, refill 8 275 us.  The
-    // stack's place is set by batch_stack_in_shared.
+    // The stack's place is set by batch_stack_in_shared.
     cbq_batch_config cfg{kBatchBlockDefault, kBatchRefillDefault, kBatchStepsDefault, 0, CBQ_STACK_LOCAL,
                          CBQ_FORM_PERSISTENT};
-    bool own_shape = false;                 // refill or steps set by the caller or the tuner
     cudaGraphExec_t exec = nullptr;
     // Persisting L2 window set on the graph's kernel nodes (l2_bytes 0: none).
     void* l2_base = nullptr;
@@ -333,7 +329,7 @@ BatchLaunch batch_launch(const cbq_batch* b, const uint32_t* perm)
     bl.steps = (uint32_t)b->cfg.steps;
     bl.shared_stack = b->cfg.stack == CBQ_STACK_SHARED;
     bl.stack_rows = b->stack_rows;
-    bl.spread = !b->own_shape;
+    bl.spread = !own_shape(b->cfg);
     bl.lod = !(b->query.max_footprint < 0.0f);
     bl.perm = perm;
     return bl;
@@ -531,7 +527,6 @@ cbq_status cbq_batch_set_config(cbq_batch* b, int32_t block, uint32_t refill_min
     if (!b || block < 0 || block > 256 || (block % 32) != 0 || refill_min > 32) return CBQ_ERR_INVALID_ARGUMENT;
     b->cfg.block = block ? block : kBatchBlockDefault;
     b->cfg.refill_min = refill_min ? refill_min : kBatchRefillDefault;
-    b->own_shape = refill_min != 0;
     drop_graph(b);
     return CBQ_OK;
 }
@@ -552,7 +547,6 @@ cbq_status cbq_batch_set_launch_config(cbq_batch* b, const cbq_batch_config* cfg
     if (st != CBQ_OK) return st;
     if (cfg->form == CBQ_FORM_SORTED && (st = ensure_sort_scratch(b)) != CBQ_OK) return st;
     b->cfg = *cfg;
-    b->own_shape = true;
     drop_graph(b);
     return CBQ_OK;
 }
@@ -622,8 +616,6 @@ cbq_status cbq_batch_autotune(cbq_batch* b, cbq_stream_t stream, int32_t repetit
     cudaEvent_t e0, e1;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return CBQ_ERR_CUDA;
     const cbq_batch_config saved = b->cfg;
-    const bool saved_own = b->own_shape;
-    b->own_shape = true;
     cbq_batch_config best_cfg = saved;
     float best = 1e30f;
     cbq_status st = CBQ_OK;
@@ -655,7 +647,6 @@ cbq_status cbq_batch_autotune(cbq_batch* b, cbq_stream_t stream, int32_t repetit
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     b->cfg = st == CBQ_OK ? best_cfg : saved;
-    if (st != CBQ_OK) b->own_shape = saved_own;
     drop_graph(b);
     if (st == CBQ_OK)
         cbq::log(CBQ_LOG_INFO,

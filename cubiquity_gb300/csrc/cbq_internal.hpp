@@ -94,6 +94,23 @@ cbq_status intersect_device_count(const cbq_dag* dag, const cbq_rays* rays, uint
                                   const cbq_query* query, const cbq_hits* hits, uint64_t* zeroed_counter,
                                   cbq_stream_t stream);
 
+// Batch launches: 12 volumes, 2.2 M rays, shared stack: refill 16 at 8 iterations 264 us, refill 8
+// 275 us.
+constexpr uint32_t kBatchRefillDefault = 16;
+constexpr int32_t kBatchStepsDefault = 8;
+
+// Whether a configuration sets a launch shape of its own; otherwise small launches are spread
+// over the chip (spread_warp_rays).  It depends on the values alone, so a configuration that was
+// read and set again gives the same launches.
+inline bool own_shape(const cbq_launch_config& c)
+{
+    return c.refill_min != 0 || c.steps != 0 || c.form != CBQ_FORM_PERSISTENT;
+}
+inline bool own_shape(const cbq_batch_config& c)
+{
+    return c.refill_min != kBatchRefillDefault || c.steps != kBatchStepsDefault || c.form != CBQ_FORM_PERSISTENT;
+}
+
 }  // namespace cbq
 
 // The opaque DAG handle.

@@ -322,7 +322,10 @@ cbq_status cbq_batch_create(const cbq_job* jobs, int32_t job_count, const cbq_qu
 cbq_status cbq_batch_set_config(cbq_batch* b, int32_t block, uint32_t refill_min);
 cbq_status cbq_batch_get_config(const cbq_batch* b, int32_t* block, uint32_t* refill_min, uint64_t* total_rays);
 
-/* The batch's full launch configuration.  Every choice gives the same results. */
+/* The batch's full launch configuration.  Every choice gives the same results.
+ * Refill 16 at 8 steps in CBQ_FORM_PERSISTENT is the default shape, with which a
+ * batch small enough for the device to hold all its rays at once is spread over
+ * the SMs; any other value is taken as it is. */
 typedef struct cbq_batch_config {
     int32_t block;            /* threads per block: 32..256, a multiple of 32 */
     uint32_t refill_min;      /* idle lanes that trigger a warp's refill: 1..32 */
