@@ -585,17 +585,13 @@ cbq_status cbq_intersect_auto(const cbq_dag* dag, const cbq_rays* rays, uint64_t
     uint64_t* counter = (uint64_t*)scratch;
     uint32_t* counts = (uint32_t*)((char*)scratch + 64);
     uint32_t* perm = (uint32_t*)((char*)scratch + 256);
-    const int form = dag->cfg.form;
-    if (form == CBQ_FORM_PLAIN || !use_flat(dag)) {
-        if (form == CBQ_FORM_PLAIN) return cbq_intersect(dag, rays, n, query, hits, stream);
+    if (dag->cfg.form == CBQ_FORM_PLAIN) return cbq_intersect(dag, rays, n, query, hits, stream);
+    if (dag->cfg.form == CBQ_FORM_PERSISTENT || !use_flat(dag))
         return cbq_intersect_persistent(dag, rays, n, query, hits, counter, 0u, stream);
-    }
+    st = launch_octant_sort((const float4*)rays->direction, n, counts, perm, dag->device, (cudaStream_t)stream);
+    if (st != CBQ_OK) return st;
     FlatLaunch fl = flat_launch(dag, true, counter, 0u);
-    if (form == CBQ_FORM_SORTED) {
-        st = launch_octant_sort((const float4*)rays->direction, n, counts, perm, dag->device, (cudaStream_t)stream);
-        if (st != CBQ_OK) return st;
-        fl.perm = perm;
-    }
+    fl.perm = perm;
     return launch_flat(dag, make_dag_params(dag), make_query(query), make_hits(hits),
                        (const float4*)rays->origin_tmax, (const float4*)rays->direction, n, nullptr, fl,
                        (cudaStream_t)stream);
@@ -613,41 +609,27 @@ cbq_status cbq_autotune(cbq_dag* dag, const cbq_rays* rays, uint64_t n, const cb
     cbq_launch_config winner = saved;
     float win_ms = 1e30f;
     cbq_status st = CBQ_OK;
-    static const int blocks[] = {64, 128, 256};
-    static const uint32_t refills[] = {8, 16, 24};
-    static const int stacks[] = {CBQ_STACK_SHARED, CBQ_STACK_LOCAL};
-    static const int step_counts[] = {4, 8, 16, 32};
-    for (int form = CBQ_FORM_PLAIN; form <= CBQ_FORM_SORTED && st == CBQ_OK; form++) {
-        for (int blk : blocks) {
-            for (uint32_t rf : refills) {
-                if (form == CBQ_FORM_PLAIN && rf != refills[0]) continue;  // refill unused
-                for (int v = 0; v < 8; v++) {
-                    cbq_launch_config c = saved;
-                    c.kernel = CBQ_KERNEL_FLAT;
-                    c.block = blk;
-                    c.refill_min = rf;
-                    c.stack = stacks[v & 1];
-                    c.form = form;
-                    c.steps = step_counts[v >> 1];
-                    c.registers = 0;
-                    dag->cfg = c;
-                    st = cbq_intersect_auto(dag, rays, n, query, hits, scratch, scratch_bytes, stream);  // warm-up
-                    if (st != CBQ_OK) break;
-                    cudaEventRecord(e0, (cudaStream_t)stream);
-                    for (int r = 0; r < repetitions && st == CBQ_OK; r++)
-                        st = cbq_intersect_auto(dag, rays, n, query, hits, scratch, scratch_bytes, stream);
-                    cudaEventRecord(e1, (cudaStream_t)stream);
-                    if (st != CBQ_OK || cudaEventSynchronize(e1) != cudaSuccess) { st = CBQ_ERR_CUDA; break; }
-                    float ms = 0;
-                    cudaEventElapsedTime(&ms, e0, e1);
-                    ms /= (float)repetitions;
-                    if (ms < win_ms) { win_ms = ms; winner = c; }
-                }
-                if (st != CBQ_OK) break;
-            }
-            if (st != CBQ_OK) break;
+    for_each_tuned_config(saved, [&](const cbq_launch_config& c) {
+        dag->cfg = c;
+        st = cbq_intersect_auto(dag, rays, n, query, hits, scratch, scratch_bytes, stream);  // warm-up
+        if (st != CBQ_OK) return false;
+        cudaEventRecord(e0, (cudaStream_t)stream);
+        for (int r = 0; r < repetitions && st == CBQ_OK; r++)
+            st = cbq_intersect_auto(dag, rays, n, query, hits, scratch, scratch_bytes, stream);
+        cudaEventRecord(e1, (cudaStream_t)stream);
+        if (st != CBQ_OK || cudaEventSynchronize(e1) != cudaSuccess) {
+            st = CBQ_ERR_CUDA;
+            return false;
         }
-    }
+        float ms = 0;
+        cudaEventElapsedTime(&ms, e0, e1);
+        ms /= (float)repetitions;
+        if (ms < win_ms) {
+            win_ms = ms;
+            winner = c;
+        }
+        return true;
+    });
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     dag->cfg = st == CBQ_OK ? winner : saved;

@@ -111,6 +111,32 @@ inline bool own_shape(const cbq_batch_config& c)
     return c.refill_min != kBatchRefillDefault || c.steps != kBatchStepsDefault || c.form != CBQ_FORM_PERSISTENT;
 }
 
+// The configurations that cbq_autotune times, as long as f(configuration) is true: every form,
+// block size and stack; one thread per ray at four step counts, the refilled forms at the
+// automatic shape and at three refills by four step counts.
+template <typename F>
+void for_each_tuned_config(const cbq_launch_config& base, F f)
+{
+    for (int form = CBQ_FORM_PLAIN; form <= CBQ_FORM_SORTED; form++)
+        for (int block : {64, 128, 256})
+            for (uint32_t refill : {0u, 8u, 16u, 24u}) {
+                if (form == CBQ_FORM_PLAIN && refill != 0u) continue;  // refill unused
+                for (int steps : {0, 4, 8, 16, 32})
+                    for (int stack : {CBQ_STACK_SHARED, CBQ_STACK_LOCAL}) {
+                        if ((steps == 0) != (refill == 0u && form != CBQ_FORM_PLAIN)) continue;
+                        cbq_launch_config c = base;
+                        c.kernel = CBQ_KERNEL_FLAT;
+                        c.block = block;
+                        c.refill_min = refill;
+                        c.stack = stack;
+                        c.form = form;
+                        c.steps = steps;
+                        c.registers = 0;
+                        if (!f(c)) return;
+                    }
+            }
+}
+
 }  // namespace cbq
 
 // The opaque DAG handle.

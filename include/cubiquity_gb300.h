@@ -220,9 +220,10 @@ uint64_t cbq_scratch_bytes(uint64_t n);
 cbq_status cbq_intersect_auto(const cbq_dag* dag, const cbq_rays* rays, uint64_t n, const cbq_query* query,
                               const cbq_hits* hits, void* scratch, uint64_t scratch_bytes, cbq_stream_t stream);
 
-/* Autotuner: times every form x block {64,128,256} x refill {8,16,24} x stack
- * {shared, local} x steps {4,8,16,32} on these rays (synchronous; `repetitions`
- * launches each), stores the fastest in the DAG's launch config and returns it with its time. */
+/* Autotuner: times every form x block {64,128,256} x stack {shared, local} x
+ * {the automatic refill and steps, refill {8,16,24} x steps {4,8,16,32}} on these
+ * rays (synchronous; `repetitions` launches each), stores the fastest in the
+ * DAG's launch config and returns it with its time. */
 cbq_status cbq_autotune(cbq_dag* dag, const cbq_rays* rays, uint64_t n, const cbq_query* query,
                         const cbq_hits* hits, void* scratch, uint64_t scratch_bytes, int32_t repetitions,
                         cbq_launch_config* best, float* best_ms, cbq_stream_t stream);

@@ -1,5 +1,6 @@
 // Prints whether launch configurations count as a shape of the caller's own
-// (cbq_internal.hpp): "volume" and "batch", refill, steps and form per line.
+// (cbq_internal.hpp): "volume" and "batch", refill, steps and form per line; then
+// the configurations the tuner times: "tuned", form, block, refill, steps, stack.
 #include "../cubiquity_gb300/csrc/cbq_internal.hpp"
 
 #include <cstdio>
@@ -17,5 +18,11 @@ int main()
                 std::printf("volume %u %d %d %d\nbatch %u %d %d %d\n", refill, steps, form, cbq::own_shape(v), refill,
                             steps, form, cbq::own_shape(b));
             }
+    cbq_launch_config base{};
+    base.chunk = 77;
+    cbq::for_each_tuned_config(base, [](const cbq_launch_config& c) {
+        std::printf("tuned %d %d %u %d %d\n", c.form, c.block, c.refill_min, c.steps, c.chunk == 77 ? c.stack : -1);
+        return true;
+    });
     return 0;
 }
