@@ -4,9 +4,9 @@ The native tuner (cbq_autotune) times every form (one thread per ray,
 persistent with lane refill, octant-sorted persistent) x block size x refill
 threshold x stack placement (shared or local memory) on the caller's rays and
 keeps the fastest.  Results are cached in a JSON file keyed by GPU, DAG size
-class (rounded log2 of its bytes) and ray mix (coherent or incoherent, from
-how often consecutive rays share an octant), so a known configuration is
-applied without re-timing.
+class (rounded log2 of its bytes), ray count class (likewise) and ray mix
+(coherent or incoherent, from how often consecutive rays share an octant), so a
+known configuration is applied without re-timing.
 """
 from __future__ import annotations
 
@@ -39,8 +39,10 @@ def cache_key(dag: cbq.Dag, direction) -> str:
     gpu = torch.cuda.get_device_name() if torch.cuda.is_available() else "cpu"
     size_class = int(round(math.log2(max(1, dag.bytes))))
     layout = "|compact" if getattr(dag, "layout", 0) == cbq.LAYOUT_COMPACT else ""
+    # A call of a thousand rays and one of millions are best served by different launches.
+    count_class = int(round(math.log2(max(1, int(direction.shape[0])))))
     # "walk2": shapes tuned for another walk are not taken over.
-    return f"{gpu}|dag2^{size_class}{layout}|{ray_mix(direction)}|walk2"
+    return f"{gpu}|dag2^{size_class}{layout}|rays2^{count_class}|{ray_mix(direction)}|walk2"
 
 
 def _load() -> dict:
