@@ -186,7 +186,7 @@ bool host_staging(const float* o, const float* d, uint64_t n, const cbq_hits& h,
 // A zeroed work counter of the persistent form for the next launch on `stream`
 // (from the stream's ring, allocated on first use), or nullptr where none can be
 // had: the id query fails, or the stream is being captured (no allocation inside
-// a capture).  The launch is queued while `lk` holds counter_lock.  A memset
+// a capture).  The launch is queued while `lk` is held.  A memset
 // before every launch took 2 us of the stream (1.5 M shadow rays 123.4 us,
 // without 121.4; city camera with LOD 150.5, 148.7).
 uint64_t* stream_counter(const cbq_dag* cdag, cudaStream_t stream, std::unique_lock<std::mutex>& lk)
@@ -204,24 +204,20 @@ uint64_t* stream_counter(const cbq_dag* cdag, cudaStream_t stream, std::unique_l
         cudaGetLastError();
         return nullptr;
     }
-    lk = std::unique_lock<std::mutex>(dag->counter_lock);
-    cbq_dag::CounterRing& ring = dag->stream_counters[id];
-    if (!ring.at) {
-        if (cudaMalloc((void**)&ring.at, cbq_dag::kCounterRing * sizeof(uint64_t)) != cudaSuccess) {
+    return dag->stream_counters.take(
+        id,
+        [] {
+            void* p = nullptr;
+            if (cudaMalloc(&p, CounterRings::kSize * sizeof(uint64_t)) == cudaSuccess) return (uint64_t*)p;
             cudaGetLastError();
-            ring.at = nullptr;
-            return nullptr;
-        }
-        ring.used = cbq_dag::kCounterRing;
-    }
-    if (ring.used == cbq_dag::kCounterRing) {
-        if (cudaMemsetAsync(ring.at, 0, cbq_dag::kCounterRing * sizeof(uint64_t), stream) != cudaSuccess) {
+            return (uint64_t*)nullptr;
+        },
+        [&](uint64_t* ring) {
+            if (cudaMemsetAsync(ring, 0, CounterRings::kSize * sizeof(uint64_t), stream) == cudaSuccess) return true;
             cudaGetLastError();
-            return nullptr;
-        }
-        ring.used = 0;
-    }
-    return ring.at + ring.used++;
+            return false;
+        },
+        lk);
 }
 
 cbq_status check_rays(const cbq_rays* rays)
@@ -467,8 +463,7 @@ cbq_status cbq_dag_destroy(cbq_dag* dag)
 {
     if (!dag) return CBQ_ERR_INVALID_ARGUMENT;
     cudaFree(dag->d_nodes);
-    for (auto& kv : dag->stream_counters)
-        if (kv.second.at) cudaFree(kv.second.at);
+    dag->stream_counters.release([](uint64_t* ring) { cudaFree(ring); });
     pt_workspace_release(dag->pt);
     for (auto& hs : dag->stages) {
         if (hs->d_stage) cudaFree(hs->d_stage);

@@ -3,10 +3,10 @@
 #pragma once
 
 #include "../../include/cubiquity_gb300.h"
+#include "cbq_counters.hpp"
 #include "cbq_hostcopy.hpp"
 
 #include <cstdint>
-#include <map>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -175,16 +175,5 @@ struct cbq_dag {
     std::vector<std::unique_ptr<cbq::HostStage>> stages;
     std::mutex pt_lock;  // held by the frame that uses `pt`
     cbq::PtWorkspace pt;
-    // Work counters of cbq_intersect's persistent form, one per stream id (ids are unique
-    // for the context's lifetime, so launches sharing a counter are ordered by their stream).
-    std::mutex counter_lock;
-    // Each launch takes the next counter of its stream's ring, which is zeroed as a whole when it
-    // has been used up: one memset in kCounterRing launches.  Taking a counter and queueing its
-    // launch happen under counter_lock.
-    struct CounterRing {
-        uint64_t* at = nullptr;
-        uint32_t used = 0;
-    };
-    static constexpr uint32_t kCounterRing = 256;
-    std::map<unsigned long long, CounterRing> stream_counters;
+    cbq::CounterRings stream_counters;  // of cbq_intersect's persistent form
 };
