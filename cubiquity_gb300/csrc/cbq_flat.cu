@@ -273,7 +273,9 @@ cbq_status launch_counted(const Ctx& c, uint64_t n, const FlatLaunch& fl, int ro
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, fl.block, smem) != cudaSuccess)
         return CBQ_ERR_CUDA;
     const uint64_t full = (uint64_t)sms * std::max(per_sm, 1);
-    const unsigned grid = (unsigned)std::min<uint64_t>(full, (n + 31) / 32);  // n may be far above the count
+    // A warp for every ray, as far as the chip holds them (n may be far above the count).
+    const uint64_t warps = (uint64_t)fl.block / 32u;
+    const unsigned grid = (unsigned)std::min<uint64_t>(full, (n + warps - 1) / warps);
     kernel<<<grid, fl.block, smem, stream>>>(c, n, (unsigned long long*)fl.counter, fl.refill_min, fl.steps, fl.n_dev);
     return cudaGetLastError() == cudaSuccess ? CBQ_OK : CBQ_ERR_CUDA;
 }

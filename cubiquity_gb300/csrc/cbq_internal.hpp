@@ -75,14 +75,17 @@ struct HostStage {
 // frames (at most kPtKeptBytes of memory); a frame that finds it in use by another
 // thread makes its own.
 constexpr uint64_t kPtKeptBytes = 1ull << 30;
+// Waves that a frame is queued ahead of the last one whose ray count the host has looked at.
+constexpr int kPtAhead = 4;
 struct PtWorkspace {
     char* base = nullptr;
     uint64_t bytes = 0;
     struct CUstream_st* wave = nullptr;    // extension waves and shading (higher priority)
     struct CUstream_st* shadow = nullptr;  // shadow waves
     struct CUevent_st* begin = nullptr;
-    struct CUevent_st* shaded[2] = {};     // a depth's shadow rays are written
+    struct CUevent_st* shaded[kPtAhead] = {};  // a depth's shadow rays are written
     struct CUevent_st* traced[2] = {};     // ... and traced (their set may be written again)
+    uint32_t* seen = nullptr;              // page-locked: the ray counts of the last kPtAhead waves shaded
 };
 void pt_workspace_release(PtWorkspace& w);
 
