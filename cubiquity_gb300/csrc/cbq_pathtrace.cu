@@ -341,8 +341,16 @@ extern "C" cbq_status cbq_pathtrace(const cbq_dag* dag, const cbq_pt_config* cfg
             host_sh.emission[m][a] = cfg->materials[m].emission[a];
         }
 
-    // Buffers for one pass: two extension sets (ping-pong) and two shadow sets (a depth's
-    // shadow wave runs beside the next depth's extension wave).
+    // Without a wave callback the host waits for nothing until the frame is done: a wave's ray
+    // count stays on the device (the shading that compacts the next wave's rays leaves it
+    // there), and shadow waves run on a stream of their own beside the next extension wave,
+    // each filling the SMs that the other's last rays leave.
+    const bool ahead = !on_wave && cbq::takes_device_count(dag);
+    // Buffers for one pass: two extension sets (ping-pong) and one shadow set (260 bytes a path),
+    // or two where a depth's shadow wave may still run while the next depth is shaded (358): in
+    // frames whose workspace is kept.  ms, one set / two: city-2048, 4 bounces, 1920x1080 1.69 /
+    // 1.58, 640x360 0.53 / 0.48; with 2 samples, where the workspace is allocated for the frame,
+    // 3.63 / 3.80, 16 samples 23.0 / 23.6 (their waves fill the chip by themselves).
     const uint64_t per_pass = std::max<uint64_t>(
         1, std::min<uint64_t>((uint64_t)cfg->samples_per_pixel, kPtRaysPerPass / npix));
     const size_t ext = npix * per_pass, sha = 2 * ext;
@@ -350,20 +358,19 @@ extern "C" cbq_status cbq_pathtrace(const cbq_dag* dag, const cbq_pt_config* cfg
     const size_t waves = passes * ((size_t)cfg->bounces + 1);
     const size_t per_ext = 2 * 16 + sizeof(PathState) + 1 + 4 + 12 + 12;
     const size_t control = waves * (8 + 2 * 8);  // per wave: shadow and next count, two work counters
-    const size_t bytes = 2 * (ext * per_ext + sha * (16 * 3 + 1)) + control + sizeof(Shading) + 40 * 256;  // + carve padding
+    const auto frame_bytes = [&](int sets) {
+        return 2 * ext * per_ext + sets * sha * (16 * 3 + 1) + control + sizeof(Shading) + 40 * 256;  // + carve padding
+    };
+    const int sets = ahead && frame_bytes(2) <= cbq::kPtKeptBytes ? 2 : 1;
+    const size_t bytes = frame_bytes(sets);
 
     // The DAG's workspace, or one of this frame's own where another frame has it.
     cbq_dag* owner = const_cast<cbq_dag*>(dag);
     std::unique_lock<std::mutex> lock(owner->pt_lock, std::try_to_lock);
     cbq::PtWorkspace own;
     cbq::PtWorkspace& ws = lock.owns_lock() ? owner->pt : own;
-    // Without a wave callback the host waits for nothing until the frame is done: a wave's ray
-    // count stays on the device (the shading that compacts the next wave's rays leaves it
-    // there), and shadow waves run on a stream of their own beside the next extension wave,
-    // each filling the SMs that the other's last rays leave.
-    const bool ahead = !on_wave && cbq::takes_device_count(dag);
-    // But the paths of a frame of many bounces may all have ended long before the last, so each
-    // shading also leaves its wave's count in host memory, and the host looks at it kPtAhead waves
+    // The paths of a frame of many bounces may all have ended long before the last, so each
+    // shading (ahead) also leaves its wave's count in host memory, and the host looks at it kPtAhead waves
     // later, which keeps the device busy: smaller grids, and no more waves once one had no rays.
     // One sphere, 64 bounces: 640x360 1,030 -> 295 us, 2048x2048, 10 samples 25.2 -> 8.7 ms.
     const bool look = ahead && cfg->bounces >= cbq::kPtAhead;
@@ -394,6 +401,8 @@ extern "C" cbq_status cbq_pathtrace(const cbq_dag* dag, const cbq_pt_config* cfg
         e[k].material = carve<uint32_t>(p, ext);
         e[k].position = carve<float>(p, 3 * ext);
         e[k].normal = carve<float>(p, 3 * ext);
+    }
+    for (int k = 0; k < sets; k++) {
         s2[k].o = carve<float4>(p, sha);
         s2[k].d = carve<float4>(p, sha);
         s2[k].w = carve<float4>(p, sha);
@@ -457,7 +466,7 @@ extern "C" cbq_status cbq_pathtrace(const cbq_dag* dag, const cbq_pt_config* cfg
             }
             Ext& E = e[cur];
             Ext& N = e[cur ^ 1];
-            const int set = (int)(wave & 1u);
+            const int set = (int)(wave % (size_t)sets);
             Sha& S = s2[set];
             uint32_t* count = (uint32_t*)(counts + wave);                 // [0] shadow rays, [1] next extension rays
             uint64_t* work = counts + waves + 2 * wave;                   // extension and shadow work counters
