@@ -72,14 +72,16 @@ struct HostStage {
 };
 
 // The pathtracer's device memory, streams and events.  A DAG keeps one set between
-// frames (at most kPtKeptBytes of memory); a frame that finds it in use by another
-// thread makes its own.
+// frames; a frame that finds it in use by another thread makes its own.  The memory
+// kept is at most kPtKeptBytes over all DAGs of the process: a frame that would go
+// beyond gives its own back when it is done.
 constexpr uint64_t kPtKeptBytes = 1ull << 30;
 // Waves that a frame is queued ahead of the last one whose ray count the host has looked at.
 constexpr int kPtAhead = 4;
 struct PtWorkspace {
     char* base = nullptr;
     uint64_t bytes = 0;
+    uint64_t kept = 0;                     // its part of the memory kept by the process
     struct CUstream_st* wave = nullptr;    // extension waves and shading (higher priority)
     struct CUstream_st* shadow = nullptr;  // shadow waves
     struct CUevent_st* begin = nullptr;

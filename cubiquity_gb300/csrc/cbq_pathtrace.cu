@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -223,11 +224,28 @@ __global__ void cbq_k_pt_scale(float* image, size_t count, float scale)
     if (i < count) image[i] *= scale;
 }
 
+std::atomic<uint64_t> g_kept{0};  // bytes of the workspaces kept between frames
+
 void release_memory(cbq::PtWorkspace& w)
 {
     if (w.base) cudaFree(w.base);
     w.base = nullptr;
     w.bytes = 0;
+    g_kept -= w.kept;
+    w.kept = 0;
+}
+
+// After a frame: keeps the memory of `w` for the next, or gives it back.
+void keep_or_release(cbq::PtWorkspace& w)
+{
+    const uint64_t more = w.bytes - w.kept;  // a kept workspace only grows
+    uint64_t total = g_kept.load();
+    while (total + more <= cbq::kPtKeptBytes && !g_kept.compare_exchange_weak(total, total + more)) {
+    }
+    if (total + more <= cbq::kPtKeptBytes)
+        w.kept = w.bytes;
+    else
+        release_memory(w);
 }
 
 template <typename F>
@@ -561,7 +579,7 @@ extern "C" cbq_status cbq_pathtrace(const cbq_dag* dag, const cbq_pt_config* cfg
         ext_rays += h_counts[w] >> 32;
     }
     if (!lock.owns_lock()) cbq::pt_workspace_release(own);
-    else if (ws.bytes > cbq::kPtKeptBytes) release_memory(ws);
+    else keep_or_release(ws);
     if (stats) {
         stats->extension_rays = ext_rays;
         stats->shadow_rays = shadow_rays;

@@ -51,3 +51,27 @@ def test_kept_between_frames(scene):
     torch.cuda.empty_cache()
     assert _used() - before <= SLACK
     dag.destroy()
+
+
+def test_kept_over_all_volumes(scene):
+    """Nine volumes that rendered a frame of 330 MB keep 1 GiB together; destroyed, nothing."""
+    before = _used()
+    dags = [cbq.Dag(*scene) for _ in range(9)]
+    volumes = _used() - before
+    want = None
+    for dag in dags + dags[::-1]:
+        image, stats = _frame(dag, 640, 360, 4)
+        want = stats if want is None else want
+        assert stats["extension_rays"] == want["extension_rays"] and stats["shadow_rays"] == want["shadow_rays"]
+    del image
+    torch.cuda.empty_cache()
+    kept = _used() - before - volumes
+    assert 358 * 640 * 360 * 4 * 2 < kept <= (1 << 30) + 9 * (2 << 20) + SLACK
+    for dag in dags:
+        dag.destroy()
+    dag = cbq.Dag(*scene)
+    _frame(dag, 640, 360, 4)  # room again
+    torch.cuda.empty_cache()
+    assert _used() - before > 300 * 640 * 360 * 4
+    dag.destroy()
+    assert _used() - before <= SLACK
