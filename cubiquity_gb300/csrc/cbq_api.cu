@@ -411,22 +411,24 @@ cbq_status cbq_dag_create_ex(const uint32_t* host_nodes, uint64_t node_count, ui
     dag->device_bytes = bytes;
     const bool tag = dag->flat_ok && dag->layout == CBQ_DAG_LAYOUT_REFERENCE && node_count <= kTaggedMaxNodes;
     // One allocation: the node array, its tagged copy and the tables of upper cells (a cudaMalloc
-    // takes 70 us).  Without memory for all of it there is the node array alone, and the walk
-    // takes that.
+    // takes 70 us).
     const bool masks = tag || dag->layout == CBQ_DAG_LAYOUT_COMPACT;
     const size_t part = (bytes + 255u) & ~(size_t)255u;
     const size_t top_bytes = masks ? (size_t)number_top_tables(dag) * dev::kTopCells * 32u : 0u;
-    const size_t total = part + (tag ? part : 0u) + top_bytes;
-    const bool whole = cudaMalloc((void**)&dag->d_nodes, total) == cudaSuccess;
-    if (!whole) {
+    const size_t total = masks ? part + (tag ? part : 0u) + top_bytes : bytes;
+    bool whole = false;
+    dag->d_nodes = (uint32_t*)allocate_store(total, bytes, [](uint64_t n) {
+        void* p = nullptr;
+        if (cudaMalloc(&p, n) == cudaSuccess) return p;
         cudaGetLastError();
-        for (uint32_t& t : dag->top_index) t = 0u;
-        if (cudaMalloc((void**)&dag->d_nodes, bytes) != cudaSuccess) {
-            cudaGetLastError();
-            delete dag;
-            return CBQ_ERR_OUT_OF_MEMORY;
-        }
+        return (void*)nullptr;
+    }, &whole);
+    if (!dag->d_nodes) {
+        delete dag;
+        return CBQ_ERR_OUT_OF_MEMORY;
     }
+    if (!whole)
+        for (uint32_t& t : dag->top_index) t = 0u;
     cudaError_t e = cudaMemcpy(dag->d_nodes, src, bytes, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && whole && tag) {
         dag->d_tagged = dag->d_nodes + part / 4u;

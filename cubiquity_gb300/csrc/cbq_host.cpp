@@ -96,6 +96,20 @@ void log(int level, const char* fmt, ...)
     fn(g_log_user.load(), level, buf);
 }
 
+void* allocate_store(uint64_t whole, uint64_t store, void* (*allocate)(uint64_t bytes), bool* is_whole)
+{
+    void* p = allocate(whole);
+    *is_whole = p != nullptr;
+    if (p || whole <= store) return p;
+    p = allocate(store);
+    if (p)
+        log(CBQ_LOG_WARNING,
+            "no device memory for the %.1f MB that the fast walk takes beside the node store (%.1f MB): "
+            "traversals of this DAG take the node array itself, and run on their own in batches",
+            (double)(whole - store) / 1e6, (double)store / 1e6);
+    return p;
+}
+
 cbq_status validate_heights(const uint32_t* nodes, uint64_t node_count, const cbq_subdag subdags[8])
 {
     // Heights (0..31) at which each internal node has been reached.

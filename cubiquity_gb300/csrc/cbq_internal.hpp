@@ -26,6 +26,13 @@ cbq_status validate_nodes(const uint32_t* nodes, uint64_t node_count, uint32_t r
 // overflows nor underflows, s / t > max_footprint exactly when t <= s * that.
 float footprint_exit_max(float max_footprint);
 
+// Device memory for a DAG: `whole` bytes (the node store, the walk's copy of it and the tables of
+// upper cells), or, with a warning in the log, `store` bytes for the node store alone, where the
+// walk takes the plain array (4 Mi bounce rays on terrain-4096 658 us instead of 526) and the
+// batch kernel does not take the DAG (12 volumes 676 us instead of 213).  nullptr without memory
+// for that either.
+void* allocate_store(uint64_t whole, uint64_t store, void* (*allocate)(uint64_t bytes), bool* is_whole);
+
 // printf-style message to the registered log handler (no-op without one).
 void log(int level, const char* fmt, ...)
 #if defined(__GNUC__)
