@@ -850,10 +850,17 @@ __device__ __forceinline__ void lane_walk_steps(Lane& L, const Src& c, Stack& st
     if (L.mode == kLaneWalk && L.fetches >= kMaxFetches) L.mode = kLaneLimit;
 }
 
+// Steps of the reference form between a warp's checks, at least: an incoherent
+// warp's eight iterations are made for the ordered walk, whose iteration takes up
+// to two steps.  With eight, 1 Mi incoherent rays from 2^24 voxels away 329 us,
+// with sixteen 323.
+constexpr uint32_t kReferenceSteps = 16u;
+
 // The walk of a whole warp (all 32 lanes must call it), then the results of
 // the rays that finished in it are written.  Float positions: ordered lanes walk
 // until `idle_min` of the warp's lanes do not (checked every `steps`
-// iterations), the others take up to `steps` steps of the reference form.
+// iterations), the others take up to `steps` steps of the reference form, or
+// kReferenceSteps.
 // Integer positions: the FAST min/max when every walking lane's ray allows it.
 template <typename Src, typename Stack>
 __device__ __forceinline__ void warp_walk_steps(Lane& L, const Src& c, Stack& stack, uint32_t steps,
@@ -870,7 +877,8 @@ __device__ __forceinline__ void warp_walk_steps(Lane& L, const Src& c, Stack& st
             const uint32_t walking = __ballot_sync(0xffffffffu, L.mode == kLaneWalk && L.fast);
             if (walking == 0u || 32u - __popc(walking) >= idle_min) break;
         }
-        if (L.mode == kLaneWalk && !L.fast) lane_walk_steps<false>(L, c, stack, steps);
+        if (L.mode == kLaneWalk && !L.fast)
+            lane_walk_steps<false>(L, c, stack, steps < kReferenceSteps ? kReferenceSteps : steps);
         __syncwarp();
         if (L.mode == kLaneNext) lane_next(L, c);
     }

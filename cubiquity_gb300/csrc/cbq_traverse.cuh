@@ -154,10 +154,13 @@ __device__ __forceinline__ uint32_t first_child(const RayFrame& f, float entry, 
 // hasLargeFootprint = (childNodeSize / tChildExit) > maxFootprint
 // (raytracing.cpp:276).  With the LOD disabled (maxFootprint < 0) and a positive
 // exit the quotient is positive, so the division is skipped; every other case
-// divides exactly as the reference does.
+// divides exactly as the reference does.  The exit is opaque there, so that the
+// division stays in its branch: the compiler otherwise made one in every step
+// (rays from 2^24 voxels away, camera / incoherent 204 / 323 us, now 196 / 312).
 __device__ __forceinline__ bool large_footprint(float cns, float t_exit, float mf)
 {
     if (mf < 0.0f && t_exit > 0.0f) return true;
+    asm volatile("" : "+f"(t_exit));
     return (cns / t_exit) > mf;
 }
 __device__ __forceinline__ bool large_footprint(int32_t cns, float t_exit, float mf)
