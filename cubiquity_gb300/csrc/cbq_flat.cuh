@@ -126,7 +126,9 @@ struct FlatCtxT {
     __device__ __forceinline__ uint32_t occupied(const Lane&) const { return dag.occupied; }
     __device__ __forceinline__ const uint4* top(const Lane&) const { return dag.top; }
     __device__ __forceinline__ const SubDag& subdag(const Lane&, uint32_t k) const { return dag.sd[k]; }
-    // Rays are read once: streaming loads (evict-first) leave L2 to the node store.
+    // A ray is read where its walk starts and again where it ends in a hit (flush_held), crosses
+    // octants by the quotients or starts again; streaming loads (evict-first) leave L2 to the node
+    // store, at up to 32 bytes of DRAM traffic for a hit's second read.
     __device__ __forceinline__ float4 ray_origin(const Lane&, uint64_t i) const { return __ldcs(orig + i); }
     __device__ __forceinline__ float4 ray_direction(const Lane&, uint64_t i) const { return __ldcs(dir + i); }
     __device__ __forceinline__ void write(const Lane& L, const RayResult& r) const
@@ -894,7 +896,8 @@ __device__ __forceinline__ void warp_walk_steps(Lane& L, const Src& c, Stack& st
 // and checks every 32 iterations, else for 16 and every 8.  Both ways, us:
 // terrain-4096 camera rays 331 / 365, bounce rays 569 / 545 (camera rays checked
 // every 16 iterations 333).  Equal directions (sun rays from scattered surfaces)
-// tell less: every 16 (1.5 M shadow rays 123, every 32 125).  The batch and
+// tell less: every 16 (1.5 M shadow rays of a frame in its pixels' order 136, every
+// 32 138; the same rays shuffled 165 / 178).  The batch and
 // server launches keep 16 and 8: their small volumes' camera rays gain nothing
 // from waiting (12 volumes: 240 us, chosen by the rays 245).
 struct WarpRefill {

@@ -122,8 +122,8 @@ extern "C" cbq_status cbq_intersect_host_noalloc(const cbq_dag* dag, const float
     if (!host_hits->voxel) launch.voxel = nullptr;
     if (!host_hits->status) launch.status = nullptr;
     cbq_rays rays{d_o, d_d};
-    // Always the persistent form (whatever the DAG's launch form): its work
-    // counter lives in the array too.  Results are the same bits in every form.
+    // The persistent entry point (whatever the DAG's launch form): where it takes a work
+    // counter, that lives in the array too.  Results are the same bits in every form.
     st = cbq_intersect_persistent(dag, &rays, n, query, &launch, d_counter, 0u, (cbq_stream_t)s);
     if (st != CBQ_OK) return drain(st);
     struct Copy { void* dst; const void* src; size_t bytes; };

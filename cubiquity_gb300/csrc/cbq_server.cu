@@ -100,9 +100,9 @@ void resolve_buffers(Request& rq)
 }
 
 // Copies of a launch between its requests' page-locked buffers and the pool, two
-// kernels for every request of a launch (cbq_stage.cuh): 24 requests of 1 Ki to
-// 64 Ki rays submitted from one Python thread 1,040 -> 828 us (median latency of
-// one 136 -> 107 us) against the copy engine's calls.
+// kernels for every request of a launch (cbq_stage.cuh).  Against the copy engine's
+// calls, the rest alike: one request at a time of 64 / 2,048 / 16,384 rays 87 / 100
+// / 103 -> 68 / 81 / 88 us, the serving benchmark's peak 34.1 k -> 60.5 k requests/s.
 constexpr uint64_t kStageRequestsMax = 4096;  // per launch: seven times that are grid rows
 
 // Row y of the grid copies the rays of in[y]; the last row the job table (in

@@ -121,8 +121,10 @@ typedef struct cbq_dag_info {
     cbq_subdag subdags[8];
     const uint32_t* device_nodes;
     uint32_t layout;          /* CBQ_DAG_LAYOUT_* in use */
-    uint64_t device_bytes;    /* bytes of the device node store (the reference layout
-                                 keeps as much again for the walk's own copy) */
+    uint64_t device_bytes;    /* bytes of the device node store.  Beside it the reference
+                                 layout keeps as much again for the walk's own copy (DAGs
+                                 of up to 2^24 nodes within +-2^21), and both layouts 1 MiB
+                                 per SubDAG of height 6 or more */
 } cbq_dag_info;
 
 /* ---------------------------------------------------------------- basics */
@@ -241,19 +243,25 @@ cbq_status cbq_dag_set_l2_persistence(const cbq_dag* dag, cbq_stream_t stream, f
 
 /* intersectVolume (raytracing.h:72-76 / raytracing.cpp:397-478) for n rays:
  * one launch, device rays in, device hits out, stream-ordered.  It runs in the
- * DAG's launch form: persistent by default, with a work counter the DAG keeps
- * per stream (allocated on the first call on a stream, so launches sharing it
- * are ordered by that stream), or one thread per ray for CBQ_FORM_PLAIN and
- * while the stream is being captured into a graph. */
+ * DAG's launch form: persistent by default, with work counters the DAG keeps
+ * per stream (allocated on the first such call on a stream, so launches sharing
+ * them are ordered by that stream).  Launched without a counter: with
+ * CBQ_FORM_PLAIN and while the stream is being captured into a graph, one thread
+ * per ray; with the default refill and steps, calls that the device holds at once
+ * (SMs * 1,024 rays), spread over its warps, and images (image_width) of up to
+ * 3 * 2^19 rays, one thread per ray. */
 cbq_status cbq_intersect(const cbq_dag* dag, const cbq_rays* rays, uint64_t n,
                          const cbq_query* query, const cbq_hits* hits, cbq_stream_t stream);
 
 /* As cbq_intersect, with HOST rays and HOST hits: copies in, traverses, copies
- * out, and waits for completion.  Calls of 2^19 rays or more are split into up
- * to 8 chunks whose copies overlap the traversal of their neighbours (own
- * streams; page-locked host buffers copy fastest); each chunk takes every k-th
- * of about 4k blocks of consecutive rays, so chunks carry even work.  Allocates
- * and caches device staging buffers and streams per dag.  Calls on one dag from
+ * out, and waits for completion.  With page-locked (or managed) buffers, calls of
+ * 196,608 rays or more are split into two to four chunks of 1:2:3:4 parts whose
+ * copies overlap the traversal of their neighbours (own streams); each chunk
+ * takes its part of each of four blocks of consecutive rays, so chunks carry even
+ * work.  Smaller calls are copied by one kernel each way.  Both need every buffer
+ * to lie whole in one page-locked allocation or registration; other calls take
+ * one chunk, as copies from and to pageable memory block the calling thread.
+ * Allocates and caches device staging buffers and streams per dag.  Calls on one dag from
  * several host threads run concurrently, each with its own staging set (up to
  * four sets per dag, created as needed; further calls wait for one), so one
  * call's copies and traversal overlap another's.  On an error every copy and
@@ -278,7 +286,7 @@ cbq_status cbq_intersect_host(const cbq_dag* dag, const float* host_origin_tmax,
  *   - The current device must be the DAG's device.
  *   - Copies and the launch go on the calling thread's per-thread stream
  *     (cudaStreamPerThread), so the call neither waits for nor holds up other
- *     streams.  It always runs the persistent form (same results as every
+ *     streams.  It runs cbq_intersect_persistent's launch (same results as every
  *     other form, whatever the DAG's launch configuration says).
  *   - Every call on a device shares the array and leaves its contents behind;
  *     each call rewrites what it reads (rays, hits) and zeroes the counter.
@@ -293,7 +301,8 @@ cbq_status cbq_intersect_host_noalloc(const cbq_dag* dag, const float* host_orig
 
 /* Persistent form: a grid sized to the device's SMs whose warps pull rays from
  * an atomic work counter.  `work_counter` is caller-owned device scratch (one
- * uint64, zeroed by this call on `stream`).  With the flat kernel a warp takes
+ * uint64, zeroed by this call on `stream`, or not used where a small call is
+ * spread without one, see cbq_intersect).  With the flat kernel a warp takes
  * new rays whenever `chunk` (<= 32) of its lanes are idle; with the nested one
  * it takes `chunk` rays at a time.  chunk = 0 selects the tuned default. */
 cbq_status cbq_intersect_persistent(const cbq_dag* dag, const cbq_rays* rays, uint64_t n,
@@ -498,7 +507,10 @@ typedef void (*cbq_pt_wave_fn)(void* user, int32_t kind, int32_t depth, int32_t 
 cbq_status cbq_copy_to_host(void* host_dst, const void* device_src, uint64_t bytes);
 
 /* Renders into device_image (width * height * 3 floats, the mean over samples).
- * Synchronous; allocates its wave buffers for the call. */
+ * Synchronous.  Its wave buffers take 260 bytes of device memory per path of a
+ * pass, or 358 in frames without a callback for which that is 1 GiB at most.  They
+ * are kept with the DAG for its next frame as long as those of all DAGs of the
+ * process come to 1 GiB at most, else freed with the frame. */
 cbq_status cbq_pathtrace(const cbq_dag* dag, const cbq_pt_config* cfg, float* device_image,
                          cbq_pt_wave_fn on_wave, void* user, cbq_pt_stats* stats, cbq_stream_t stream);
 
