@@ -1,5 +1,7 @@
 """Device memory of a frame: 260 bytes a path, and in frames small enough for their
 workspace to be kept, traced without a callback, a second shadow set (98 more)."""
+import gc
+
 import pytest
 
 import cubiquity_gb300 as cbq
@@ -14,6 +16,14 @@ SLACK = 8 << 20  # the image, counters, padding, CUDA's own granularity
 def _used():
     free, total = torch.cuda.mem_get_info()
     return total - free
+
+
+@pytest.fixture(autouse=True)
+def nothing_left_over():
+    """Device memory of earlier tests is given back before a test looks at what is used."""
+    gc.collect()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
 
 
 @pytest.fixture(scope="module")
